@@ -61,6 +61,9 @@ long long ow3d_test_set_coop_max_points(long long points);
  * captured graphs keep what they were captured with. Returns the previous
  * value. Process-wide. */
 int ow3d_test_set_pdl(int on);
+/* 0: every multigrid level takes the per-phase kernels, 1 (default): levels
+ * that have a tile form (mg_tile.cu) take it. Returns the previous value. */
+int ow3d_test_set_tiles(int on);
 long long ow3d_test_set_tail_max_points(long long points);
 int ow3d_test_set_tail_cluster(int blocks);
 

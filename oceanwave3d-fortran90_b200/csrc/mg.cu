@@ -23,6 +23,7 @@
 // barriers, instead of one launch per phase.
 #include "ow3d_internal.h"
 #include "mg_device.cuh"
+#include "mg_tile.cuh"
 #include <cooperative_groups.h>
 #include <cstring>
 #include <vector>
@@ -592,6 +593,7 @@ std::atomic<int> g_tail_cluster{16};
 // launcher).
 std::atomic<int> g_colour_tiles{0};
 std::atomic<int> g_colour_prefetch{-1};
+std::atomic<int> g_tiles{1};
 // Programmatic dependent launch between the solver-path kernels (launch_k).
 std::atomic<int> g_pdl{1};
 
@@ -726,19 +728,43 @@ static int coop_level(const LevelDev<T>* lev, int nlev) {
     return lc;
 }
 
-// MultiGridSolver.f90:5-192 (V cycle, gam = 1), levels lev[0] coarsest;
-// level ld is solved by the dense operator M.
+// Whether level l takes the fused tile kernels (they hold one smoothing step
+// either side of the coarse correction, from a zero iterate).
 template <typename T>
-static void vcycle(LevelDev<T>* lev, int l, int lc, int ld, const T* M, int nu1, int nu2, LevelTable<T>& pack,
-                   cudaStream_t st) {
-    if (l == ld) { launch_dense_apply(lev[l], M, st); return; }
-    if (l <= lc) {
+static bool tiled(const LevelTable<T>& pack, int l, int ld) {
+    return l > ld && pack.tile && pack.tile[l].mode != kTileNone;
+}
+
+// MultiGridSolver.f90:5-192 (V cycle, gam = 1), levels lev[0] coarsest;
+// level ld is solved by the dense operator M. top is the level the cycle
+// started from, whose iterate receives the result; tiles allows the fused
+// tile kernels. Returns where level l's result is: a tiled level's smoothed
+// iterate goes out of place (from xv to rv, at the top from rv to xv),
+// because a tile's halo is read while its neighbours are written.
+template <typename T>
+static T* vcycle(LevelDev<T>* lev, int top, int l, int lc, int ld, const T* M, int nu1, int nu2, bool tiles,
+                 LevelTable<T>& pack, cudaStream_t st) {
+    if (l == ld) { launch_dense_apply(lev[l], M, st); return lev[l].xv; }
+    // the fused coarse cycle takes all levels from lc down unless each of
+    // them has its tile form
+    bool all = tiles;
+    for (int q = ld + 1; q <= l && all; ++q) all = tiled(pack, q, ld);
+    if (l <= lc && !all) {
         if (lev[0].Nyg > 1) coarse_cycle<T, true>(lev, l, ld, M, nu1, nu2, pack, st);
         else coarse_cycle<T, false>(lev, l, ld, M, nu1, nu2, pack, st);
-        return;
+        return lev[l].xv;
     }
     const LevelDev<T>& F = lev[l];
     LevelDev<T>& Cc = lev[l - 1];
+    if (tiles && tiled(pack, l, ld)) {
+        T* const xs = l == top ? F.rv : F.xv;
+        T* const out = l == top ? F.xv : F.rv;
+        const bool clear = l - 1 > ld && !(all || (l - 1 > lc && tiled(pack, l - 1, ld)));
+        launch_tile_down(F, Cc, pack.tile[l], (const T*)F.bv, xs, Cc.bv, clear ? Cc.xv : (T*)nullptr, st);
+        const T* const xc = vcycle(lev, top, l - 1, lc, ld, M, nu1, nu2, tiles, pack, st);
+        launch_tile_up(F, Cc, pack.tile[l], (const T*)F.bv, (const T*)xs, xc, out, st);
+        return out;
+    }
     if (pack.lex) launch_lo_smooth_lex(F, nu1, st);
     else launch_lo_smooth(F, nu1, st);
     if (F.Nyg > 1) {
@@ -749,10 +775,11 @@ static void vcycle(LevelDev<T>* lev, int l, int lc, int ld, const T* M, int nu1,
         else launch_k(k_lo_residual<T, false, false>, dim3(nblk(F.N)), dim3(256), 0, st, F);
     }
     launch_restrict(F, Cc, (const T*)F.rv, Cc.bv, st);   // also zeroes Cc.xv
-    vcycle(lev, l - 1, lc, ld, M, nu1, nu2, pack, st);
-    launch_prolong_add(F, Cc, (const T*)Cc.xv, F.xv, st);
+    const T* const xc = vcycle(lev, top, l - 1, lc, ld, M, nu1, nu2, tiles, pack, st);
+    launch_prolong_add(F, Cc, xc, F.xv, st);
     if (pack.lex) launch_lo_smooth_lex(F, nu2, st);
     else launch_lo_smooth(F, nu2, st);
+    return F.xv;
 }
 
 // One V cycle from level l (its b set, its x zeroed by the caller) down to the
@@ -761,7 +788,7 @@ template <typename T>
 void launch_mg_subcycle(LevelDev<T>* lev, int nlev, int l, int ld, const T* M, int nu1, int nu2, LevelTable<T>& pack,
                         cudaStream_t st) {
     const int lc = (nlev > 1 && !pack.lex) ? coop_level(lev, nlev) : -1;
-    vcycle(lev, l, lc, ld, M, nu1, nu2, pack, st);
+    vcycle(lev, l, l, lc, ld, M, nu1, nu2, false, pack, st);
 }
 
 // MultiGridSolveLinearSystem.f90:26-91: u = 0, then maxit cycles.
@@ -769,11 +796,14 @@ template <typename T>
 void launch_mg_vcycle(LevelDev<T>* lev, int nlev, const T* M, int ld, int nu1, int nu2, int maxit, LevelTable<T>& pack,
                       cudaStream_t st) {
     LevelDev<T>& F = lev[nlev - 1];
-    launch_fill<T>(F.xv, T(0), F.N, st);
+    const bool tiles = nlev > 1 && nu1 == 1 && nu2 == 1 && maxit == 1 && !pack.lex && pack.tile &&
+                       g_tiles.load(std::memory_order_relaxed) != 0;
+    // a tiled finest level starts from a zero iterate by itself
+    if (!(tiles && tiled(pack, nlev - 1, ld))) launch_fill<T>(F.xv, T(0), F.N, st);
     const int lc = (nlev > 1 && !pack.lex) ? coop_level(lev, nlev) : -1;
     for (int it = 1; it <= maxit; ++it) {
         if (nlev == 1 && it > 1) break;
-        vcycle(lev, nlev - 1, lc, ld, M, nu1, nu2, pack, st);
+        vcycle(lev, nlev - 1, nlev - 1, lc, ld, M, nu1, nu2, tiles, pack, st);
     }
 }
 

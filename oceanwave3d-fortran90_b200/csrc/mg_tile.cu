@@ -1,0 +1,1167 @@
+// Multigrid levels as two launches each: one for the way down (one smoothing
+// step from a zero iterate, residual, restriction) and one for the way up
+// (prolongation, correction, one smoothing step). The per-phase kernels of
+// mg.cu make 9 launches (2 colours) or 15 (4 colours) of the same work, each
+// a pass over the level in memory.
+//
+// A block owns a core of cx x cy columns and works on it plus a halo in
+// shared memory; every phase recomputes the halo columns that the following
+// phases of the core need, so no phase waits for another block. With nc
+// colours the halo is
+//   uniform levels  down 3: colour 0 at distance <= 3 of the core, colour 1 at
+//                   <= 2, residual at <= 1; up 2.
+//   cross levels    down nc + 3: bottom rows at <= nc + 3, colour c at
+//                   <= nc + 2 - c, bottom rows again at <= 2, residual at <= 1;
+//                   up nc + 2.
+// The arithmetic per row is the colour pass's (mg_device.cuh) up to the order
+// of the sums.
+//
+// On uniform levels one thread solves one column bottom to top: the sums over
+// neighbour columns do not depend on the row below, only
+// x_k = q_k - g_k x_{k-1} is a chain. On cross levels, whose rows cost an
+// order more, the lanes of a segment share a column. Columns lie in shared memory with an odd
+// pitch and the columns of one parity of i side by side, so that the threads
+// of a warp, which take every other column, meet no bank conflict.
+#include "mg_tile.cuh"
+#include "mg_device.cuh"
+
+#include <algorithm>
+
+namespace ow3d {
+
+namespace {
+using namespace mgdev;
+
+constexpr int kCrossThreads = 512;
+constexpr size_t kTileSmemMax = 220 * 1024, kTileSmemTwo = 112 * 1024;
+
+// Core and staged region of a block, 1-based columns; on a periodic level i
+// runs past the ends and is taken cyclically (gcol).
+struct Reg {
+    int ia, ib, ra, rb, W;   // core and region in x
+    int ja, jb, sa, sb, H;   // in y
+};
+
+// Core t of columns 1..n (the first `rem` cores hold q + 1 columns, the others
+// q). A core holds three columns or more, so a wall's ghost column always lies
+// in a core with the two interior columns that determine it.
+__host__ __device__ inline void span(int n, int t, int q, int rem, int halo, int& a, int& b, int& ra, int& rb) {
+    a = 1 + t * q + (t < rem ? t : rem);
+    b = a + q - 1 + (t < rem ? 1 : 0);
+    ra = a - halo > 1 ? a - halo : 1;
+    if (ra <= 3) ra = 1;                 // a region that holds column 2 or 3 holds the ghost column too
+    rb = b + halo < n ? b + halo : n;
+    if (rb >= n - 2) rb = n;
+}
+__host__ __device__ inline Reg region(int Nxg, int Nyg, int per, const TileGeo& g, int bx, int by, bool three) {
+    Reg r;
+    if (per) {
+        span(Nxg, bx, g.qx, g.remx, 0, r.ia, r.ib, r.ra, r.rb);
+        r.ia += 1; r.ib += 1;            // the distinct columns 2..Nxg-2
+        r.ra = r.ia - g.halo;
+        r.rb = r.ib + g.halo;
+    } else {
+        span(Nxg, bx, g.qx, g.remx, g.halo, r.ia, r.ib, r.ra, r.rb);
+    }
+    if (three) span(Nyg, by, g.qy, g.remy, g.halo, r.ja, r.jb, r.sa, r.sb);
+    else r.ja = r.jb = r.sa = r.sb = 1;
+    r.W = r.rb - r.ra + 1;
+    r.H = r.sb - r.sa + 1;
+    return r;
+}
+// Whether the region touches a wall (and so holds ghost columns).
+__device__ __forceinline__ bool at_wall(int Nxg, int Nyg, int per, const Reg& r, bool three) {
+    return (!per && (r.ra == 1 || r.rb == Nxg)) || (three && (r.sa == 1 || r.sb == Nyg));
+}
+// Periodic x: the distinct column that stands at i.
+__device__ __forceinline__ int gcol(int i, int Nxg, int per) {
+    if (!per) return i;
+    const int M = Nxg - 3;
+    int t = (i - 2) % M;
+    if (t < 0) t += M;
+    return 2 + t;
+}
+
+template <typename T> struct Pair;
+template <> struct Pair<double> { using type = double2; };
+template <> struct Pair<float> { using type = float2; };
+template <typename T>
+__device__ __forceinline__ typename Pair<T>::type pair_at(const T* p) {
+    return *reinterpret_cast<const typename Pair<T>::type*>(p);
+}
+
+// Visit H rows of W columns of Nzg values each: a thread keeps one place k in
+// the column (N rows: 2 where Nzg is even -- a pair then lies on its own
+// alignment -- else 1) and steps through the columns, U visits in flight, so
+// that an access costs a few additions of index arithmetic. acc.ld<N>(v, c, q)
+// reads column c of row q, acc.st<N>(c, q, v) stores; acc is made for the
+// thread's k.
+template <int N, int U, typename T, int M, typename ACC>
+__device__ __forceinline__ void sweep_n(int W, int H, int Nzg, ACC make) {
+    const int nu = Nzg / N, cg = threadIdx.x / nu, step = blockDim.x / nu;
+    if (cg >= step) return;
+    const auto acc = make(N * (threadIdx.x - cg * nu));
+    int q = cg / W, c = cg - q * W;
+    const int dq = step / W, dc = step - dq * W;
+    while (q < H) {
+        T v[U][M * N];
+        int cc[U], qq[U];
+#pragma unroll
+        for (int m = 0; m < U; ++m) {
+            cc[m] = c;
+            qq[m] = q;
+            if (q < H) acc.template ld<N>(v[m], c, q);
+            c += dc;
+            q += dq;
+            if (c >= W) { c -= W; ++q; }
+        }
+#pragma unroll
+        for (int m = 0; m < U; ++m)
+            if (qq[m] < H) acc.template st<N>(cc[m], qq[m], v[m]);
+    }
+}
+template <int U, typename T, int M, typename ACC>
+__device__ __forceinline__ void sweep(int W, int H, int Nzg, ACC make) {
+    if ((Nzg & 1) == 0) sweep_n<2, U, T, M>(W, H, Nzg, make);
+    else sweep_n<1, U, T, M>(W, H, Nzg, make);
+}
+template <typename T>
+__device__ __forceinline__ void put_pair(T* p, T a, T b) {
+    typename Pair<T>::type q;
+    q.x = a; q.y = b;
+    *reinterpret_cast<typename Pair<T>::type*>(p) = q;
+}
+// N values to a staged array; VEC: its columns have an even pitch (uniform
+// levels), so that pairs go in one access.
+template <int N, bool VEC, typename T>
+__device__ __forceinline__ void put(T* p, const T* v) {
+    if constexpr (N == 2 && VEC) put_pair(p, v[0], v[1]);
+    else if constexpr (N == 2) { p[0] = v[0]; p[1] = v[1]; }
+    else p[0] = v[0];
+}
+template <int N, typename T>
+__device__ __forceinline__ void get(T* v, const T* p) {
+    if constexpr (N == 2) { const auto q = pair_at(p); v[0] = q.x; v[1] = q.y; }
+    else v[0] = p[0];
+}
+
+// Offset of column (li, lj) of the region (0-based) in a staged array.
+__device__ __forceinline__ int slot(const TileGeo& g, int li, int lj) {
+    return ((lj * 2 + (li & 1)) * g.HW + (li >> 1)) * g.NZP;
+}
+// The same within a row (add row_slot of its row).
+__device__ __forceinline__ int col_slot(const TileGeo& g, int li) { return ((li & 1) * g.HW + (li >> 1)) * g.NZP; }
+__device__ __forceinline__ int row_slot(const TileGeo& g, int lj) { return 2 * lj * g.HW * g.NZP; }
+// Offsets to the left and right neighbour columns of a column of parity li & 1.
+__device__ __forceinline__ int near_l(const TileGeo& g, int li) { return li & 1 ? -g.HW * g.NZP : (g.HW - 1) * g.NZP; }
+__device__ __forceinline__ int near_r(const TileGeo& g, int li) { return li & 1 ? (1 - g.HW) * g.NZP : g.HW * g.NZP; }
+
+// The interior columns of `colour` at distance <= d of the core, one per
+// thread in turn: f(i, j).
+template <bool THREE, typename F>
+__device__ __forceinline__ void colour_columns(int Nxg, int Nyg, int per, const Reg& r, int ncolor, int colour, int d,
+                                               F f) {
+    int ilo = r.ia - d, ihi = r.ib + d, jlo = 1, jhi = 1;
+    if (!per) { ilo = max(ilo, 2); ihi = min(ihi, Nxg - 1); }
+    if (THREE) { jlo = max(r.ja - d, 2); jhi = min(r.jb + d, Nyg - 1); }
+    const bool four = ncolor == 4;
+    int js = 1;
+    if (THREE && four) {
+        jlo += (jlo ^ (colour >> 1)) & 1;
+        js = 2;
+    }
+    const int ni = (ihi - ilo + 2) >> 1, nj = jhi >= jlo ? (jhi - jlo) / js + 1 : 0;
+    for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
+        const int tj = t / ni, j = jlo + tj * js;
+        const int par = four ? colour & 1 : (colour + j) & 1;
+        const int i = ilo + ((ilo ^ par) & 1) + 2 * (t - tj * ni);
+        if (i <= ihi) f(i, j);
+    }
+}
+
+// All interior columns at distance <= d of the core.
+template <bool THREE, typename F>
+__device__ __forceinline__ void all_columns(int Nxg, int Nyg, int per, const Reg& r, int d, F f) {
+    int ilo = r.ia - d, ihi = r.ib + d, jlo = 1, jhi = 1;
+    if (!per) { ilo = max(ilo, 2); ihi = min(ihi, Nxg - 1); }
+    if (THREE) { jlo = max(r.ja - d, 2); jhi = min(r.jb + d, Nyg - 1); }
+    const int ni = max(ihi - ilo + 1, 0), nj = max(jhi - jlo + 1, 0);
+    for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
+        const int tj = t / ni;
+        f(ilo + t - tj * ni, jlo + tj);
+    }
+}
+
+// The ghost columns of the region (corners excluded): f(place of row k in the
+// ghost column, in its nearest and in its second interior column, i and j of
+// the nearest, whether the wall is an x wall, 0 or 1 for the low or high one)
+// for the 0-based rows k = 1..Nzg-1. All walls in one loop.
+template <bool THREE, typename F>
+__device__ __forceinline__ void ghost_rows(int Nxg, int Nyg, int per, int Nzg, uint32_t mz, int sz, const Reg& r,
+                                           const TileGeo& g, F f) {
+    const int jlo = THREE ? max(r.sa, 2) : 1, jhi = THREE ? min(r.sb, Nyg - 1) : 1;
+    const int ilo = per ? r.ra : max(r.ra, 2), ihi = per ? r.rb : min(r.rb, Nxg - 1);
+    const int nx = jhi - jlo + 1, ny = ihi - ilo + 1;
+    const int n0 = !per && r.ra == 1 ? nx : 0, n1 = n0 + (!per && r.rb == Nxg ? nx : 0);
+    const int n2 = n1 + (THREE && r.sa == 1 ? ny : 0), n3 = n2 + (THREE && r.sb == Nyg ? ny : 0);
+    const int row = 2 * g.HW * g.NZP;
+    for (int t = threadIdx.x; t < n3 * Nzg; t += blockDim.x) {
+        const int q = (int)div32((uint32_t)t, mz, sz), k = t - q * Nzg;
+        if (k == 0) continue;
+        const bool xw = q < n1;
+        const int side = xw ? (q >= n0) : (q >= n2);
+        const int p = q - (xw ? (side ? n0 : 0) : (side ? n2 : n1));
+        if (xw) {
+            const int gi = side ? Nxg : 1, d = side ? -1 : 1, j = jlo + p, li = gi - r.ra, lj = j - r.sa;
+            f(slot(g, li, lj) + k, slot(g, li + d, lj) + k, slot(g, li + 2 * d, lj) + k, gi + d, j, true, side);
+        } else {
+            const int gj = side ? Nyg : 1, d = side ? -1 : 1, i = ilo + p, s = slot(g, i - r.ra, gj - r.sa) + k;
+            f(s, s + d * row, s + 2 * d * row, i, gj + d, false, side);
+        }
+    }
+}
+
+// The same two rows at a time (arrays of even pitch): f(place of the pair in
+// the ghost column, the nearest, the second; x wall; side; first row).
+template <bool THREE, typename F>
+__device__ __forceinline__ void ghost_pairs(int Nxg, int Nyg, int per, const Reg& r, const TileGeo& g, F f) {
+    const int jlo = THREE ? max(r.sa, 2) : 1, jhi = THREE ? min(r.sb, Nyg - 1) : 1;
+    const int ilo = per ? r.ra : max(r.ra, 2), ihi = per ? r.rb : min(r.rb, Nxg - 1);
+    const int nx = jhi - jlo + 1, ny = ihi - ilo + 1;
+    const int n0 = !per && r.ra == 1 ? nx : 0, n1 = n0 + (!per && r.rb == Nxg ? nx : 0);
+    const int n2 = n1 + (THREE && r.sa == 1 ? ny : 0), n3 = n2 + (THREE && r.sb == Nyg ? ny : 0);
+    const int row = row_slot(g, 1);
+    for (int t = threadIdx.x; t < n3 * g.np; t += blockDim.x) {
+        const int q = (int)div32((uint32_t)t, g.mnp, g.snp), k = 2 * (t - q * g.np);
+        const bool xw = q < n1;
+        const int side = xw ? (q >= n0) : (q >= n2);
+        const int p = q - (xw ? (side ? n0 : 0) : (side ? n2 : n1));
+        if (xw) {
+            const int d = side ? -1 : 1, li = (side ? Nxg : 1) - r.ra, o = row_slot(g, jlo + p - r.sa) + k;
+            f(o + col_slot(g, li), o + col_slot(g, li + d), o + col_slot(g, li + 2 * d), true, side, k);
+        } else {
+            const int d = side ? -row : row, s = slot(g, ilo + p - r.ra, (side ? Nyg : 1) - r.sa) + k;
+            f(s, s + d, s + 2 * d, false, side, k);
+        }
+    }
+}
+
+// Owned coarse columns of a core span [a, b] of an axis of nf fine and nc
+// coarse columns, coarsened (F = 2) or not (F = 1).
+__device__ __forceinline__ void owned(int a, int b, int nf, int nc, int F, int per, int& lo, int& hi) {
+    const int s = F - 1;
+    if (per) { lo = 2 + ((a - 2 + s) >> s); hi = 2 + ((b - 2) >> s); return; }
+    lo = a == 1 ? 1 : (a == nf ? nc : 2 + ((a - 2 + s) >> s));
+    hi = b == nf ? nc : (b == 1 ? 1 : 2 + ((b - 2) >> s));
+}
+
+// Restrict the residual staged in rs to the owned coarse columns
+// (MGRestriction3DExplicit.f90:19-128; on a uniform grid the weights in x and
+// y are 1/4, 1/2, 1/4). The residual is zero on the ghost columns, in the
+// bottom rows and in the free-surface row: a smoothing step ends with these
+// rows relaxed last. Four lanes share a coarse column.
+template <bool THREE, bool VEC, typename T>
+__device__ __forceinline__ void restrict_tile(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileGeo& g,
+                                              const Reg& r, int bx, const T* rs, T* __restrict__ rc,
+                                              T* __restrict__ zero) {
+    const int per = F.per, Ncz = Cc.Nzg, xc = Cc.xc, yc = THREE ? Cc.yc : 0;
+    int clo, chi, dlo = 1, dhi = 1;
+    owned(r.ia, r.ib, F.Nxg, Cc.Nxg, 1 + xc, per, clo, chi);
+    if (THREE) owned(r.ja, r.jb, F.Nyg, Cc.Nyg, 1 + yc, 0, dlo, dhi);
+    const int nx = chi - clo + 1, ny = dhi - dlo + 1;
+    constexpr int P = 4;
+    const int part = threadIdx.x % P;
+    for (int cq = threadIdx.x / P; cq < nx * ny; cq += blockDim.x / P) {
+        const int cj = cq / nx, ic = clo + cq - cj * nx, jc = dlo + cj;
+        T* const ro = rc + (int64_t)Ncz * ((ic - 1) + Cc.Nxg * (jc - 1));
+        T* const zo = zero ? zero + (ro - rc) : nullptr;
+        const bool ghost = (!per && (ic == 1 || ic == Cc.Nxg)) || (THREE && (jc == 1 || jc == Cc.Nyg));
+        const int i = 2 + (ic - 2) * (1 + xc), j = THREE ? 2 + (jc - 2) * (1 + yc) : 1;
+        const int li = ghost ? 0 : i - r.ra, lj = ghost ? 0 : j - r.sa;
+        const T* const p = rs + slot(g, li, lj);
+        const int nl = near_l(g, li), nr = near_r(g, li), row = row_slot(g, 1);
+        // zero weight for ghost neighbours
+        const T wl = !per && i == 2 ? T(0) : T(0.25), wr = !per && i == F.Nxg - 1 ? T(0) : T(0.25);
+        const T wd = j == 2 ? T(0) : T(0.25), wu = j == F.Nyg - 1 ? T(0) : T(0.25);
+        auto xsum = [&](const T* q) -> T { return xc ? T(0.5) * q[0] + (wl * q[nl] + wr * q[nr]) : q[0]; };
+        auto plane = [&](int k) -> T {
+            const T* const q = p + k;
+            return yc ? T(0.5) * xsum(q) + (wd * xsum(q - row) + wu * xsum(q + row)) : xsum(q);
+        };
+        if (VEC && !Cc.zc && (Ncz & 1) == 0) {   // two rows at a time
+            for (int kc = 2 * part; kc < Ncz; kc += 2 * P) {
+                T v0 = 0, v1 = 0;
+                if (!ghost) {
+                    auto xsum2 = [&](const T* q, T& a, T& b) {
+                        const auto m = pair_at(q);
+                        if (!xc) { a = m.x; b = m.y; return; }
+                        const auto l = pair_at(q + nl), h = pair_at(q + nr);
+                        a = T(0.5) * m.x + (wl * l.x + wr * h.x);
+                        b = T(0.5) * m.y + (wl * l.y + wr * h.y);
+                    };
+                    xsum2(p + kc, v0, v1);
+                    if (yc) {
+                        T d0, d1, u0, u1;
+                        xsum2(p + kc - row, d0, d1);
+                        xsum2(p + kc + row, u0, u1);
+                        v0 = T(0.5) * v0 + (wd * d0 + wu * u0);
+                        v1 = T(0.5) * v1 + (wd * d1 + wu * u1);
+                    }
+                    if (kc == 0) v0 = 0;
+                    if (kc + 2 == Ncz) v1 = 0;
+                }
+                put_pair(ro + kc, v0, v1);
+                if (zo) put_pair(zo + kc, T(0), T(0));
+            }
+            continue;
+        }
+        for (int kc = part; kc < Ncz; kc += P) {
+            T v = 0;
+            if (!ghost && kc >= 1 && kc <= Ncz - 2) {
+                if (!Cc.zc) {
+                    v = plane(kc);
+                } else {
+                    const int k = 1 + (kc - 1) * 2;   // 0-based fine row
+                    const double dU = F.z[k + 1] - F.z[k], dD = F.z[k] - F.z[k - 1];
+                    const T h = T(0.5) * T(F.iz[k]);
+                    v = T(0.5) * plane(k);
+                    if (k > 1) v += h * T(dD) * plane(k - 1);
+                    if (k + 1 <= F.Nzg - 2) v += h * T(dU) * plane(k + 1);
+                }
+            }
+            ro[kc] = v;
+            if (zo) zo[kc] = T(0);
+        }
+    }
+    if (per && bx == 0) {   // the coarse image columns
+        for (int t = threadIdx.x; t < 3 * ny * Ncz; t += blockDim.x) {
+            const int cq = t / Ncz, k = t - cq * Ncz, jc = dlo + cq / 3, w = cq % 3;
+            const int col = w == 0 ? 1 : (w == 1 ? Cc.Nxg - 1 : Cc.Nxg);
+            const int o = k + Ncz * ((col - 1) + Cc.Nxg * (jc - 1));
+            rc[o] = T(0);
+            if (zero) zero[o] = T(0);
+        }
+    }
+}
+
+// Accessor of stage_up (sweep_n).
+template <typename T, bool THREE, bool VEC>
+struct UpAcc {
+    const T *b, *x, *xc;        // at column 1 of the region's first row, and the coarse field, at the thread's k
+    T *xs, *bs;
+    const LevelDev<T>& F;
+    const LevelDev<T>& Cc;
+    const TileGeo& g;
+    int ra, sa, k;
+    bool first, last;           // this k is the bottom row / ends in the free-surface row
+    template <int N>
+    __device__ __forceinline__ void avg(T* o, const T* c0, const T* c1, int i0, int i1) const {
+        T a[N], e[N];
+        get<N>(a, c0 + i0);
+        get<N>(e, c0 + i1);
+#pragma unroll
+        for (int n = 0; n < N; ++n) o[n] = a[n] + e[n];
+        if (THREE) {
+            get<N>(a, c1 + i0);
+            get<N>(e, c1 + i1);
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) o[n] = THREE ? T(0.25) * (o[n] + (a[n] + e[n])) : T(0.5) * o[n];
+    }
+    // v: N values of x, then N of b
+    template <int N>
+    __device__ __forceinline__ void ld(T* v, int c, int q) const {
+        const int i = gcol(ra + c, F.Nxg, F.per), j = sa + q;
+        const int e = F.Nzg * (i - 1 + F.Nxg * q);
+        get<N>(v, x + e);
+        get<N>(v + N, b + e);
+        if ((!F.per && (i == 1 || i == F.Nxg)) || (THREE && (j == 1 || j == F.Nyg))) return;
+        const int Ncz = Cc.Nzg;
+        int i0 = Cc.xc ? 1 + ((i - 2) >> 1) : i - 1;   // 0-based coarse columns
+        int i1 = Cc.xc ? i0 + (i & 1) : i0;
+        if (F.per && i1 == Cc.Nxg - 2) i1 = 1;
+        i0 *= Ncz;
+        i1 *= Ncz;
+        const int j0 = !THREE ? 0 : (Cc.yc ? 1 + ((j - 2) >> 1) : j - 1);
+        const T* const c0 = xc + Ncz * Cc.Nxg * j0;
+        const T* const c1 = c0 + (THREE && Cc.yc && (j & 1) ? Ncz * Cc.Nxg : 0);
+        T d[N];
+        if (!Cc.zc) {
+            avg<N>(d, c0, c1, i0, i1);
+            if (!first) v[0] += d[0];
+            if (N == 2) { if (!last) v[N - 1] += d[N - 1]; }
+            else if (last && !first) v[0] -= d[0];
+            return;
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const int kk = k + n;
+            if (kk < 1 || kk > F.Nzg - 2) continue;
+            const int z0 = __ldg(F.piz + 2 * kk) - 1, z1 = __ldg(F.piz + 2 * kk + 1) - 1;
+            avg<1>(d, c0 + z0, c1 + z0, i0, i1);
+            v[n] += __ldg(F.pwz + 2 * kk) * d[0];
+            const T w1 = __ldg(F.pwz + 2 * kk + 1);
+            if (w1 != T(0)) {
+                avg<1>(d, c0 + z1, c1 + z1, i0, i1);
+                v[n] += w1 * d[0];
+            }
+        }
+    }
+    template <int N>
+    __device__ __forceinline__ void st(int c, int q, const T* v) const {
+        const int s = slot(g, c, q);
+        put<N, VEC>(xs + s, v);
+        put<N, VEC>(bs + s, v + N);
+    }
+};
+
+// Stage the corrected iterate xin + P xc (MGProlongation3DExplicit.f90:19-110;
+// in x and y the average of the one, two or four coarse columns around a
+// point, in sigma by the level's table where the coarse grid is coarsened
+// there too; ghost columns, bottom and free-surface rows take no correction)
+// in xs and the right-hand side in bs.
+template <bool THREE, bool VEC, typename T>
+__device__ __forceinline__ void stage_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileGeo& g, const Reg& r,
+                                         const T* __restrict__ b, const T* __restrict__ xin, const T* __restrict__ xc,
+                                         T* xs, T* bs) {
+    const int64_t o = (int64_t)F.Nzg * F.Nxg * (r.sa - 1);
+    sweep<2, T, 2>(r.W, r.H, F.Nzg, [&](int k) {
+        const int end = k + ((F.Nzg & 1) == 0 ? 1 : 0);
+        return UpAcc<T, THREE, VEC>{b + o + k, xin + o + k, xc + (Cc.zc ? 0 : k), xs + k, bs + k, F, Cc, g, r.ra, r.sa, k,
+                                    k == 0, end == F.Nzg - 1};
+    });
+}
+
+// Accessor of stage_down (sweep_n).
+template <typename T, bool THREE, bool VEC>
+struct DownAcc {
+    const T* b;                 // at the thread's k
+    T *xs, *bs;
+    const TileGeo& g;
+    const T (*gx)[3], (*gy)[3];
+    int ra, sa, Nxg, Nyg, per, nz;
+    bool first;                 // this k is the bottom row
+    template <int N>
+    __device__ __forceinline__ void ld(T* v, int c, int q) const {
+        get<N>(v, b + nz * (gcol(ra + c, Nxg, per) - 1 + Nxg * q));
+    }
+    template <int N>
+    __device__ __forceinline__ void st(int c, int q, const T* v) const {
+        const int s = slot(g, c, q), i = ra + c, j = sa + q;
+        put<N, VEC>(bs + s, v);
+        T x[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) x[n] = T(0);
+        const bool x0 = !per && i == 1, x1 = !per && i == Nxg, y0 = THREE && j == 1, y1 = THREE && j == Nyg;
+        if (x0 || x1 || y0 || y1) {
+            const T w = (x0 || x1) && (y0 || y1) ? T(1) : (gx ? (x0 || x1 ? gx[x1][2] : gy[y1][2]) : T(0));
+#pragma unroll
+            for (int n = 0; n < N; ++n) x[n] = first && n == 0 ? v[n] : w * v[n];
+        }
+        put<N, VEC>(xs + s, x);
+    }
+};
+
+// Stage the right-hand side in bs and in xs the zero iterate with its identity
+// rows (corner columns, level 1 of the ghost columns: b) and, gx[w][2] and
+// gy[w][2] being one over the ghost weight of wall w, its ghost rows relaxed
+// (null: left at zero).
+template <bool THREE, bool VEC, typename T>
+__device__ __forceinline__ void stage_down(const LevelDev<T>& F, const TileGeo& g, const Reg& r,
+                                           const T* __restrict__ b, T* xs, T* bs, const T (*gx)[3], const T (*gy)[3]) {
+    const int64_t o = (int64_t)F.Nzg * F.Nxg * (r.sa - 1);
+    sweep<4, T, 1>(r.W, r.H, F.Nzg, [&](int k) {
+        return DownAcc<T, THREE, VEC>{b + o + k, xs + k, bs + k, g, gx, gy, r.ra, r.sa, F.Nxg, F.Nyg, F.per, F.Nzg, k == 0};
+    });
+}
+
+// Accessor of write_core (sweep_n).
+template <typename T, bool VEC>
+struct CoreAcc {
+    const T* xs;                // at the thread's k
+    T* out;                     // at the core's first column and the thread's k
+    const TileGeo& g;
+    int c0, q0, nz, Nxg;
+    template <int N>
+    __device__ __forceinline__ void ld(T* v, int c, int q) const {
+        const T* const p = xs + slot(g, c + c0, q + q0);
+        if constexpr (N == 2 && VEC) {
+            get<2>(v, p);
+        } else {
+#pragma unroll
+            for (int n = 0; n < N; ++n) v[n] = p[n];
+        }
+    }
+    template <int N>
+    __device__ __forceinline__ void st(int c, int q, const T* v) const {
+        put<N, true>(out + nz * (c + Nxg * q), v);
+    }
+};
+
+// Write the core columns of the staged array (periodic x: and zeros in the
+// image columns).
+template <bool THREE, bool VEC, typename T>
+__device__ __forceinline__ void write_core(const LevelDev<T>& F, const Reg& r, const TileGeo& g, int bx, const T* xs,
+                                           T* __restrict__ out) {
+    const int Nzg = F.Nzg, Nxg = F.Nxg, H = r.jb - r.ja + 1;
+    T* const o = out + (int64_t)Nzg * ((r.ia - 1) + (int64_t)Nxg * (r.ja - 1));
+    sweep<4, T, 1>(r.ib - r.ia + 1, H, Nzg, [&](int k) {
+        return CoreAcc<T, VEC>{xs + k, o + k, g, r.ia - r.ra, r.ja - r.sa, Nzg, Nxg};
+    });
+    if (F.per && bx == 0)
+        for (int t = threadIdx.x; t < 3 * H * Nzg; t += blockDim.x) {
+            const int cq = t / Nzg, k = t - cq * Nzg, w = cq % 3;
+            const int col = w == 0 ? 1 : (w == 1 ? Nxg - 1 : Nxg);
+            out[k + Nzg * ((col - 1) + Nxg * (r.ja + cq / 3 - 1))] = T(0);
+        }
+}
+
+// ----------------------------------------------------------- uniform levels
+
+// A uniform column's rows lie in pairs (even pitch): every access of the
+// column code below moves two rows, half the shared-memory instructions.
+// Pitch / 2 is odd, so that the pairs of neighbouring columns, which the
+// threads of a warp take together, fall on different banks.
+
+// Neighbour columns' part of rows k and k + 1.
+template <bool THREE, typename T>
+__device__ __forceinline__ void uni_off(const UniTab<T>& u, const T* xp, int l, int r, int row, int k, T* o) {
+    const auto a = pair_at(xp + l + k), b = pair_at(xp + r + k);
+    o[0] = u.wxl * a.x + u.wxr * b.x;
+    o[1] = u.wxl * a.y + u.wxr * b.y;
+    if (THREE) {
+        const auto d = pair_at(xp - row + k), e = pair_at(xp + row + k);
+        o[0] += u.wyd * d.x + u.wyu * e.x;
+        o[1] += u.wyd * d.y + u.wyu * e.y;
+    }
+}
+
+// Rows 2..Nzg-1 of the column at xp bottom to top, then its bottom row and
+// its free-surface row: x_k = (b_k - off_k - up_k x_{k+1}) id_k - g_k x_{k-1}.
+// All rows' sums are formed before the first new value is stored, so their
+// loads are in flight together and only the chain's one multiply-add per row
+// is serial. off(k, o): the neighbour columns' part of rows k, k + 1; ZERO: the
+// column's own old iterate is zero.
+template <int NZG, bool ZERO, typename T, typename OFF>
+__device__ __forceinline__ void uni_column(const UniTab<T>& u, int nzg, T* xp, const T* bp, OFF off) {
+    const int Nzg = NZG > 0 ? NZG : nzg;
+    constexpr int CH = NZG > 0 ? (NZG + 1) / 2 * 2 : 8;   // rows per chunk
+    const T b1 = bp[0];
+    T xprev = ZERO ? b1 * u.t6 : (b1 - u.t0 * xp[1] - u.t1 * xp[2]) * u.t6;
+    T x2 = 0, x3 = 0;
+    for (int k0 = 0; k0 < Nzg; k0 += CH) {
+        T q[CH], xo[CH + 1];
+        if (!ZERO) {
+#pragma unroll
+            for (int m = 0; m < CH; m += 2)
+                if (NZG > 0 || k0 + m < Nzg) { const auto v = pair_at(xp + k0 + m); xo[m] = v.x; xo[m + 1] = v.y; }
+            xo[CH] = NZG == 0 && k0 + CH < Nzg ? xp[k0 + CH] : T(0);
+        }
+#pragma unroll
+        for (int m = 0; m < CH; m += 2) {
+            if (NZG == 0 && k0 + m >= Nzg) continue;
+            const auto v = pair_at(bp + k0 + m);
+            T o[2];
+            off(k0 + m, o);
+            q[m] = v.x; q[m + 1] = v.y;
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int k = k0 + m + n;
+                if (k >= 1 && k < Nzg - 1)
+                    q[m + n] = ((ZERO ? q[m + n] : q[m + n] - u.up[k] * xo[m + n + 1]) - o[n]) * u.id[k];
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < CH; ++m) {
+            const int k = k0 + m;
+            if (k >= 1 && k < Nzg - 1) {
+                xprev = q[m] - u.g[k] * xprev;
+                q[m] = xprev;
+                if (k == 1) x2 = xprev;
+                if (k == 2) x3 = xprev;
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < CH; m += 2)
+            if (NZG > 0 || k0 + m < Nzg) put_pair(xp + k0 + m, q[m], q[m + 1]);   // the free-surface row: b
+    }
+    xp[0] = (b1 - u.t0 * x2 - u.t1 * x3) * u.t6;
+}
+
+// Replace the right-hand side of the column's rows 2..Nzg-1 by the residual.
+template <bool THREE, int NZG, typename T>
+__device__ __forceinline__ void uni_residual(const UniTab<T>& u, int nzg, const T* xp, T* bp, int l, int r, int row) {
+    const int Nzg = NZG > 0 ? NZG : nzg;
+    constexpr int CH = NZG > 0 ? (NZG + 1) / 2 * 2 : 8;
+    T xm = 0;
+    for (int k0 = 0; k0 < Nzg; k0 += CH) {
+        T x[CH + 2];            // rows k0 - 1 .. k0 + CH
+        x[0] = xm;
+#pragma unroll
+        for (int m = 0; m < CH; m += 2)
+            if (NZG > 0 || k0 + m < Nzg) { const auto v = pair_at(xp + k0 + m); x[m + 1] = v.x; x[m + 2] = v.y; }
+        x[CH + 1] = NZG == 0 && k0 + CH < Nzg ? xp[k0 + CH] : T(0);
+        xm = x[CH];
+#pragma unroll
+        for (int m = 0; m < CH; m += 2) {
+            if (NZG == 0 && k0 + m >= Nzg) continue;
+            const auto v = pair_at(bp + k0 + m);
+            T q[2] = {v.x, v.y}, o[2];
+            uni_off<THREE>(u, xp, l, r, row, k0 + m, o);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int k = k0 + m + n, i = m + n + 1;
+                if (k >= 1 && k < Nzg - 1) q[n] -= o[n] + u.lo[k] * x[i - 1] + u.up[k] * x[i + 1] + u.dg[k] * x[i];
+            }
+            put_pair(bp + k0 + m, q[0], q[1]);
+        }
+    }
+}
+
+// One smoothing step on the staged iterate: colour c at distance <= d - c,
+// the ghost rows relaxed before, between and after. ZERO: the iterate is zero
+// and its ghost rows are relaxed; colour 0 then reads no neighbour columns but
+// ghosts, so it may reach the region's edge.
+template <bool THREE, int NZG, bool ZERO, typename T>
+__device__ __forceinline__ void uni_smooth(const LevelDev<T>& F, const UniTab<T>& u, const TileGeo& g, const Reg& r,
+                                           T* xs, const T* bs, int d) {
+    const int Nxg = F.Nxg, Nyg = F.Nyg, per = F.per;
+    const bool wall = at_wall(Nxg, Nyg, per, r, THREE);
+    auto ghosts = [&]() {
+        if (!wall) return;
+        ghost_pairs<THREE>(Nxg, Nyg, per, r, g, [&](int s, int sa, int sb, bool xw, int side, int k) {
+            const T* const w = xw ? u.gx[side] : u.gy[side];
+            const auto b = pair_at(bs + s), a = pair_at(xs + sa), c = pair_at(xs + sb);
+            const T v0 = (b.x - w[0] * a.x - w[1] * c.x) * w[2], v1 = (b.y - w[0] * a.y - w[1] * c.y) * w[2];
+            put_pair(xs + s, k == 0 ? b.x : v0, v1);   // level 1: an identity row
+        });
+        __syncthreads();
+    };
+    if (!ZERO) ghosts();
+    const int row = row_slot(g, 1);
+    for (int colour = 0; colour < 2; ++colour) {
+        colour_columns<THREE>(Nxg, Nyg, per, r, 2, colour, d - colour, [&](int i, int j) {
+            const int li = i - r.ra, s = slot(g, li, j - r.sa), l = near_l(g, li), h = near_r(g, li);
+            T* const xp = xs + s;
+            if (ZERO && colour == 0) {
+                const bool el = !per && i == 2, er = !per && i == Nxg - 1;
+                const bool ed = THREE && j == 2, eu = THREE && j == Nyg - 1;
+                if (el || er || ed || eu) {
+                    uni_column<NZG, true>(u, F.Nzg, xp, bs + s, [&](int k, T* o) {
+                        o[0] = o[1] = T(0);
+                        auto add = [&](bool on, T w, int at) {
+                            if (!on) return;
+                            const auto v = pair_at(xp + at + k);
+                            o[0] += w * v.x;
+                            o[1] += w * v.y;
+                        };
+                        add(el, u.wxl, l);
+                        add(er, u.wxr, h);
+                        add(ed, u.wyd, -row);
+                        add(eu, u.wyu, row);
+                    });
+                } else {
+                    uni_column<NZG, true>(u, F.Nzg, xp, bs + s, [&](int, T* o) { o[0] = o[1] = T(0); });
+                }
+                return;
+            }
+            uni_column<NZG, ZERO>(u, F.Nzg, xp, bs + s, [&](int k, T* o) { uni_off<THREE>(u, xp, l, h, row, k, o); });
+        });
+        __syncthreads();
+        ghosts();
+    }
+}
+
+template <typename T, bool THREE, int NZG>
+__global__ void __launch_bounds__(256, 2) k_mg_down_uni(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
+                                                     T* __restrict__ xout, T* __restrict__ rc, T* __restrict__ zero,
+                                                     const __grid_constant__ UniTab<T> u, TileGeo g) {
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    T* const xs = reinterpret_cast<T*>(tile_smem);
+    T* const bs = xs + 2 * g.HW * g.PH * g.NZP;
+    const int bx = blockIdx.x, by = blockIdx.y;
+    const Reg r = region(F.Nxg, F.Nyg, F.per, g, bx, by, THREE);
+    stage_down<THREE, true>(F, g, r, b, xs, bs, u.gx, u.gy);
+    __syncthreads();
+    uni_smooth<THREE, NZG, true>(F, u, g, r, xs, bs, 3);
+    write_core<THREE, true>(F, r, g, bx, xs, xout);
+    const int row = row_slot(g, 1);
+    all_columns<THREE>(F.Nxg, F.Nyg, F.per, r, 1, [&](int i, int j) {
+        const int li = i - r.ra, s = slot(g, li, j - r.sa);
+        uni_residual<THREE, NZG>(u, F.Nzg, xs + s, bs + s, near_l(g, li), near_r(g, li), row);
+    });
+    __syncthreads();
+    restrict_tile<THREE, true>(F, Cc, g, r, bx, bs, rc, zero);
+}
+
+template <typename T, bool THREE, int NZG>
+__global__ void __launch_bounds__(256, 2) k_mg_up_uni(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
+                                                   const T* __restrict__ xin, const T* __restrict__ xc,
+                                                   T* __restrict__ out, const __grid_constant__ UniTab<T> u, TileGeo g) {
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    T* const xs = reinterpret_cast<T*>(tile_smem);
+    T* const bs = xs + 2 * g.HW * g.PH * g.NZP;
+    const int bx = blockIdx.x, by = blockIdx.y;
+    const Reg r = region(F.Nxg, F.Nyg, F.per, g, bx, by, THREE);
+    stage_up<THREE, true>(F, Cc, g, r, b, xin, xc, xs, bs);
+    __syncthreads();
+    uni_smooth<THREE, NZG, false>(F, u, g, r, xs, bs, 1);
+    write_core<THREE, true>(F, r, g, bx, xs, out);
+}
+
+// ------------------------------------------------------------- cross levels
+
+// The mixed derivatives d2/dxds (replicated over three y planes) and d2/dyds
+// (over three x planes) of row k are om_k sum_m z_m D(k-1+m) with one
+// horizontal 9-point sum per level
+//   D(k) = sum_ab 2 (ca sx_a + cb sy_b) x(i-1+a, j-1+b, k),
+// the factors ca = h_x/h, cb = h_y/h taken out of the sums (54 products per
+// row as the two sums are written, 9 this way).
+template <typename T, bool THREE>
+struct CrossCol {
+    T ih, ca, cb, c3;           // 1/h, h_x/h, h_y/h and the sigma-3 factor
+    T W[THREE ? 9 : 3];
+    __device__ __forceinline__ CrossCol(const T* cf, const RowTab<T>& t) : ih(cf[0]), ca(cf[1]), cb(cf[2]), c3(cf[3]) {
+#pragma unroll
+        for (int b = 0; b < (THREE ? 3 : 1); ++b)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                W[3 * b + a] = T(2) * ca * t.sx1[a];
+                if (THREE) W[3 * b + a] += T(2) * cb * t.sy1[b];
+            }
+    }
+    __device__ __forceinline__ T centre() const { return W[THREE ? 4 : 1]; }
+    // row coefficients below, on and above the diagonal without the mixed terms
+    __device__ __forceinline__ void row(const RowTab<T>& t, int k, T& lo, T& dg, T& up) const {
+        const T om = t.om[k], s3 = om * c3, cz = om * om * (ca * ca + cb * cb) + ih * ih;
+        lo = s3 * t.z0[k] + cz * t.y0[k];
+        dg = s3 * t.z1[k] + cz * t.y1[k] + t.sx2[1] + (THREE ? t.sy2[1] : T(0));
+        up = s3 * t.z2[k] + cz * t.y2[k];
+    }
+};
+
+// Staged arrays of a cross tile: the columns' coefficients ([slot][4]), the
+// iterate, and the right-hand side (replaced by the residual on the way down).
+template <typename T>
+struct CrossTile {
+    T *cf, *xs, *bs;
+};
+
+// D(k) without the own column at p = the column's row k; off: the axis
+// neighbours' part of the row (d2/dx2, d2/dy2).
+template <typename T, bool THREE>
+__device__ __forceinline__ T cross_sum(const CrossCol<T, THREE>& c, const RowTab<T>& t, const T* p, int nl, int nr,
+                                       int nrow, T& off) {
+    const T xl = p[nl], xr = p[nr];
+    off = t.sx2[0] * xl + t.sx2[2] * xr;
+    if (!THREE) return c.W[0] * xl + c.W[2] * xr;
+    const T xd = p[-nrow], xu = p[nrow];
+    off += t.sy2[0] * xd + t.sy2[2] * xu;
+    return (c.W[0] * p[nl - nrow] + c.W[1] * xd + c.W[2] * p[nr - nrow]) + (c.W[3] * xl + c.W[5] * xr) +
+           (c.W[6] * p[nl + nrow] + c.W[7] * xu + c.W[8] * p[nr + nrow]);
+}
+
+// D(1), the level below the bottom, the own column included, next to a wall:
+// its stencils are shifted off the ghost corner columns.
+template <typename T, bool THREE>
+__device__ T cross_level1(const CrossCol<T, THREE>& c, const RowTab<T>& t, const TileGeo& g, const T* xs, int Nxg,
+                          int Nyg, int i, int j, int li, int lj) {
+    const int sh = i == 2 ? 1 : (i == Nxg - 1 ? -1 : 0);
+    const int shy = !THREE ? 0 : (j == 2 ? 1 : (j == Nyg - 1 ? -1 : 0));
+    const T* const wx = sh == 0 ? t.sx1 : t.ex[sh > 0 ? 0 : 1];
+    T vx = 0, vy = 0;
+    for (int b = (THREE ? -1 : 0); b <= (THREE ? 1 : 0); ++b)
+        for (int a = 0; a < 3; ++a) vx += wx[a] * xs[slot(g, li - 1 + sh + a, lj + b)];
+    if (THREE) {
+        const T* const wy = shy == 0 ? t.sy1 : t.ey[shy > 0 ? 0 : 1];
+        for (int a = -1; a <= 1; ++a)
+            for (int b = 0; b < 3; ++b) vy += wy[b] * xs[slot(g, li + a, lj - 1 + shy + b)];
+    }
+    return T(2) * c.ca * vx + T(2) * c.cb * vy;
+}
+
+// Columns of `colour` at distance <= d of the core, one per segment of S
+// lanes, lane r holding rows 1+2r and 2+2r (0-based): the sums of a column's
+// rows are formed by its lanes together, and the chain over the rows is a
+// shuffle scan of the lanes' composed maps x -> a x + b. (One thread per
+// column instead: 31-33 us per launch at any level size, the latency of 8
+// rows one after another per colour.) RES: replace the right-hand side by the
+// residual instead of solving.
+template <typename T, bool THREE, int S, bool RES>
+__device__ __forceinline__ void cross_pass(const LevelDev<T>& F, const RowTab<T>& t, const TileGeo& g, const Reg& r,
+                                           const CrossTile<T>& w, int ncolor, int colour, int d) {
+    const int Nxg = F.Nxg, Nyg = F.Nyg, Nzg = F.Nzg;
+    const int ilo = max(r.ia - d, 2), ihi = min(r.ib + d, Nxg - 1);
+    int jlo = 1, jhi = 1, js = 1;
+    if (THREE) { jlo = max(r.ja - d, 2); jhi = min(r.jb + d, Nyg - 1); }
+    const bool four = ncolor == 4;
+    if (!RES && THREE && four) { jlo += (jlo ^ (colour >> 1)) & 1; js = 2; }
+    const int ni = RES ? max(ihi - ilo + 1, 0) : (ihi - ilo + 2) >> 1, nj = jhi >= jlo ? (jhi - jlo) / js + 1 : 0;
+    const int total = ni * nj, lane = threadIdx.x & 31, rr = lane & (S - 1);
+    const int per_warp = 32 / S, step = (blockDim.x >> 5) * per_warp;
+    const int ka = 1 + 2 * rr, kb = ka + 1;
+    const int kac = min(ka, Nzg - 1), kbc = min(kb, Nzg - 1);
+    const int nrow = row_slot(g, 1);
+    for (int base = (threadIdx.x >> 5) * per_warp; base < total; base += step) {
+        const int q = base + lane / S;
+        const int tq = min(q, total - 1), tj = tq / ni, j = jlo + tj * js;
+        const int par = four ? colour & 1 : (colour + j) & 1;
+        int i = RES ? ilo + tq - tj * ni : ilo + ((ilo ^ par) & 1) + 2 * (tq - tj * ni);
+        const bool act = q < total && i <= ihi;
+        if (i > ihi) i = ihi;                       // an idle segment reads a column in range
+        const int li = i - r.ra, lj = j - r.sa;
+        const int cs = (lj * 2 + (li & 1)) * g.HW + (li >> 1), s = cs * g.NZP;
+        const int nl = near_l(g, li), nr = near_r(g, li);
+        const CrossCol<T, THREE> c(w.cf + 4 * cs, t);
+        T* const p = w.xs + s;
+        T* const bp = w.bs + s;
+        const T wc = c.centre();
+        T offa, offb, offx;
+        T Da = cross_sum<T, THREE>(c, t, p + kac, nl, nr, nrow, offa);
+        T Db = cross_sum<T, THREE>(c, t, p + kbc, nl, nr, nrow, offb);
+        // lane 0: the level below the bottom; the last row's lane: the free surface
+        const int kx = rr == 0 ? 0 : Nzg - 1;
+        T Dx = cross_sum<T, THREE>(c, t, p + kx, nl, nr, nrow, offx);
+        if (rr == 0) {
+            if (i == 2 || i == Nxg - 1 || (THREE && (j == 2 || j == Nyg - 1)))
+                Dx = cross_level1<T, THREE>(c, t, g, w.xs, Nxg, Nyg, i, j, li, lj);
+            else
+                Dx += wc * p[0];
+        }
+        if (RES) {
+            Da += wc * p[kac];
+            Db += wc * p[kbc];
+            if (rr != 0) Dx += wc * p[kx];
+        }
+        T Dm = __shfl_up_sync(0xffffffffu, Db, 1, S), Dn = __shfl_down_sync(0xffffffffu, Da, 1, S);
+        if (rr == 0) Dm = Dx;
+        if (kb == Nzg - 2) Dn = Dx;
+        const T xka = p[kac], xkb = p[kbc], xkn = p[min(kb + 1, Nzg - 1)];
+        const int ra = min(ka, Nzg - 2), rb = min(kb, Nzg - 2);   // row constants
+        T loa, dga, upa, lob, dgb, upb;
+        c.row(t, ra, loa, dga, upa);
+        c.row(t, rb, lob, dgb, upb);
+        const T oma = t.om[ra], omb = t.om[rb];
+        T fa = bp[kac] - offa - oma * (t.z0[ra] * Dm + t.z1[ra] * Da + t.z2[ra] * Db);
+        T fb = bp[kbc] - offb - omb * (t.z0[rb] * Da + t.z1[rb] * Db + t.z2[rb] * Dn);
+        if (RES) {
+            if (act) {
+                if (ka <= Nzg - 2) bp[ka] = fa - loa * p[kac - 1] - dga * xka - upa * xkb;
+                if (kb <= Nzg - 2) bp[kb] = fb - lob * xka - dgb * xkb - upb * xkn;
+            }
+        } else {
+            // the own column's mixed terms join the chain (row 2's lower one is in D(1))
+            const T wa = oma * wc, wb = omb * wc;
+            if (rr != 0) loa += wa * t.z0[ra];
+            dga += wa * t.z1[ra]; upa += wa * t.z2[ra];
+            lob += wb * t.z0[rb]; dgb += wb * t.z1[rb]; upb += wb * t.z2[rb];
+            const T ida = T(1) / dga, idb = T(1) / dgb;
+            const T qa = (fa - upa * xkb) * ida, ga = loa * ida;
+            const T qb = (fb - upb * xkn) * idb, gb = lob * idb;
+            const bool va = ka <= Nzg - 2, vb = kb <= Nzg - 2;
+            T a = 1, bb = 0;
+            if (va) { bb = qa; a = -ga; }
+            if (vb) { bb = qb - gb * bb; a = -gb * a; }
+#pragma unroll
+            for (int dd = 1; dd < S; dd <<= 1) {
+                const T ap = __shfl_up_sync(0xffffffffu, a, dd, S);
+                const T bq = __shfl_up_sync(0xffffffffu, bb, dd, S);
+                if (rr >= dd) { bb = a * bq + bb; a = a * ap; }
+            }
+            const T ae = __shfl_up_sync(0xffffffffu, a, 1, S), be = __shfl_up_sync(0xffffffffu, bb, 1, S);
+            const T x1 = p[0];                       // the bottom row is fixed during the pass
+            const T xin = rr == 0 ? x1 : ae * x1 + be;
+            const T xa = qa - ga * xin, xb = qb - gb * xa;
+            const T xf = bp[Nzg - 1];
+            __syncwarp();
+            if (act) {
+                if (va) p[ka] = xa;
+                if (vb) p[kb] = xb;
+                if (rr == 0) p[Nzg - 1] = xf;
+            }
+        }
+    }
+}
+
+// Bottom row (k = 1) of every interior column at distance <= d, from its rows
+// 2, 3 and the neighbours' row 2 (BuildLinearSystemMatrix.f90:50-70, the row
+// times 1/h). FIRST: the iterate is zero.
+template <typename T, bool THREE, bool FIRST>
+__device__ __forceinline__ void cross_bottoms(const LevelDev<T>& F, const RowTab<T>& t, const TileGeo& g, const Reg& r,
+                                              const CrossTile<T>& w, int d) {
+    const int Nxg = F.Nxg, Nyg = F.Nyg, nrow = row_slot(g, 1);
+    all_columns<THREE>(Nxg, Nyg, 0, r, d, [&](int i, int j) {
+        const int li = i - r.ra, lj = j - r.sa;
+        const int cs = (lj * 2 + (li & 1)) * g.HW + (li >> 1), s = cs * g.NZP;
+        const T ih = w.cf[4 * cs], ca = w.cf[4 * cs + 1], cb = w.cf[4 * cs + 2];
+        const T f = ih * ih + t.om[1] * (ca * ca + cb * cb);
+        T* const p = w.xs + s;
+        T v = w.bs[s] * ih;
+        if (!FIRST) {
+            const T* const p2 = p + 1;
+            v -= f * (t.z1[1] * p[1] + t.z2[1] * p[2]) +
+                 ca * (t.sx1[0] * p2[near_l(g, li)] + t.sx1[1] * p[1] + t.sx1[2] * p2[near_r(g, li)]);
+            if (THREE) v -= cb * (t.sy1[0] * p2[-nrow] + t.sy1[1] * p[1] + t.sy1[2] * p2[nrow]);
+        }
+        p[0] = v / (f * t.z0[1]);
+    });
+    __syncthreads();
+}
+
+// Relax ghost rows from the current values: those whose stencil holds a
+// column of colour `post` (just solved) and those next to a column of colour
+// `pre` (to be solved, which reads them).
+template <typename T, bool THREE>
+__device__ __forceinline__ void cross_ghosts(const LevelDev<T>& F, const RowTab<T>& t, const Reg& r, const TileGeo& g,
+                                             const CrossTile<T>& w, int ncolor, int post, int pre) {
+    ghost_rows<THREE>(F.Nxg, F.Nyg, 0, F.Nzg, F.mz32, F.sz32, r, g, [&](int s, int sa, int sb, int ni, int nj, bool xw,
+                                                                        int side) {
+        auto has = [&](int i, int j, int colour) {
+            return ncolor == 4 ? ((i & 1) == (colour & 1) && (j & 1) == (colour >> 1)) : ((i + j) & 1) == colour;
+        };
+        const int di = xw ? (side ? -1 : 1) : 0, dj = xw ? 0 : (side ? -1 : 1);
+        const bool a = post >= 0 && (has(ni, nj, post) || has(ni + di, nj + dj, post));
+        if (!a && !(pre < ncolor && has(ni, nj, pre))) return;
+        const T* const gw = xw ? t.gx[side] : t.gy[side];
+        w.xs[s] = (w.bs[s] - gw[0] * w.xs[sa] - gw[1] * w.xs[sb]) * gw[2];
+    });
+    __syncthreads();
+}
+
+// The colours of one smoothing step on the staged iterate (colour c at
+// distance <= d1 - c), then the bottom rows at <= d2.
+template <typename T, bool THREE, int S>
+__device__ __forceinline__ void cross_smooth(const LevelDev<T>& F, const RowTab<T>& t, const TileGeo& g, const Reg& r,
+                                             const CrossTile<T>& w, int d1, int d2) {
+    const int nc = F.ncolor;
+    const bool wall = at_wall(F.Nxg, F.Nyg, 0, r, THREE);
+    if (wall) cross_ghosts<T, THREE>(F, t, r, g, w, nc, -1, 0);
+    for (int c = 0; c < nc; ++c) {
+        cross_pass<T, THREE, S, false>(F, t, g, r, w, nc, c, d1 - c);
+        __syncthreads();
+        if (wall) cross_ghosts<T, THREE>(F, t, r, g, w, nc, c, c + 1);
+    }
+    cross_bottoms<T, THREE, false>(F, t, g, r, w, d2);
+}
+
+template <typename T>
+__device__ __forceinline__ CrossTile<T> cross_arrays(const TileGeo& g, T* sm) {
+    const int cols = 2 * g.HW * g.PH;
+    return CrossTile<T>{sm, sm + 4 * cols, sm + (4 + g.NZP) * cols};
+}
+template <bool THREE, typename T>
+__device__ __forceinline__ void stage_cf(const LevelDev<T>& F, const TileGeo& g, const Reg& r, T* cf) {
+    for (int q = threadIdx.x; q < r.W * r.H; q += blockDim.x) {
+        const int lj = q / r.W, li = q - lj * r.W;
+        T a, b, c, d;
+        load_cf(F.cf, (int64_t)(r.ra + li - 1) + (int64_t)F.Nxg * (r.sa + lj - 1), a, b, c, d);
+        T* const o = cf + 4 * ((lj * 2 + (li & 1)) * g.HW + (li >> 1));
+        o[0] = a; o[1] = b; o[2] = THREE ? c : T(0); o[3] = d;
+    }
+}
+
+template <typename T, bool THREE, int S>
+__global__ void __launch_bounds__(kCrossThreads) k_mg_down_cross(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
+                                                                 T* __restrict__ xout, T* __restrict__ rc,
+                                                                 T* __restrict__ zero,
+                                                                 const __grid_constant__ RowTab<T> t, TileGeo g) {
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    const CrossTile<T> w = cross_arrays(g, reinterpret_cast<T*>(tile_smem));
+    const int nc = F.ncolor, bx = blockIdx.x, by = blockIdx.y;
+    const Reg r = region(F.Nxg, F.Nyg, 0, g, bx, by, THREE);
+    stage_cf<THREE>(F, g, r, w.cf);
+    stage_down<THREE, false>(F, g, r, b, w.xs, w.bs, (const T(*)[3])nullptr, (const T(*)[3])nullptr);
+    __syncthreads();
+    cross_bottoms<T, THREE, true>(F, t, g, r, w, g.halo);
+    cross_smooth<T, THREE, S>(F, t, g, r, w, nc + 2, 2);
+    write_core<THREE, false>(F, r, g, bx, w.xs, xout);
+    cross_pass<T, THREE, S, true>(F, t, g, r, w, nc, 0, 1);
+    __syncthreads();
+    restrict_tile<THREE, false>(F, Cc, g, r, bx, w.bs, rc, zero);
+}
+
+template <typename T, bool THREE, int S>
+__global__ void __launch_bounds__(kCrossThreads) k_mg_up_cross(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
+                                                               const T* __restrict__ xin, const T* __restrict__ xc,
+                                                               T* __restrict__ out,
+                                                               const __grid_constant__ RowTab<T> t, TileGeo g) {
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    const CrossTile<T> w = cross_arrays(g, reinterpret_cast<T*>(tile_smem));
+    const int nc = F.ncolor, bx = blockIdx.x, by = blockIdx.y;
+    const Reg r = region(F.Nxg, F.Nyg, 0, g, bx, by, THREE);
+    stage_cf<THREE>(F, g, r, w.cf);
+    stage_up<THREE, false>(F, Cc, g, r, b, xin, xc, w.xs, w.bs);
+    __syncthreads();
+    cross_bottoms<T, THREE, false>(F, t, g, r, w, nc + 1);
+    cross_smooth<T, THREE, S>(F, t, g, r, w, nc, 0);
+    write_core<THREE, false>(F, r, g, bx, w.xs, out);
+}
+
+// ------------------------------------------------------------ host side
+
+// Column pitch in shared memory. Cross levels, whose lanes take rows of a
+// column one by one: odd. Uniform levels, two rows at a time: twice an odd
+// number.
+inline int tile_pitch(int nzg, bool cross) { return cross ? nzg | 1 : ((nzg + 1) / 2 | 1) * 2; }
+
+// Cores, slots and shared memory of a launch over all its tiles.
+template <typename T>
+void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross) {
+    const bool three = L.Nyg > 1;
+    auto cores = [](int n, int c, int& nt, int& q, int& rem, int& most) {
+        nt = (n + c - 1) / c;
+        if (n / nt < 3) nt = n / 3;      // n >= 4 columns on every level
+        q = n / nt;
+        rem = n - q * nt;
+        most = q + (rem > 0 ? 1 : 0);
+    };
+    cores(L.per ? L.Nxg - 3 : L.Nxg, cx, g.ntx, g.qx, g.remx, g.cx);
+    if (three) cores(L.Nyg, cy, g.nty, g.qy, g.remy, g.cy);
+    else { g.nty = 1; g.qy = 1; g.remy = 0; g.cy = 1; }
+    g.NZP = tile_pitch(L.Nzg, cross);
+    g.np = (L.Nzg + 1) / 2;
+    div_magic32((uint32_t)g.np, g.mnp, g.snp);
+    int W = 0, H = 0;
+    for (int bx = 0; bx < g.ntx; ++bx) W = std::max(W, region(L.Nxg, L.Nyg, L.per, g, bx, 0, three).W);
+    for (int by = 0; by < g.nty; ++by) H = std::max(H, region(L.Nxg, L.Nyg, L.per, g, 0, by, three).H);
+    g.HW = (W + 1) / 2;
+    g.PH = H;
+    const size_t cols = (size_t)2 * g.HW * g.PH;
+    g.smem = (cols * g.NZP * 2 + (cross ? 4 * cols : 0)) * sizeof(T);   // iterate, right-hand side, coefficients
+}
+
+}  // namespace
+
+template <typename T>
+void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
+    const bool three = L.Nyg > 1, cross = t.mode == kTileCross;
+    // The largest core that leaves room for two blocks per SM, on levels with
+    // at least a tile per SM of that size; smaller levels take smaller cores.
+    static const int uni3[][2] = {{32, 8}, {16, 8}, {8, 4}}, cross3[][2] = {{16, 16}, {16, 8}, {8, 8}, {4, 4}};
+    static const int line[][2] = {{64, 1}, {32, 1}, {16, 1}};
+    const int (*cand)[2] = three ? (cross ? cross3 : uni3) : line;
+    const int ncand = three && cross ? 4 : 3;
+    auto pick = [&](TileGeo& g, int halo) {
+        g.halo = halo;
+        bool found = false;
+        TileGeo best{};
+        for (int q = 0; q < ncand; ++q) {
+            size_geo(L, g, cand[q][0], cand[q][1], cross);
+            if (g.smem > kTileSmemMax || (g.smem > kTileSmemTwo && q + 1 < ncand)) continue;
+            const int lanes = cross ? (L.Nzg <= 10 ? 4 : (L.Nzg <= 18 ? 8 : 16)) : 1;
+            const int cols = (g.cx + 2 * halo) * (three ? g.cy + 2 * halo : 1) / L.ncolor * lanes;
+            g.threads = std::max(256, std::min(cross ? kCrossThreads : 256, (cols + 31) / 32 * 32));
+            found = true;
+            best = g;
+            if (g.ntx * g.nty >= 148) break;
+        }
+        g = best;
+        return found;
+    };
+    if (t.mode == kTileNone) return;
+    const int nc = L.ncolor;
+    if (!pick(t.down, cross ? nc + 3 : 3) || !pick(t.up, cross ? nc + 2 : 2)) t.mode = kTileNone;
+}
+
+namespace {
+template <typename K>
+void allow_smem(K kernel, std::atomic<unsigned long long>& set) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(set.load(std::memory_order_relaxed) & bit)) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
+        set.fetch_or(bit, std::memory_order_relaxed);
+    }
+}
+
+template <typename T, bool THREE, int NZG>
+void down_uni(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, T* xs, T* rc, T* zero,
+              cudaStream_t st) {
+    static std::atomic<unsigned long long> set{0ull};
+    const TileGeo& g = t.down;
+    allow_smem(k_mg_down_uni<T, THREE, NZG>, set);
+    launch_k(k_mg_down_uni<T, THREE, NZG>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc,
+             b, xs, rc, zero, t.u, g);
+}
+template <typename T, bool THREE, int NZG>
+void up_uni(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, const T* xs, const T* xc,
+            T* out, cudaStream_t st) {
+    static std::atomic<unsigned long long> set{0ull};
+    const TileGeo& g = t.up;
+    allow_smem(k_mg_up_uni<T, THREE, NZG>, set);
+    launch_k(k_mg_up_uni<T, THREE, NZG>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc, b,
+             xs, xc, out, t.u, g);
+}
+template <typename T, bool THREE, int S>
+void down_cross(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, T* xs, T* rc, T* zero,
+                cudaStream_t st) {
+    static std::atomic<unsigned long long> set{0ull};
+    const TileGeo& g = t.down;
+    allow_smem(k_mg_down_cross<T, THREE, S>, set);
+    launch_k(k_mg_down_cross<T, THREE, S>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc,
+             b, xs, rc, zero, t.r, g);
+}
+template <typename T, bool THREE, int S>
+void up_cross(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, const T* xs, const T* xc,
+              T* out, cudaStream_t st) {
+    static std::atomic<unsigned long long> set{0ull};
+    const TileGeo& g = t.up;
+    allow_smem(k_mg_up_cross<T, THREE, S>, set);
+    launch_k(k_mg_up_cross<T, THREE, S>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc, b,
+             xs, xc, out, t.r, g);
+}
+}  // namespace
+
+// Uniform levels: the level counts of the decks' usual Nz unrolled. Cross
+// levels (FP64): the lanes per column, two rows each.
+#define OW3D_TILE(way, ...)                                                \
+    do {                                                                   \
+        if (t.mode == kTileUniform) {                                      \
+            if (F.Nyg > 1) {                                               \
+                if (F.Nzg == 18) way##_uni<T, true, 18>(__VA_ARGS__);      \
+                else if (F.Nzg == 10) way##_uni<T, true, 10>(__VA_ARGS__); \
+                else way##_uni<T, true, 0>(__VA_ARGS__);                   \
+            } else {                                                       \
+                if (F.Nzg == 10) way##_uni<T, false, 10>(__VA_ARGS__);     \
+                else way##_uni<T, false, 0>(__VA_ARGS__);                  \
+            }                                                              \
+        } else if constexpr (sizeof(T) == 8) {                             \
+            if (F.Nyg > 1) {                                               \
+                if (F.Nzg <= 10) way##_cross<T, true, 4>(__VA_ARGS__);     \
+                else if (F.Nzg <= 18) way##_cross<T, true, 8>(__VA_ARGS__); \
+                else way##_cross<T, true, 16>(__VA_ARGS__);                \
+            } else {                                                       \
+                if (F.Nzg <= 10) way##_cross<T, false, 4>(__VA_ARGS__);    \
+                else if (F.Nzg <= 18) way##_cross<T, false, 8>(__VA_ARGS__); \
+                else way##_cross<T, false, 16>(__VA_ARGS__);               \
+            }                                                              \
+        }                                                                  \
+    } while (0)
+
+template <typename T>
+void launch_tile_down(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, T* xs, T* rc,
+                      T* zero, cudaStream_t st) {
+    OW3D_TILE(down, F, Cc, t, b, xs, rc, zero, st);
+}
+template <typename T>
+void launch_tile_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, const T* xs,
+                    const T* xc, T* out, cudaStream_t st) {
+    OW3D_TILE(up, F, Cc, t, b, xs, xc, out, st);
+}
+
+#define OW3D_INST(T)                                                                                              \
+    template void tile_geometry<T>(const LevelDev<T>&, TileLevel<T>&);                                            \
+    template void launch_tile_down<T>(const LevelDev<T>&, const LevelDev<T>&, const TileLevel<T>&, const T*, T*,  \
+                                      T*, T*, cudaStream_t);                                                      \
+    template void launch_tile_up<T>(const LevelDev<T>&, const LevelDev<T>&, const TileLevel<T>&, const T*,        \
+                                    const T*, const T*, T*, cudaStream_t);
+OW3D_INST(double)
+OW3D_INST(float)
+#undef OW3D_INST
+
+}  // namespace ow3d

@@ -18,6 +18,7 @@
 
 #include "ow3d_fs.h"
 #include "ow3d_internal.h"
+#include "mg_tile.cuh"
 #include "../../include/ow3d_test.h"
 #include "setup.h"
 
@@ -45,6 +46,7 @@ struct MgSet {
     T* dense_op = nullptr;  // dense operator of level dense_level (coarse_inv when 0)
     int dense_level = 0;
     LevelTable<T> table;    // level table of the fused coarse-level kernel
+    std::vector<TileLevel<T>> tile;   // per level, its form in the fused tile kernels
     T* fine_b = nullptr;    // right-hand side of the finest level
     T* fine_x = nullptr;    // iterate of the finest level when not written in place
 };
@@ -168,10 +170,93 @@ int upload(ow3d_handle* H, T** p, const std::vector<double>& v) {
 
 #define TRY(x) do { int r_ = (x); if (r_) return r_; } while (0)
 
+// The form a level takes in the fused tile kernels, and its row constants.
+// Both forms need a uniform grid in x and y (one centred stencil for all
+// interior columns, checked value by value). Uniform: no mixed-derivative
+// terms and the same coefficients in every interior column (flat bottom) -- a
+// varying depth given without its slopes keeps the per-phase kernels. Cross:
+// mixed-derivative terms, walls, FP64 only: in FP32 another order of the sums
+// moves the steep basins' results by up to 1e-8 (65x33x9 shoal, which stops at
+// the matvec limit: 2e-9; two-dimensional 65x17 and 257x17 flumes: 1e-9), in
+// FP64 by 1e-12. Flat levels move by 1e-11 at most in FP32. Periodic levels
+// with an odd period (the two colours would meet at its ends) have none.
+template <typename T>
+TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vector<double>& cf,
+                        const std::vector<double>& bt) {
+    TileLevel<T> t;
+    if (h.Nzg > kTileMaxNzg || h.Nzg < 5) return t;
+    const bool three = h.Nyg > 1;
+    const int nx = h.Nxg, ny = h.Nyg;
+    const int jlo = three ? 2 : 1, jhi = three ? ny - 1 : 1, ihi = d.per ? nx - 2 : nx - 1;
+    auto sz = [&](int o, int k, int m) { return h.SZ.w[((size_t)(o - 1) * h.Nzg + (k - 1)) * 3 + m]; };
+    auto sx = [&](int o, int i, int m) { return h.SX.w[((size_t)(o - 1) * nx + (i - 1)) * 3 + m]; };
+    auto sy = [&](int o, int j, int m) { return h.SY.w[((size_t)(o - 1) * ny + (j - 1)) * 3 + m]; };
+    for (int o = 1; o <= 2; ++o)
+        for (int m = 0; m < 3; ++m) {
+            for (int i = 2; i <= ihi; ++i) if (sx(o, i, m) != sx(o, 2, m)) return t;
+            if (three) for (int j = 2; j <= jhi; ++j) if (sy(o, j, m) != sy(o, 2, m)) return t;
+        }
+    const double gx[2][3] = {{sx(1, 2, 1), sx(1, 2, 2), 1.0 / sx(1, 2, 0)},
+                             {sx(1, nx - 1, 1), sx(1, nx - 1, 0), 1.0 / sx(1, nx - 1, 2)}};
+    double gy[2][3] = {{0, 0, 0}, {0, 0, 0}};
+    if (three) {
+        gy[0][0] = sy(1, 2, 1); gy[0][1] = sy(1, 2, 2); gy[0][2] = 1.0 / sy(1, 2, 0);
+        gy[1][0] = sy(1, ny - 1, 1); gy[1][1] = sy(1, ny - 1, 0); gy[1][2] = 1.0 / sy(1, ny - 1, 2);
+    }
+    if (d.cross) {
+        if (d.per || d.ncolor != (three ? 4 : 2) || sizeof(T) != 8) return t;
+        t.mode = kTileCross;
+        RowTab<T>& r = t.r;
+        for (int k = 1; k <= h.Nzg; ++k) {
+            r.om[k - 1] = T(1.0 - h.zs[k - 1]);
+            r.z0[k - 1] = T(sz(1, k, 0)); r.z1[k - 1] = T(sz(1, k, 1)); r.z2[k - 1] = T(sz(1, k, 2));
+            r.y0[k - 1] = T(sz(2, k, 0)); r.y1[k - 1] = T(sz(2, k, 1)); r.y2[k - 1] = T(sz(2, k, 2));
+        }
+        for (int m = 0; m < 3; ++m) {
+            r.sx1[m] = T(sx(1, 2, m)); r.sx2[m] = T(sx(2, 2, m));
+            r.ex[0][m] = T(sx(1, 1, m)); r.ex[1][m] = T(sx(1, nx, m));
+            r.sy1[m] = T(three ? sy(1, 2, m) : 0.0); r.sy2[m] = T(three ? sy(2, 2, m) : 0.0);
+            r.ey[0][m] = T(three ? sy(1, 1, m) : 0.0); r.ey[1][m] = T(three ? sy(1, ny, m) : 0.0);
+            for (int s = 0; s < 2; ++s) { r.gx[s][m] = T(gx[s][m]); r.gy[s][m] = T(gy[s][m]); }
+        }
+        tile_geometry(d, t);
+        return t;
+    }
+    if (d.ncolor != 2 || (d.per && (nx - 3) % 2 != 0)) return t;
+    const size_t q0 = 1 + (size_t)nx * (jlo - 1);
+    for (int j = jlo; j <= jhi; ++j)
+        for (int i = 2; i <= ihi; ++i) {
+            const size_t q = (size_t)(i - 1) + (size_t)nx * (j - 1);
+            for (int m = 0; m < 4; ++m) if (cf[4 * q + m] != cf[4 * q0 + m]) return t;
+            for (int m = 0; m < 8; ++m) if (bt[8 * q + m] != bt[8 * q0 + m]) return t;
+        }
+    for (int m = 2; m < 6; ++m) if (bt[8 * q0 + m] != 0.0) return t;
+    t.mode = kTileUniform;
+    UniTab<T>& u = t.u;
+    const double ih = cf[4 * q0], ca = cf[4 * q0 + 1], cb = cf[4 * q0 + 2], c3 = cf[4 * q0 + 3];
+    for (int k = 2; k <= h.Nzg - 1; ++k) {
+        const double om = 1.0 - h.zs[k - 1], s2 = om * ca, s4 = om * cb, s3 = om * c3;
+        const double cz = s2 * s2 + s4 * s4 + ih * ih;
+        const double dg = sx(2, 2, 1) + (three ? sy(2, 2, 1) : 0.0) + s3 * sz(1, k, 1) + cz * sz(2, k, 1);
+        const double lo = s3 * sz(1, k, 0) + cz * sz(2, k, 0), up = s3 * sz(1, k, 2) + cz * sz(2, k, 2);
+        u.id[k - 1] = T(1.0 / dg);
+        u.g[k - 1] = T(lo / dg);
+        u.lo[k - 1] = T(lo); u.dg[k - 1] = T(dg); u.up[k - 1] = T(up);
+    }
+    u.t0 = T(bt[8 * q0]); u.t1 = T(bt[8 * q0 + 1]); u.t6 = T(bt[8 * q0 + 6]);
+    u.wxl = T(sx(2, 2, 0)); u.wxr = T(sx(2, 2, 2));
+    u.wyd = three ? T(sy(2, 2, 0)) : T(0); u.wyu = three ? T(sy(2, 2, 2)) : T(0);
+    for (int s = 0; s < 2; ++s)
+        for (int m = 0; m < 3; ++m) { u.gx[s][m] = T(gx[s][m]); u.gy[s][m] = T(gy[s][m]); }
+    tile_geometry(d, t);
+    return t;
+}
+
 template <typename T>
 int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
     const int L = (int)H->G.levels.size();
     S.lev.resize(L);
+    S.tile.assign((size_t)L, TileLevel<T>());
     for (int l = 0; l < L; ++l) {
         const LevelHost& h = H->G.levels[l];
         LevelDev<T>& d = S.lev[l];
@@ -199,8 +284,8 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
         };
         TRY(upload(H, &ix, recip(h.x))); TRY(upload(H, &iy, recip(h.y))); TRY(upload(H, &iz, recip(h.z)));
         d.ix = ix; d.iy = iy; d.iz = iz;
+        std::vector<double> cf(4 * h.h.size()), bt(8 * h.h.size(), 0.0);
         {
-            std::vector<double> cf(4 * h.h.size());
             for (size_t q = 0; q < h.h.size(); ++q) {
                 const double ih = 1.0 / h.h[q];
                 const bool three = h.Nyg > 1;   // 2-D levels ignore any y-derivatives of h
@@ -220,7 +305,6 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
             const bool three = h.Nyg > 1;
             const double omb = 1.0 - h.zs[1];
             const double z0 = h.SZ.w[3 + 0], z1 = h.SZ.w[3 + 1], z2 = h.SZ.w[3 + 2];   // order 1, row 2
-            std::vector<double> bt(8 * h.h.size(), 0.0);
             for (int jj = 1; jj <= h.Nyg; ++jj)
                 for (int ii = 1; ii <= h.Nxg; ++ii) {
                     const size_t q = (size_t)(ii - 1) + (size_t)h.Nxg * (jj - 1);
@@ -304,6 +388,7 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
             TRY(upload(H, &a1, wx_)); TRY(upload(H, &a2, wy_)); TRY(upload(H, &a3, wz_));
             d.pwx = a1; d.pwy = a2; d.pwz = a3;
         }
+        if (l > 0) S.tile[(size_t)l] = tile_level<T>(h, d, cf, bt);
         T* r;
         TRY(dalloc(H, &r, d.N)); d.rv = r;
         if (l < L - 1) {
@@ -314,6 +399,7 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
     }
     TRY(dalloc(H, &S.table.dev, (size_t)kMaxLevels));
     std::memset((void*)S.table.host, 0, sizeof(S.table.host));
+    S.table.tile = S.tile.data();
     LevelDev<T>& F = S.lev[L - 1];
     TRY(dalloc(H, &S.fine_b, F.N));
     F.bv = S.fine_b;
@@ -1194,6 +1280,7 @@ int ow3d_test_set_colour_prefetch(int mode) { return g_colour_prefetch.exchange(
 long long ow3d_test_set_tail_max_points(long long points) {
     return g_tail_max_points.exchange(points < 0 ? 0 : (int64_t)points);
 }
+int ow3d_test_set_tiles(int on) { return g_tiles.exchange(on ? 1 : 0); }
 int ow3d_test_set_pdl(int on) { return g_pdl.exchange(on ? 1 : 0); }
 int ow3d_test_set_tail_cluster(int blocks) { return g_tail_cluster.exchange(blocks < 0 ? 0 : blocks); }
 long long ow3d_test_set_coop_max_points(long long points) {

@@ -27,6 +27,8 @@ extern std::atomic<int64_t> g_tail_max_points;
 extern std::atomic<int> g_tail_cluster;
 extern std::atomic<int> g_colour_tiles;
 extern std::atomic<int> g_colour_prefetch;
+// 0: every level takes the per-phase multigrid kernels (a testing knob)
+extern std::atomic<int> g_tiles;
 
 // Set (on the capturing thread) when a launch sequence under stream capture
 // issued a host-to-device copy whose source the host later overwrites.
@@ -235,6 +237,8 @@ void launch_ho_matvec(const HoGrid& g, const Surface& s, const TIN* phi, const d
 // Device copy of the level table for the fused coarse-level kernel, with the
 // host image of what was last uploaded.
 template <typename T>
+struct TileLevel;   // mg_tile.cuh
+template <typename T>
 struct LevelTable {
     LevelDev<T>* dev = nullptr;
     LevelDev<T> host[kMaxLevels];
@@ -245,6 +249,8 @@ struct LevelTable {
     // (ow3d_set_smoother_order): no fused coarse cycle, no dense sub-cycle
     // operator (the V cycle descends to the coarsest level's inverse)
     bool lex = false;
+    // per level, the form of the fused tile kernels (mg_tile.cu); null: none
+    const TileLevel<T>* tile = nullptr;
 };
 
 // M: dense operator of level ld (the coarsest level's inverse when ld = 0).
