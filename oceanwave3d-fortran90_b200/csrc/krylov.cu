@@ -12,6 +12,7 @@
 // Basis vectors are stored unnormalised with a scale factor s_i = 1/|V_i|,
 // which saves the normalisation pass.
 #include "ow3d_internal.h"
+#include <algorithm>
 #include <cmath>
 
 namespace ow3d {
@@ -25,6 +26,29 @@ __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// Sums over the warp of M values per lane (M a power of two <= 32): lane l gets
+// the sum of value l / (32 / M), in each of the 32 / M lanes that share it. A
+// step folds the lanes' values in half, so M values cost M - 1 + log2(32 / M)
+// shuffles instead of 5 M.
+template <int M>
+__device__ __forceinline__ double warp_sums(double* v) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = M; n > 1; n >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n / 2; ++i) {
+            const double send = up ? v[i] : v[i + n / 2], keep = up ? v[i + n / 2] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    double s = v[0];
+#pragma unroll
+    for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
 }
 
 // Block-reduce `nv` values per thread into partial[v*nblocks + blockIdx.x].
@@ -59,21 +83,28 @@ __device__ bool last_block_reduce(double* partial, int nv, int nblocks, unsigned
     if (!amlast) return false;
     __threadfence();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int v = wid; v < nv; v += nw) {
-        const double* pv = partial + (int64_t)v * nblocks;
-        double s = 0;
-        int b = lane;
-        // eight independent L2 loads in flight per lane, then added in order
-        for (; b + 7 * 32 < nblocks; b += 8 * 32) {
-            double q[8];
+    // three vectors a warp, four L2 loads of each in flight per lane
+    for (int v0 = wid; v0 < nv; v0 += 3 * nw) {
+        double s[3] = {0.0, 0.0, 0.0};
+        for (int b = lane; b < nblocks; b += 4 * 32) {
+            double q[3][4];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) q[u] = __ldcg(pv + b + u * 32);
+            for (int g = 0; g < 3; ++g)
 #pragma unroll
-            for (int u = 0; u < 8; ++u) s += q[u];
+                for (int u = 0; u < 4; ++u) {
+                    const int v = v0 + g * nw, bb = b + 32 * u;
+                    q[g][u] = v < nv && bb < nblocks ? __ldcg(partial + (int64_t)v * nblocks + bb) : 0.0;
+                }
+#pragma unroll
+            for (int g = 0; g < 3; ++g)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[g] += q[g][u];
         }
-        for (; b < nblocks; b += 32) s += __ldcg(pv + b);
-        s = warp_sum(s);
-        if (lane == 0) out[v] = s;
+#pragma unroll
+        for (int g = 0; g < 3; ++g) s[g] = warp_sum(s[g]);
+        if (lane == 0)
+            for (int g = 0; g < 3; ++g)
+                if (v0 + g * nw < nv) out[v0 + g * nw] = s[g];
     }
     __syncthreads();
     if (threadIdx.x == 0) *counter = 0u;
@@ -110,33 +141,49 @@ __global__ void __launch_bounds__(kThreads) k_norm_init(const double* __restrict
     }
 }
 
-// Upper-triangular solve R y = g for the current k (1 thread); R is the
-// in-place rotated H (left GMRES) or the separate rotated copy (FGMRES).
+// Upper-triangular solve R y = g for the current k, one warp: R and g in shared
+// memory, lane l holding the right-hand sides of rows l and l + 32; each step
+// fixes one unknown and the lanes subtract its column. (One thread reading R
+// from memory: 18-32 us at 16-22 columns, a chain of loads.)
 // With in_basis set (left preconditioning), the coefficients of the vectors
 // the Arnoldi steps multiplied are taken to the final basis, y <- T y, so
 // that the update is x += sum_i y_i v_i.
-__global__ void k_backsolve(KrylovState* ks, int rotated_R, int in_basis) {
+__global__ void __launch_bounds__(kThreads) k_backsolve(KrylovState* ks, int in_basis) {
     pdl_entry();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    auto Rv = [&](int col, int row) -> double { return rotated_R ? ks->R[col][row] : ks->H[col][row]; };
-    int kk = ks->k;
-    while (kk > 0 && Rv(kk - 1, kk - 1) == 0.0) --kk;
-    for (int i = kk - 1; i >= 0; --i) {
-        double t = ks->g[i];
-        for (int j = i + 1; j < kk; ++j) t -= Rv(j, i) * ks->y[j];
-        ks->y[i] = t / Rv(i, i);
+    __shared__ double R[kMaxKrylov + 1][kMaxKrylov + 1], y[kMaxKrylov + 1];
+    __shared__ int kk;
+    const int k0 = ks->k, tid = threadIdx.x;
+    for (int t = tid; t < k0 * k0; t += blockDim.x) {
+        const int c = t / k0, r = t - c * k0;
+        R[c][r] = r <= c ? ks->R[c][r] : 0.0;
     }
-    if (in_basis) {
-        // T is upper triangular in (i, j): entry i of T y reads y[j >= i]
-        // only, so it can replace y[i] in increasing i
-        for (int i = 0; i < kk; ++i) {
-            double c = 0.0;
-            for (int j = i; j < kk; ++j) c += ks->T[j][i] * ks->y[j];
-            ks->y[i] = c;
+    __syncthreads();
+    if (tid < 32) {
+        int k = k0;
+        while (k > 0 && R[k - 1][k - 1] == 0.0) --k;
+        const int r0 = tid, r1 = tid + 32;
+        double g0 = r0 < k ? ks->g[r0] : 0.0, g1 = r1 < k ? ks->g[r1] : 0.0;
+        const double i0 = r0 < k ? 1.0 / R[r0][r0] : 0.0, i1 = r1 < k ? 1.0 / R[r1][r1] : 0.0;
+        for (int i = k - 1; i >= 0; --i) {
+            const double v = __shfl_sync(0xffffffffu, i < 32 ? g0 * i0 : g1 * i1, i & 31);
+            if (r0 < i) g0 -= R[i][r0] * v;
+            if (r1 < i) g1 -= R[i][r1] * v;
+            if (tid == 0) y[i] = v;
         }
+        if (tid == 0) kk = k;
     }
-    for (int i = kk; i <= kMaxKrylov; ++i) ks->y[i] = 0.0;
-    ks->k = kk;
+    __syncthreads();
+    const int k = kk;
+    for (int i = tid; i <= kMaxKrylov; i += blockDim.x) {
+        double c = i < k ? y[i] : 0.0;
+        if (in_basis && i < k) {
+            c = 0.0;
+            for (int j = i; j < k; ++j) c += ks->T[j][i] * y[j];
+        }
+        ks->y[i] = c;
+    }
+    __syncthreads();
+    if (tid == 0) ks->k = k;
 }
 
 // x += sum_i y_i * (use_scale ? scale_i : 1) * Z_i
@@ -152,7 +199,15 @@ __global__ void __launch_bounds__(kThreads) k_solution_update(double* __restrict
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += stride) {
         double a = x[t];
-        for (int v = 0; v < k; ++v) a += coef[v] * (double)__ldcs(Z + (int64_t)v * ldz + t);
+        int v = 0;
+        for (; v + 8 <= k; v += 8) {   // eight vectors' loads in flight
+            TZ z[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) z[u] = __ldcs(Z + (int64_t)(v + u) * ldz + t);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) a += coef[v + u] * (double)z[u];
+        }
+        for (; v < k; ++v) a += coef[v] * (double)__ldcs(Z + (int64_t)v * ldz + t);
         x[t] = a;
     }
 }
@@ -172,129 +227,176 @@ __global__ void k_krylov_reset(KrylovState* ks) {
 // reduction, so each Arnoldi step reads the basis twice (reduce, update)
 // instead of four times. V_0..V_{j-1} are final, V_j has had one pass.
 
-// rotate unrotated column col of H with rotations 0..col-1 into R, form
-// rotation col, rotate g from its value before rotation col; returns |g[col+1]|
-__device__ double dcgs_rotate(KrylovState* ks, int col) {
-    for (int r = 0; r <= col + 1; ++r) ks->R[col][r] = ks->H[col][r];
-    for (int i = 0; i < col; ++i) {
-        const double a0 = ks->R[col][i];
-        ks->R[col][i] = ks->cs[i] * a0 + ks->sn[i] * ks->R[col][i + 1];
-        ks->R[col][i + 1] = ks->cs[i] * ks->R[col][i + 1] - ks->sn[i] * a0;
+// The scalar work of a step runs in the warp that ends a kernel's last block,
+// with its columns in shared memory: lane l takes entries l and l + 32, and
+// only the chain of rotations is serial, on registers' distance instead of a
+// chain of loads from the state in memory.
+struct ColScratch {
+    double h[kMaxKrylov + 2], cs[kMaxKrylov + 1], sn[kMaxKrylov + 1], scale[kMaxKrylov + 2];
+};
+
+// One warp: rotate the unrotated column col of H (w.h[0..col+1]) with
+// rotations 0..col-1 into R, form rotation col, rotate g from its value
+// before rotation col (g0); w.cs, w.sn hold rotations 0..col-1 and get
+// rotation col. Returns |g[col+1]|.
+__device__ double dcgs_rotate(KrylovState* ks, ColScratch& w, int col, double g0) {
+    const int lane = threadIdx.x & 31;
+    double a = w.h[0];
+    double al = 0.0, gc = 0.0;
+    if (lane == 0) {
+        for (int i = 0; i < col; ++i) {
+            const double n = w.h[i + 1];
+            w.h[i] = w.cs[i] * a + w.sn[i] * n;
+            a = w.cs[i] * n - w.sn[i] * a;
+        }
+        const double yv = w.h[col + 1];
+        const double r = sqrt(a * a + yv * yv);
+        double c = 1.0, sg = 0.0, d = a;
+        if (r != 0.0) { c = a / r; sg = yv / r; d = r; }
+        w.h[col] = d;
+        w.h[col + 1] = r != 0.0 ? 0.0 : yv;
+        w.cs[col] = c; w.sn[col] = sg;
+        ks->cs[col] = c; ks->sn[col] = sg;
+        al = -sg * g0;
+        gc = c * g0;
+        ks->g[col] = gc;
+        ks->g[col + 1] = al;
     }
-    const double x = ks->R[col][col], yv = ks->R[col][col + 1];
-    const double r = sqrt(x * x + yv * yv);
-    double c = 1.0, sg = 0.0;
-    if (r != 0.0) { c = x / r; sg = yv / r; ks->R[col][col] = r; ks->R[col][col + 1] = 0.0; }
-    ks->cs[col] = c; ks->sn[col] = sg;
-    const double g0 = ks->gsave[col];
-    const double al = -sg * g0;
-    ks->g[col] = c * g0;
-    ks->g[col + 1] = al;
-    return fabs(al);
+    __syncwarp();
+    for (int r = lane; r <= col + 1; r += 32) ks->R[col][r] = w.h[r];
+    __syncwarp();
+    return fabs(__shfl_sync(0xffffffffu, al, 0));
 }
 
-// One thread, after step j's reduction: res[2i] = <V_i, V_j>, res[2i+1] = <V_i, W>, i <= j.
+// One warp, after step j's reduction: res[2i] = <V_i, V_j>, res[2i+1] = <V_i, W>, i <= j.
 // The vector step j multiplied, scale_j V_j with V_j after one pass and
 // scale_j its provisional scale, is scale_j (nu q_j + sum sigma_i q_i) in
 // the final basis: column j of T (used by left preconditioning, whose
 // solution is a combination of those vectors).
-__device__ void dcgs_column(KrylovState* ks, int j, const double* res) {
-    double ss = 0.0, corr = 0.0;
+__device__ void dcgs_column(KrylovState* ks, ColScratch& w, int j, const double* res) {
+    const int lane = threadIdx.x & 31;
+    double sig[2] = {0.0, 0.0}, sc[2] = {0.0, 0.0};
+    double g0 = 0.0, scj = ks->scale[j];
     if (j >= 1) {
-        const double sp = ks->scale[j];
-        for (int i = 0; i < j; ++i) {
-            const double sig = ks->scale[i] * res[2 * i];
-            ks->coefA[i] = sig;          // sigma_i, scaled below
-            ks->T[j][i] = sp * sig;
-            ss += sig * sig;
+        g0 = ks->gsave[j - 1];
+        double ss = 0.0;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = lane + 32 * q;
+            if (i < j) {
+                sc[q] = ks->scale[i];
+                const double h = ks->H[j - 1][i];
+                if (i < j - 1) { w.cs[i] = ks->cs[i]; w.sn[i] = ks->sn[i]; }
+                sig[q] = sc[q] * res[2 * i];
+                ks->T[j][i] = scj * sig[q];
+                // complete column j-1: W_{j-1} = sum (h + sigma) q_i + nu q_j
+                ks->H[j - 1][i] = h + sig[q];
+                w.h[i] = h + sig[q];
+                ss += sig[q] * sig[q];
+            }
         }
+        ss = warp_sum(ss);
         const double nu = sqrt(fmax(res[2 * j] - ss, 0.0));
-        ks->T[j][j] = sp * nu;
-        // complete column j-1: W_{j-1} = sum (h + sigma) q_i + nu q_j
-        for (int i = 0; i < j; ++i) ks->H[j - 1][i] += ks->coefA[i];
-        ks->H[j - 1][j] = nu;
-        ks->scale[j] = nu > 0 ? 1.0 / nu : 0.0;
-        ks->resid = dcgs_rotate(ks, j - 1);
-    } else {
+        if (lane == 0) {
+            ks->T[j][j] = scj * nu;
+            ks->H[j - 1][j] = nu;
+            w.h[j] = nu;
+        }
+        scj = nu > 0 ? 1.0 / nu : 0.0;
+        __syncwarp();
+        const double resid = dcgs_rotate(ks, w, j - 1, g0);
+        if (lane == 0) { ks->scale[j] = scj; ks->resid = resid; }
+    } else if (lane == 0) {
         ks->T[0][0] = 1.0;   // scale_0 V_0 is final: v_0
     }
-    for (int i = 0; i < j; ++i) {
-        const double hq = ks->scale[i] * res[2 * i + 1];
-        ks->H[j][i] = hq;
-        corr += ks->coefA[i] * hq;
-        ks->coefB[i] = hq * ks->scale[i];
-        ks->coefA[i] *= ks->scale[i];
+    double corr = 0.0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int i = lane + 32 * q;
+        if (i < j) {
+            const double hq = sc[q] * res[2 * i + 1];
+            ks->H[j][i] = hq;
+            corr += sig[q] * hq;
+            ks->coefB[i] = hq * sc[q];
+            ks->coefA[i] = sig[q] * sc[q];
+        }
     }
-    const double hj = (j >= 1) ? (res[2 * j + 1] - corr) * ks->scale[j] : ks->scale[j] * res[2 * j + 1];
-    ks->H[j][j] = hj;
-    ks->coefB[j] = hj * ks->scale[j];
+    corr = warp_sum(corr);
+    if (lane == 0) {
+        const double hj = (j >= 1 ? res[2 * j + 1] - corr : res[2 * j + 1]) * scj;
+        ks->H[j][j] = hj;
+        ks->coefB[j] = hj * scj;
+    }
 }
 
 // Reduction: res[2v] = <V_v, V_j>, res[2v+1] = <V_v, W> for v <= j. The
-// vectors are cut into chunks of kDotE * blockDim.x element pairs; a block
-// takes chunks in turn, keeps its thread's kDotE pairs of V_j and W in
-// registers, and streams every V_v of the chunk once (so each vector is read
-// from memory once per step). Per vector, each warp adds its sum to its own
-// shared-memory slot; the block's slots become partial[u * gridDim.x + b];
+// vectors are cut into chunks of E * blockDim.x element pairs; a block takes
+// chunks in turn, keeps its thread's E pairs of V_j and W in registers, and
+// streams every V_v of the chunk once (so each vector is read from memory once
+// per step), G vectors' loads in flight together. The warp sums of G vectors'
+// 2 G values fold into each other (warp_sums), and a warp adds them to its own
+// shared-memory slots; the block's slots become partial[u * gridDim.x + b];
 // the last block reduces the partials in a fixed order and runs dcgs_column.
-constexpr int kDotE = 4;
-constexpr int kDotG = 4;   // vectors whose loads are issued together
-
+// E = G = 4 streams long vectors; short ones, whose few chunks leave most SMs
+// idle and whose time is the latency of the groups one after another, take
+// E = 1, G = 8.
+template <int E, int G>
 __global__ void __launch_bounds__(kThreads) k_dcgs_reduce(const double* __restrict__ V, int64_t ldv, int j,
                                                           const double* __restrict__ W, int64_t n, double* partial,
-                                                          unsigned int* counter, int nbx, KrylovState* ks) {
+                                                          unsigned int* counter, KrylovState* ks) {
     pdl_entry();
     if (ks->done) return;
-    __shared__ double acc[2 * kMaxDots][kThreads / 32];
+    __shared__ double acc[2 * kMaxDots + 2 * G][kThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int nv = 2 * (j + 1);
-    for (int u = threadIdx.x; u < nv * nw; u += blockDim.x) acc[u / nw][u % nw] = 0.0;
+    for (int u = threadIdx.x; u < (nv + 2 * G) * nw; u += blockDim.x) acc[u / nw][u % nw] = 0.0;
     __syncthreads();
     const int64_t n2 = (n + 1) / 2;
-    const int64_t chunk = (int64_t)kDotE * blockDim.x;
+    const int64_t chunk = (int64_t)E * blockDim.x;
     const int64_t nchunks = (n2 + chunk - 1) / chunk;
     const double2* q2 = reinterpret_cast<const double2*>(V + (int64_t)j * ldv);
     const double2* w2 = reinterpret_cast<const double2*>(W);
+    constexpr int L = 32 / (2 * G);   // lanes that share a sum
     for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         const int64_t t0 = ch * chunk + threadIdx.x;
-        double2 q[kDotE], w[kDotE];
+        double2 q[E], w[E];
 #pragma unroll
-        for (int e = 0; e < kDotE; ++e) {
+        for (int e = 0; e < E; ++e) {
             const int64_t t = t0 + (int64_t)e * blockDim.x;
             if (t < n2) { q[e] = q2[t]; w[e] = w2[t]; }
             else { q[e] = make_double2(0.0, 0.0); w[e] = make_double2(0.0, 0.0); }
         }
-        // vectors in groups of kDotG, all their loads in flight together; the
-        // older basis vectors are read once per pass, so they are streamed
+        // the older basis vectors are read once per pass, so they are streamed
         // (evict-first) rather than let them push the multigrid levels and
         // their coefficient tables out of L2 before the next V-cycle
-        for (int v0 = 0; v0 <= j; v0 += kDotG) {
-            double2 x[kDotG][kDotE];
+        for (int v0 = 0; v0 <= j; v0 += G) {
+            double2 x[G][E];
 #pragma unroll
-            for (int g = 0; g < kDotG; ++g) {
+            for (int g = 0; g < G; ++g) {
                 const int v = v0 + g;
                 const double2* a2 = reinterpret_cast<const double2*>(V + (int64_t)min(v, j) * ldv);
 #pragma unroll
-                for (int e = 0; e < kDotE; ++e) {
+                for (int e = 0; e < E; ++e) {
                     const int64_t t = t0 + (int64_t)e * blockDim.x;
                     x[g][e] = (v < j && t < n2) ? __ldcs(a2 + t) : make_double2(0.0, 0.0);
                 }
             }
+            double s[2 * G];
 #pragma unroll
-            for (int g = 0; g < kDotG; ++g) {
-                const int v = v0 + g;
-                if (v > j) break;
+            for (int g = 0; g < G; ++g) {
                 double sa = 0, sb = 0;
 #pragma unroll
-                for (int e = 0; e < kDotE; ++e) {
-                    const double2 xe = (v == j) ? q[e] : x[g][e];
+                for (int e = 0; e < E; ++e) {
+                    const double2 xe = (v0 + g == j) ? q[e] : x[g][e];
                     sa += xe.x * q[e].x + xe.y * q[e].y;
                     sb += xe.x * w[e].x + xe.y * w[e].y;
                 }
-                sa = warp_sum(sa);
-                sb = warp_sum(sb);
-                if (lane == 0) { acc[2 * v][wid] += sa; acc[2 * v + 1][wid] += sb; }
+                s[2 * g] = sa;
+                s[2 * g + 1] = sb;
             }
+            const double r = warp_sums<2 * G>(s);
+            // the lanes' sums of vectors past j are zero and land past nv
+            if (lane % L == 0) acc[2 * v0 + lane / L][wid] += r;
         }
     }
     __syncthreads();
@@ -303,28 +405,10 @@ __global__ void __launch_bounds__(kThreads) k_dcgs_reduce(const double* __restri
         for (int w = 0; w < nw; ++w) t += acc[u][w];
         partial[(int64_t)u * gridDim.x + blockIdx.x] = t;
     }
-    __shared__ bool amlast;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) amlast = (atomicAdd(counter, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!amlast) return;
-    __threadfence();
     __shared__ double res[2 * kMaxDots];
-    const int nb = gridDim.x;
-    for (int u = wid; u < nv; u += nw) {
-        const double* pv = partial + (int64_t)u * nb;
-        double sacc = 0;
-        for (int bb = lane; bb < nb; bb += 32) sacc += __ldcg(pv + bb);
-        sacc = warp_sum(sacc);
-        if (lane == 0) res[u] = sacc;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        *counter = 0u;
-        dcgs_column(ks, j, res);
-    }
-    (void)nbx;
+    if (!last_block_reduce(partial, nv, gridDim.x, counter, res)) return;
+    __shared__ ColScratch scratch;
+    if (wid == 0) dcgs_column(ks, scratch, j, res);
 }
 
 // Update: V_j <- V_j - sum_{i<j} coefA_i V_i,  W <- W - sum_{i<j} coefB_i V_i - coefB_j V_j(new),
@@ -368,20 +452,33 @@ __global__ void __launch_bounds__(kThreads) k_dcgs_update(double* __restrict__ V
     }
     block_store_partials(acc, 1, partial, nblocks);
     __shared__ double res[1];
-    if (last_block_reduce(partial, 1, nblocks, counter, res)) {
-        if (threadIdx.x == 0) {
-            const double nrm = sqrt(res[0]);
-            ks->H[j][j + 1] = nrm;
-            ks->scale[j + 1] = nrm > 0 ? 1.0 / nrm : 0.0;
-            ks->gsave[j] = ks->g[j];
-            ks->resid = dcgs_rotate(ks, j);
-            ks->k = j + 1;
-            ks->iters += 1;
-            const bool conv = ks->resid <= ks->tol;
-            if (conv) ks->converged = 1;
-            if (conv || j + 1 >= m || ks->iters >= maxmv || nrm == 0.0) ks->done = 1;
-            if (hnext) cudaGraphSetConditional(hnext, ks->done ? 0u : 1u);
-        }
+    if (!last_block_reduce(partial, 1, nblocks, counter, res)) return;
+    __shared__ ColScratch w;
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    for (int i = lane; i <= j; i += 32) {
+        w.h[i] = ks->H[j][i];
+        if (i < j) { w.cs[i] = ks->cs[i]; w.sn[i] = ks->sn[i]; }
+    }
+    const double g0 = ks->g[j], tol = ks->tol, nrm = sqrt(res[0]);
+    const int iters = ks->iters + 1;
+    if (lane == 0) {
+        w.h[j + 1] = nrm;
+        ks->H[j][j + 1] = nrm;
+        ks->scale[j + 1] = nrm > 0 ? 1.0 / nrm : 0.0;
+        ks->gsave[j] = g0;
+    }
+    __syncwarp();
+    const double resid = dcgs_rotate(ks, w, j, g0);
+    if (lane == 0) {
+        const bool conv = resid <= tol;
+        const int done = conv || j + 1 >= m || iters >= maxmv || nrm == 0.0;
+        ks->resid = resid;
+        ks->k = j + 1;
+        ks->iters = iters;
+        if (conv) ks->converged = 1;
+        if (done) ks->done = 1;
+        if (hnext) cudaGraphSetConditional(hnext, done ? 0u : 1u);
     }
 }
 
@@ -397,22 +494,35 @@ __global__ void k_solve_log(const KrylovState* ks, SolveLog* out) {
 
 }  // namespace
 
+// Vectors of at most this many element pairs take the short form of the
+// reduction: fewer than four chunks of the long form per SM.
+constexpr int64_t kShortPairs = 4ll * 148 * 4 * kThreads;
+
 void launch_dcgs_reduce(const double* V, int64_t ldv, int j, const double* W, int64_t n, const DotScratch& sc,
                         KrylovState* ks, cudaStream_t st) {
-    // one block per chunk up to the scratch's blocks; 2(j+1) partial rows
-    const int64_t chunks = ((n + 1) / 2 + (int64_t)kDotE * kThreads - 1) / ((int64_t)kDotE * kThreads);
-    int nb = sc.nblocks;
-    if (nb > chunks) nb = (int)chunks;
-    const int cap = (int)(((int64_t)(kMaxKrylov + 2) * sc.nblocks) / (2 * (j + 1)));   // scratch rows
-    if (nb > cap) nb = cap;
+    // one block per chunk, at most two per SM (enough loads in flight, and the
+    // last block's sum over the blocks grows with them); 2(j+1) partial rows
+    const int64_t n2 = (n + 1) / 2;
+    const bool brief = n2 <= kShortPairs;
+    const int64_t chunk = (int64_t)(brief ? 1 : 4) * kThreads;
+    int64_t nb = std::min<int64_t>((n2 + chunk - 1) / chunk, std::min(sc.nblocks, 2 * 148));
+    nb = std::min<int64_t>(nb, ((int64_t)(kMaxKrylov + 2) * sc.nblocks) / (2 * (j + 1)));   // scratch rows
     if (nb < 1) nb = 1;
-    launch_k(k_dcgs_reduce, dim3(nb), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial, sc.counter, nb, ks);
+    if (brief)
+        launch_k(k_dcgs_reduce<1, 8>, dim3((unsigned)nb), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial, sc.counter, ks);
+    else
+        launch_k(k_dcgs_reduce<4, 4>, dim3((unsigned)nb), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial, sc.counter, ks);
+}
+
+// Blocks of a pass over n2 items with one partial sum per block.
+static int pass_blocks(int64_t n2, const DotScratch& sc) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>(sc.nblocks, (n2 + kThreads - 1) / kThreads));
 }
 
 void launch_dcgs_update(double* V, int64_t ldv, int j, double* W, int64_t n, const DotScratch& sc, KrylovState* ks,
                         int maxmv, int m, cudaStream_t st, cudaGraphConditionalHandle hnext) {
-    launch_k(k_dcgs_update, dim3(sc.nblocks), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial, sc.counter, sc.nblocks,
-                                                                  ks, maxmv, m, hnext);
+    const int nb = pass_blocks((n + 1) / 2, sc);
+    launch_k(k_dcgs_update, dim3(nb), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial, sc.counter, nb, ks, maxmv, m, hnext);
 }
 void launch_solve_log(const KrylovState* ks, SolveLog* out, cudaStream_t st) {
     launch_k(k_solve_log, dim3(1), dim3(32), 0, st, ks, out);
@@ -420,12 +530,12 @@ void launch_solve_log(const KrylovState* ks, SolveLog* out, cudaStream_t st) {
 
 void launch_norm_init(const double* v, int64_t n, const DotScratch& sc, KrylovState* ks, double rtol, double atol,
                       cudaStream_t st, cudaGraphConditionalHandle hnext) {
-    launch_k(k_norm_init, dim3(sc.nblocks), dim3(kThreads), 0, st, v, n, sc.partial, sc.counter, sc.nblocks, ks, rtol, atol,
-                                                                hnext);
+    const int nb = pass_blocks(n, sc);
+    launch_k(k_norm_init, dim3(nb), dim3(kThreads), 0, st, v, n, sc.partial, sc.counter, nb, ks, rtol, atol, hnext);
 }
 
-void launch_backsolve(KrylovState* ks, cudaStream_t st, int rotated_R, int in_basis) {
-    launch_k(k_backsolve, dim3(1), dim3(32), 0, st, ks, rotated_R, in_basis);
+void launch_backsolve(KrylovState* ks, cudaStream_t st, int in_basis) {
+    launch_k(k_backsolve, dim3(1), dim3(kThreads), 0, st, ks, in_basis);
 }
 
 template <typename TZ>

@@ -600,10 +600,10 @@ void initial_residual_launches(ow3d_handle* H, const Surface& s, const double* r
 void solution_update_launches(ow3d_handle* H, double* phi) {
     const int64_t N = H->G.N;
     if (H->p.krylov == OW3D_KRYLOV_LGMRES) {
-        launch_backsolve(H->ks, H->st, 1, 1);
+        launch_backsolve(H->ks, H->st, 1);
         launch_solution_update<double>(phi, H->V, H->ldv, N, H->ks, 1, H->st);
     } else {
-        launch_backsolve(H->ks, H->st, 1, 0);
+        launch_backsolve(H->ks, H->st, 0);
         if (!H->mixed) launch_solution_update<double>(phi, (const double*)H->Z, H->ldv, N, H->ks, 0, H->st);
         else launch_solution_update<float>(phi, (const float*)H->Z, H->ldv, N, H->ks, 0, H->st);
     }

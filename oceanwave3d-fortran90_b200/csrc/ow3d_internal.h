@@ -311,7 +311,7 @@ struct SolveLog {
     double resid, beta, tol;
 };
 void launch_solve_log(const KrylovState* ks, SolveLog* out, cudaStream_t st);
-void launch_backsolve(KrylovState* ks, cudaStream_t st, int rotated_R = 0, int in_basis = 0);
+void launch_backsolve(KrylovState* ks, cudaStream_t st, int in_basis);
 template <typename TZ>
 void launch_solution_update(double* x, const TZ* Z, int64_t ldz, int64_t n, const KrylovState* ks, int use_scale,
                             cudaStream_t st);
