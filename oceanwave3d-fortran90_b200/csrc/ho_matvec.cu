@@ -21,10 +21,16 @@
 //    sigma stencil has been read, so only a window of levels is live;
 //  * wall bands: the ghost columns and the columns within kBand points of a
 //    wall (one-sided windows, shifted windows below the bottom), one thread
-//    per column reading phi from global memory, per-position stencils from
-//    the tables. These blocks come first in the grid so that they start
-//    early and overlap the tiles.
+//    per point (k fastest, whole columns per block) reading phi from global
+//    memory, per-position stencils from the tables; the horizontal
+//    derivatives of a column's levels meet in shared memory before its rows
+//    are formed. These blocks come first in the grid so that they start early
+//    and overlap the tiles. Grids of fewer tiles than SMs run wholly this way:
+//    a tile's thread walks its levels one after another, which a small grid
+//    has too few warps to hide (one thread per column in the bands, and tiles
+//    at any size: 23 us at 257x33x9, 11 us at 513x9).
 #include "ow3d_internal.h"
+#include <algorithm>
 #include <cstring>
 
 namespace ow3d {
@@ -125,128 +131,113 @@ __device__ __forceinline__ void band_col(int64_t q, int Nxg, int Nyg, bool all, 
     j = t < kBand ? t + 1 : Nyg - 2 * kBand + 1 + t;
 }
 
-// One column (i, j) of any kind, phi read from global memory, per-position
-// stencils from the tables: the general path.
-template <bool THREE, typename TIN, typename ZT>
-__device__ void ho_column_general(const HoGrid& g, const Surface& s, const TIN* __restrict__ phi, double scale,
-                                  const double* __restrict__ b, double* __restrict__ y, int mode, const ZT& zt,
-                                  int i, int j) {
+// Point (k, i, j) of any kind of column, phi read from global memory,
+// per-position stencils from the tables: the general path, one thread per
+// point of whole columns. sp, sx, sy: the block's shared phi, d/dx and d/dy of
+// this thread's column, level by level. All threads of the block call it;
+// those without a point (on false) only join the barrier.
+template <bool THREE, typename TIN>
+__device__ void ho_point_general(const HoGrid& g, const Surface& s, const TIN* __restrict__ phi, double scale,
+                                 const double* __restrict__ b, double* __restrict__ y, int mode, int i, int j,
+                                 int k, bool on, double* sp, double* sx, double* sy) {
     const int Nxg = g.Nxg, Nyg = g.Nyg, Nzg = g.Nzg;
-    auto P = [&](int k, int ii, int jj) -> double {   // 1-based
-        return (double)__ldg(phi + (int64_t)(k - 1) + (int64_t)Nzg * ((int64_t)(ii - 1) + (int64_t)Nxg * (jj - 1)));
+    auto P = [&](int kk, int ii, int jj) -> double {   // 1-based
+        return (double)__ldg(phi + (int64_t)(kk - 1) + (int64_t)Nzg * ((int64_t)(ii - 1) + (int64_t)Nxg * (jj - 1)));
     };
     const double* SX1 = g.SX;
     const double* SX2 = g.SX + (int64_t)Nxg * kHoRank;
     const double* SY1 = g.SY;
     const double* SY2 = g.SY + (int64_t)Nyg * kHoRank;
     const int64_t col = (int64_t)(i - 1) + (int64_t)Nxg * (j - 1);
-    const int64_t gb = col * Nzg;
-    auto emit = [&](int k, double v) {
-        if (mode == 0) y[gb + k - 1] = scale * v;
-        else y[gb + k - 1] = b[gb + k - 1] - v;
-    };
+    const int64_t p = col * Nzg + k - 1;
     const bool ghost_x = (i == 1 || i == Nxg);
     const bool ghost_y = THREE && (j == 1 || j == Nyg);
-    if (g.per && (ghost_x || i == Nxg - 1)) {
-        // periodic x: ghost and repeated columns are identity rows
-        for (int k = 1; k <= Nzg; ++k) emit(k, P(k, i, j));
-        return;
-    }
-    if (ghost_x || ghost_y) {
-        // Lateral Neumann rows and identity corners (BuildLinearSystem.f90:150-284)
-        const bool corner = ghost_x && ghost_y;
-        for (int k = 1; k <= Nzg; ++k) {
-            double v;
-            if (corner || k == 1) v = P(k, i, j);
-            else if (ghost_x) {
-                const int ia = (i == 1) ? 2 : Nxg - 1, ws = win_start(ia, Nxg);
-                v = 0.0;
-                for (int m = 0; m < kHoRank; ++m) v += SX1[(ia - 1) * kHoRank + m] * P(k, ws + m, j);
-            } else {
-                const int ja = (j == 1) ? 2 : Nyg - 1, ws = win_start(ja, Nyg);
-                v = 0.0;
-                for (int m = 0; m < kHoRank; ++m) v += SY1[(ja - 1) * kHoRank + m] * P(k, i, ws + m);
-            }
-            emit(k, v);
-        }
-        return;
-    }
-    // pass 1: horizontal derivatives at every level (periodic x: the centred
-    // window, its columns taken cyclically)
-    double tx[kZMax], ty[kZMax], lap[kZMax], pc[kZMax];
-    const int wsx = g.per ? i - 3 : win_start(i, Nxg);
-    const int wsy = THREE ? win_start(j, Nyg) : 1;
-    for (int k = 1; k <= Nzg; ++k) {
-        double dx = 0, dxx = 0;
-        for (int m = 0; m < kHoRank; ++m) {
-            const double v = P(k, g.per ? wrap_x(wsx + m, Nxg) : wsx + m, j);
-            dx += SX1[(i - 1) * kHoRank + m] * v;
-            dxx += SX2[(i - 1) * kHoRank + m] * v;
-        }
-        double dy = 0, dyy = 0;
-        if (THREE) {
-            for (int m = 0; m < kHoRank; ++m) {
-                const double v = P(k, i, wsy + m);
-                dy += SY1[(j - 1) * kHoRank + m] * v;
-                dyy += SY2[(j - 1) * kHoRank + m] * v;
-            }
-        }
-        tx[k - 1] = dx; ty[k - 1] = dy; lap[k - 1] = dxx + dyy;
-        pc[k - 1] = P(k, i, j);
-    }
-    // Level k = 1 (below the bottom): the x/y derivative entering the mixed
-    // derivative avoids the ghost corner columns (ConstructTableCrossDerivatives.f90:173-186,231-235).
-    {
-        int sh = 0;
-        if (!g.per && wsx == 1) sh = 1;
-        if (!g.per && wsx + 6 == Nxg) sh = -1;
-        if (sh != 0) {
-            double dx = 0;
-            for (int m = 0; m < kHoRank; ++m) dx += SX1[(i - sh - 1) * kHoRank + m] * P(1, wsx + sh + m, j);
-            tx[0] = dx;
-        }
-        if (THREE) {
-            int shy = 0;
-            if (wsy == 1) shy = 1;
-            if (wsy + 6 == Nyg) shy = -1;
-            if (shy != 0) {
-                double dy = 0;
-                for (int m = 0; m < kHoRank; ++m) dy += SY1[(j - shy - 1) * kHoRank + m] * P(1, i, wsy + shy + m);
-                ty[0] = dy;
-            }
-        }
-    }
-    const ColCoef c = col_coef<THREE>(g, s, col);
-    // pass 2: rows of this column
-    for (int k = 1; k <= Nzg; ++k) {
-        double v;
-        if (k == Nzg) {
-            v = pc[k - 1];  // free surface, Dirichlet
-        } else if (k == 1) {
-            // kinematic bottom condition evaluated at k = 2 (BuildLinearSystem.f90:121-126)
-            const double z2 = zt.zs[1];
-            const double s2 = fma(z2, c.b2, c.a2), s4 = fma(z2, c.b4, c.a4);
-            double dz = 0;
-            for (int m = 0; m < kHoRank; ++m) dz += zt.s1[1][m] * pc[m];
-            v = (c.id + c.hx * s2 + c.hy * s4) * dz + c.hx * tx[1] + c.hy * ty[1];
+    // identity rows: corners, the ghost columns' level below the bottom, and
+    // with periodic x the ghost and repeated columns
+    const bool ident = (g.per && (ghost_x || i == Nxg - 1)) || (ghost_x && ghost_y) || ((ghost_x || ghost_y) && k == 1);
+    const bool inner = on && !ghost_x && !ghost_y && !ident;
+    double v = 0.0, lap = 0.0;
+    if (on && ident) {
+        v = P(k, i, j);
+    } else if (on && !inner) {
+        // Lateral Neumann rows (BuildLinearSystem.f90:150-284)
+        if (ghost_x) {
+            const int ia = (i == 1) ? 2 : Nxg - 1, ws = win_start(ia, Nxg);
+#pragma unroll
+            for (int m = 0; m < kHoRank; ++m) v += SX1[(ia - 1) * kHoRank + m] * P(k, ws + m, j);
         } else {
-            const int wz = zwin(k, Nzg);
-            const double sg = zt.zs[k - 1];
-            const double s2 = fma(sg, c.b2, c.a2), s4 = fma(sg, c.b4, c.a4), s3 = fma(sg, c.b3, c.a3);
-            double dz = 0, dzz = 0, dzx = 0, dzy = 0;
-            for (int m = 0; m < kHoRank; ++m) {
-                const double w1 = zt.s1[k - 1][m], w2 = zt.s2[k - 1][m];
-                const int kk = wz + m - 1;
-                dz += w1 * pc[kk];
-                dzz += w2 * pc[kk];
-                dzx += w1 * tx[kk];
-                if (THREE) dzy += w1 * ty[kk];
-            }
-            const double cz = s2 * s2 + s4 * s4 + c.id * c.id;
-            v = lap[k - 1] + s3 * dz + 2.0 * (s2 * dzx + s4 * dzy) + cz * dzz;
+            const int ja = (j == 1) ? 2 : Nyg - 1, ws = win_start(ja, Nyg);
+#pragma unroll
+            for (int m = 0; m < kHoRank; ++m) v += SY1[(ja - 1) * kHoRank + m] * P(k, i, ws + m);
         }
-        emit(k, v);
+    } else if (inner) {
+        // horizontal derivatives at this level (periodic x: the centred
+        // window, its columns taken cyclically). Below the bottom (k = 1) the
+        // first derivative, which enters the mixed ones only, avoids the ghost
+        // corner columns: its window is shifted off them
+        // (ConstructTableCrossDerivatives.f90:173-186,231-235)
+        const int wsx = g.per ? i - 3 : win_start(i, Nxg);
+        double dx = 0, dxx = 0, dy = 0, dyy = 0;
+#pragma unroll
+        for (int m = 0; m < kHoRank; ++m) {
+            const double q = P(k, g.per ? wrap_x(wsx + m, Nxg) : wsx + m, j);
+            dx += SX1[(i - 1) * kHoRank + m] * q;
+            dxx += SX2[(i - 1) * kHoRank + m] * q;
+        }
+        const int sh = k != 1 || g.per ? 0 : (wsx == 1 ? 1 : (wsx + 6 == Nxg ? -1 : 0));
+        if (sh != 0) {
+            dx = 0;
+            for (int m = 0; m < kHoRank; ++m) dx += SX1[(i - sh - 1) * kHoRank + m] * P(1, wsx + sh + m, j);
+        }
+        if (THREE) {
+            const int wsy = win_start(j, Nyg);
+#pragma unroll
+            for (int m = 0; m < kHoRank; ++m) {
+                const double q = P(k, i, wsy + m);
+                dy += SY1[(j - 1) * kHoRank + m] * q;
+                dyy += SY2[(j - 1) * kHoRank + m] * q;
+            }
+            const int shy = k != 1 ? 0 : (wsy == 1 ? 1 : (wsy + 6 == Nyg ? -1 : 0));
+            if (shy != 0) {
+                dy = 0;
+                for (int m = 0; m < kHoRank; ++m) dy += SY1[(j - shy - 1) * kHoRank + m] * P(1, i, wsy + shy + m);
+            }
+        }
+        sp[k - 1] = P(k, i, j);
+        sx[k - 1] = dx;
+        if (THREE) sy[k - 1] = dy;
+        lap = dxx + dyy;
     }
+    __syncthreads();
+    if (inner) {
+        if (k == Nzg) {
+            v = sp[k - 1];  // free surface, Dirichlet
+        } else {
+            // k = 1: kinematic bottom condition evaluated at k = 2 (BuildLinearSystem.f90:121-126)
+            const int kr = k == 1 ? 2 : k, wz = zwin(kr, Nzg) - 1;
+            const ColCoef c = col_coef<THREE>(g, s, col);
+            const double sg = __ldg(g.zs + kr - 1);
+            const double s2 = fma(sg, c.b2, c.a2), s4 = fma(sg, c.b4, c.a4), s3 = fma(sg, c.b3, c.a3);
+            const double* const w1 = g.SZ + (kr - 1) * kHoRank;
+            const double* const w2 = g.SZ + (Nzg + kr - 1) * kHoRank;
+            double dz = 0, dzz = 0, dzx = 0, dzy = 0;
+#pragma unroll
+            for (int m = 0; m < kHoRank; ++m) {
+                const double a = __ldg(w1 + m), q = sp[wz + m];
+                dz += a * q;
+                dzz += __ldg(w2 + m) * q;
+                dzx += a * sx[wz + m];
+                if (THREE) dzy += a * sy[wz + m];
+            }
+            if (k == 1) {
+                v = (c.id + c.hx * s2 + c.hy * s4) * dz + c.hx * sx[1] + (THREE ? c.hy * sy[1] : 0.0);
+            } else {
+                const double cz = s2 * s2 + s4 * s4 + c.id * c.id;
+                v = lap + s3 * dz + 2.0 * (s2 * dzx + s4 * dzy) + cz * dzz;
+            }
+        }
+    }
+    if (on) y[p] = mode == 0 ? scale * v : b[p] - v;
 }
 
 // ------------------------------------------------------------ interior tiles
@@ -346,11 +337,15 @@ __global__ void __launch_bounds__(THREE ? 256 : 256, 2)
     const double scale = dscale ? *dscale : 1.0;
     const int tid = threadIdx.x;
     if ((int)blockIdx.x < band_blocks) {
-        const int64_t q = (int64_t)blockIdx.x * blockDim.x + tid;
-        if (q >= nband) return;
-        int i, j;
-        band_col(q, Nxg, Nyg, all != 0, i, j);
-        ho_column_general<THREE, TIN>(g, s, phi, scale, b, y, mode, zt, i, j);
+        const int cpb = blockDim.x / Nzg, c = tid / Nzg, k = tid - c * Nzg + 1;   // whole columns per block
+        const int64_t q = (int64_t)blockIdx.x * cpb + c;
+        const bool on = c < cpb && q < nband;
+        int i = 1, j = 1;
+        if (on) band_col(q, Nxg, Nyg, all != 0, i, j);
+        extern __shared__ __align__(16) unsigned char smraw[];
+        double* const sp = reinterpret_cast<double*>(smraw) + c * Nzg;
+        ho_point_general<THREE, TIN>(g, s, phi, scale, b, y, mode, i, j, k, on, sp, sp + blockDim.x,
+                                     sp + 2 * blockDim.x);
         return;
     }
     // interior tile: columns i0..i0+BX-1 (x), j0..j0+BY-1 (y) inside [kBand+1, N-kBand]
@@ -428,21 +423,25 @@ void launch_impl(const HoGrid& g, const Surface& s, const TIN* phi, const double
     };
     centred(g.hSX, g.Nxg, zt.cx);
     if (THREE) centred(g.hSY, g.Nyg, zt.cy);
-    const bool split = uniform && g.Nxg > 2 * kBand && (!THREE || g.Nyg > 2 * kBand);
-    int64_t nband;
     int tiles_x = 1, tiles = 0;
+    if (uniform && g.Nxg > 2 * kBand && (!THREE || g.Nyg > 2 * kBand)) {
+        tiles_x = (g.Nxg - 2 * kBand + BX - 1) / BX;
+        tiles = tiles_x * (THREE ? (g.Nyg - 2 * kBand + BY - 1) / BY : 1);
+        if (tiles < 148) tiles = 0;   // point by point (see above)
+    }
+    const bool split = tiles > 0;
+    int64_t nband;
     if (split) {
         nband = (int64_t)2 * kBand * g.Nyg + (THREE ? (int64_t)2 * kBand * (g.Nxg - 2 * kBand) : 0);
-        tiles_x = (g.Nxg - 2 * kBand + BX - 1) / BX;
-        const int tiles_y = THREE ? (g.Nyg - 2 * kBand + BY - 1) / BY : 1;
-        tiles = tiles_x * tiles_y;
     } else {
         nband = (int64_t)g.Nxg * g.Nyg;
     }
     const int threads = BX * BY;
-    const int band_blocks = (int)((nband + threads - 1) / threads);
+    const int cpb = threads / g.Nzg;
+    const int band_blocks = (int)((nband + cpb - 1) / cpb);
     const int NZP = g.Nzg | 1;
-    const size_t smem = (size_t)HX * HY * NZP * sizeof(TIN);
+    // the band blocks hold phi and its two derivatives of their columns
+    const size_t smem = std::max(tiles > 0 ? (size_t)HX * HY * NZP * sizeof(TIN) : 0, (size_t)3 * threads * sizeof(double));
     // the shared-memory opt-in is per device; setting it twice is harmless,
     // so concurrent first launches from several host threads need no lock
     static std::atomic<unsigned long long> attr_set{0ull};
