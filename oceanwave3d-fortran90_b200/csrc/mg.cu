@@ -757,12 +757,13 @@ static bool tiled(const LevelTable<T>& pack, int l, int ld) {
 // MultiGridSolver.f90:5-192 (V cycle, gam = 1), levels lev[0] coarsest;
 // level ld is solved by the dense operator M. top is the level the cycle
 // started from, whose iterate receives the result; tiles allows the fused
-// tile kernels. Returns where level l's result is: a tiled level's smoothed
+// tile kernels; src, scale: the top level's right-hand side for them (null:
+// the level's own). Returns where level l's result is: a tiled level's smoothed
 // iterate goes out of place (from xv to rv, at the top from rv to xv),
 // because a tile's halo is read while its neighbours are written.
 template <typename T>
 static T* vcycle(LevelDev<T>* lev, int top, int l, int lc, int ld, const T* M, int nu1, int nu2, bool tiles,
-                 LevelTable<T>& pack, cudaStream_t st) {
+                 LevelTable<T>& pack, cudaStream_t st, const double* src = nullptr, const double* scale = nullptr) {
     if (l == ld) { launch_dense_apply(lev[l], M, st); return lev[l].xv; }
     // the fused coarse cycle takes all levels from lc down unless each of
     // them has its tile form
@@ -779,9 +780,9 @@ static T* vcycle(LevelDev<T>* lev, int top, int l, int lc, int ld, const T* M, i
         T* const xs = l == top ? F.rv : F.xv;
         T* const out = l == top ? F.xv : F.rv;
         const bool clear = l - 1 > ld && !(all || (l - 1 > lc && tiled(pack, l - 1, ld)));
-        launch_tile_down(F, Cc, pack.tile[l], (const T*)F.bv, xs, Cc.bv, clear ? Cc.xv : (T*)nullptr, st);
+        launch_tile_down(F, Cc, pack.tile[l], src, scale, xs, Cc.bv, clear ? Cc.xv : (T*)nullptr, st);
         const T* const xc = vcycle(lev, top, l - 1, lc, ld, M, nu1, nu2, tiles, pack, st);
-        launch_tile_up(F, Cc, pack.tile[l], (const T*)F.bv, (const T*)xs, xc, out, st);
+        launch_tile_up(F, Cc, pack.tile[l], src, scale, (const T*)xs, xc, out, st);
         return out;
     }
     if (pack.lex) launch_lo_smooth_lex(F, nu1, st);
@@ -810,24 +811,34 @@ void launch_mg_subcycle(LevelDev<T>* lev, int nlev, int l, int ld, const T* M, i
     vcycle(lev, l, l, lc, ld, M, nu1, nu2, false, pack, st);
 }
 
-// MultiGridSolveLinearSystem.f90:26-91: u = 0, then maxit cycles.
+// MultiGridSolveLinearSystem.f90:26-91: u = 0, then maxit cycles, for the
+// right-hand side src * *scale (scale null: 1).
 template <typename T>
-void launch_mg_vcycle(LevelDev<T>* lev, int nlev, const T* M, int ld, int nu1, int nu2, int maxit, LevelTable<T>& pack,
-                      cudaStream_t st) {
+void launch_mg_vcycle(LevelDev<T>* lev, int nlev, const double* src, const double* scale, const T* M, int ld, int nu1,
+                      int nu2, int maxit, LevelTable<T>& pack, cudaStream_t st) {
     LevelDev<T>& F = lev[nlev - 1];
     const bool tiles = nlev > 1 && nu1 == 1 && nu2 == 1 && maxit == 1 && !pack.lex && pack.tile &&
                        g_tiles.load(std::memory_order_relaxed) != 0;
-    // a tiled finest level starts from a zero iterate by itself
-    if (!(tiles && tiled(pack, nlev - 1, ld))) launch_fill<T>(F.xv, T(0), F.N, st);
     const int lc = (nlev > 1 && !pack.lex) ? coop_level(lev, nlev) : -1;
+    // a tiled finest level starts from a zero iterate by itself and reads the
+    // solver's vector; whether it is tiled: as vcycle decides
+    bool fine = tiles && tiled(pack, nlev - 1, ld);
+    if (nlev - 1 <= lc)
+        for (int q = ld + 1; q < nlev; ++q) fine = fine && tiled(pack, q, ld);
+    if (!fine) {
+        launch_scale_copy_dev<T>(src, scale, F.bv, F.N, st);
+        launch_fill<T>(F.xv, T(0), F.N, st);
+        src = scale = nullptr;
+    }
     for (int it = 1; it <= maxit; ++it) {
         if (nlev == 1 && it > 1) break;
-        vcycle(lev, nlev - 1, nlev - 1, lc, ld, M, nu1, nu2, tiles, pack, st);
+        vcycle(lev, nlev - 1, nlev - 1, lc, ld, M, nu1, nu2, tiles, pack, st, src, scale);
     }
 }
 
 #define OW3D_INST(T)                                                                                         \
-    template void launch_mg_vcycle<T>(LevelDev<T>*, int, const T*, int, int, int, int, LevelTable<T>&, cudaStream_t); \
+    template void launch_mg_vcycle<T>(LevelDev<T>*, int, const double*, const double*, const T*, int, int, int, int, \
+                                      LevelTable<T>&, cudaStream_t);                                         \
     template void launch_mg_subcycle<T>(LevelDev<T>*, int, int, int, const T*, int, int, LevelTable<T>&, cudaStream_t); \
     template void launch_dense_apply<T>(const LevelDev<T>&, const T*, cudaStream_t);                        \
     template void launch_lo_matvec<T>(const LevelDev<T>&, const T*, T*, cudaStream_t);                      \

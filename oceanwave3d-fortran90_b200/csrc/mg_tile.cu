@@ -32,7 +32,7 @@ namespace ow3d {
 namespace {
 using namespace mgdev;
 
-constexpr int kCrossThreads = 512;
+constexpr int kCrossThreads = 512, kUniThreads = 320;
 constexpr size_t kTileSmemMax = 220 * 1024, kTileSmemTwo = 112 * 1024;
 
 // Core and staged region of a block, 1-based columns; on a periodic level i
@@ -82,6 +82,12 @@ __device__ __forceinline__ int gcol(int i, int Nxg, int per) {
     return 2 + t;
 }
 
+// a / b for 0 <= a < 2^20, 1 <= b, rb = recip(b): exact (the quotient of
+// a + 1/2 is at least 1 / (2 b) away from an integer, the error of the product
+// below that), a few instructions where an integer division is some twenty-five.
+__device__ __forceinline__ int quot(int a, float rb) { return (int)(((float)a + 0.5f) * rb); }
+__device__ __forceinline__ float recip(int b) { return __fdividef(1.0f, (float)b); }
+
 template <typename T> struct Pair;
 template <> struct Pair<double> { using type = double2; };
 template <> struct Pair<float> { using type = float2; };
@@ -93,37 +99,40 @@ __device__ __forceinline__ typename Pair<T>::type pair_at(const T* p) {
 // Visit H rows of W columns of Nzg values each: a thread keeps one place k in
 // the column (N rows: 2 where Nzg is even -- a pair then lies on its own
 // alignment -- else 1) and steps through the columns, U visits in flight, so
-// that an access costs a few additions of index arithmetic. acc.ld<N>(v, c, q)
-// reads column c of row q, acc.st<N>(c, q, v) stores; acc is made for the
-// thread's k.
-template <int N, int U, typename T, int M, typename ACC>
-__device__ __forceinline__ void sweep_n(int W, int H, int Nzg, ACC make) {
-    const int nu = Nzg / N, cg = threadIdx.x / nu, step = blockDim.x / nu;
+// that an access costs a few additions of index arithmetic. acc.ld(v, c, q)
+// only loads what column c of row q needs (no branch, no arithmetic on the
+// values: either would hold up the loads of the visits after it), acc.st(c, q,
+// v) does the rest; acc is made for the thread's k.
+template <int N, int U, typename MAKE>
+__device__ __forceinline__ void sweep_n(int W, int H, int Nzg, MAKE make) {
+    const int nu = Nzg / N;
+    const float rnu = recip(nu), rw = recip(W);
+    const int cg = quot(threadIdx.x, rnu), step = quot(blockDim.x, rnu);
     if (cg >= step) return;
     const auto acc = make(N * (threadIdx.x - cg * nu));
-    int q = cg / W, c = cg - q * W;
-    const int dq = step / W, dc = step - dq * W;
+    int q = quot(cg, rw), c = cg - q * W;
+    const int dq = quot(step, rw), dc = step - dq * W;
     while (q < H) {
-        T v[U][M * N];
+        typename decltype(make(0))::template Val<N> v[U];
         int cc[U], qq[U];
 #pragma unroll
         for (int m = 0; m < U; ++m) {
             cc[m] = c;
             qq[m] = q;
-            if (q < H) acc.template ld<N>(v[m], c, q);
+            if (q < H) acc.ld(v[m], c, q);
             c += dc;
             q += dq;
             if (c >= W) { c -= W; ++q; }
         }
 #pragma unroll
         for (int m = 0; m < U; ++m)
-            if (qq[m] < H) acc.template st<N>(cc[m], qq[m], v[m]);
+            if (qq[m] < H) acc.st(cc[m], qq[m], v[m]);
     }
 }
-template <int U, typename T, int M, typename ACC>
-__device__ __forceinline__ void sweep(int W, int H, int Nzg, ACC make) {
-    if ((Nzg & 1) == 0) sweep_n<2, U, T, M>(W, H, Nzg, make);
-    else sweep_n<1, U, T, M>(W, H, Nzg, make);
+template <int U, typename MAKE>
+__device__ __forceinline__ void sweep(int W, int H, int Nzg, MAKE make) {
+    if ((Nzg & 1) == 0) sweep_n<2, U>(W, H, Nzg, make);
+    else sweep_n<1, U>(W, H, Nzg, make);
 }
 template <typename T>
 __device__ __forceinline__ void put_pair(T* p, T a, T b) {
@@ -171,8 +180,9 @@ __device__ __forceinline__ void colour_columns(int Nxg, int Nyg, int per, const 
         js = 2;
     }
     const int ni = (ihi - ilo + 2) >> 1, nj = jhi >= jlo ? (jhi - jlo) / js + 1 : 0;
+    const float rni = recip(ni);
     for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
-        const int tj = t / ni, j = jlo + tj * js;
+        const int tj = quot(t, rni), j = jlo + tj * js;
         const int par = four ? colour & 1 : (colour + j) & 1;
         const int i = ilo + ((ilo ^ par) & 1) + 2 * (t - tj * ni);
         if (i <= ihi) f(i, j);
@@ -185,10 +195,13 @@ __device__ __forceinline__ void all_columns(int Nxg, int Nyg, int per, const Reg
     int ilo = r.ia - d, ihi = r.ib + d, jlo = 1, jhi = 1;
     if (!per) { ilo = max(ilo, 2); ihi = min(ihi, Nxg - 1); }
     if (THREE) { jlo = max(r.ja - d, 2); jhi = min(r.jb + d, Nyg - 1); }
-    const int ni = max(ihi - ilo + 1, 0), nj = max(jhi - jlo + 1, 0);
+    // in a row first every other column, then the rest: a warp's columns lie
+    // side by side in shared memory
+    const int ni = max(ihi - ilo + 1, 0), nj = max(jhi - jlo + 1, 0), first = (ni + 1) >> 1;
+    const float rni = recip(ni);
     for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
-        const int tj = t / ni;
-        f(ilo + t - tj * ni, jlo + tj);
+        const int tj = quot(t, rni), q = t - tj * ni;
+        f(ilo + (q < first ? 2 * q : 2 * (q - first) + 1), jlo + tj);
     }
 }
 
@@ -197,17 +210,16 @@ __device__ __forceinline__ void all_columns(int Nxg, int Nyg, int per, const Reg
 // the nearest, whether the wall is an x wall, 0 or 1 for the low or high one)
 // for the 0-based rows k = 1..Nzg-1. All walls in one loop.
 template <bool THREE, typename F>
-__device__ __forceinline__ void ghost_rows(int Nxg, int Nyg, int per, int Nzg, uint32_t mz, int sz, const Reg& r,
-                                           const TileGeo& g, F f) {
+__device__ __forceinline__ void ghost_rows(int Nxg, int Nyg, int per, int Nzg, const Reg& r, const TileGeo& g, F f) {
     const int jlo = THREE ? max(r.sa, 2) : 1, jhi = THREE ? min(r.sb, Nyg - 1) : 1;
     const int ilo = per ? r.ra : max(r.ra, 2), ihi = per ? r.rb : min(r.rb, Nxg - 1);
     const int nx = jhi - jlo + 1, ny = ihi - ilo + 1;
     const int n0 = !per && r.ra == 1 ? nx : 0, n1 = n0 + (!per && r.rb == Nxg ? nx : 0);
     const int n2 = n1 + (THREE && r.sa == 1 ? ny : 0), n3 = n2 + (THREE && r.sb == Nyg ? ny : 0);
-    const int row = 2 * g.HW * g.NZP;
-    for (int t = threadIdx.x; t < n3 * Nzg; t += blockDim.x) {
-        const int q = (int)div32((uint32_t)t, mz, sz), k = t - q * Nzg;
-        if (k == 0) continue;
+    const int row = 2 * g.HW * g.NZP, nk = Nzg - 1;
+    const float rnk = recip(nk);
+    for (int t = threadIdx.x; t < n3 * nk; t += blockDim.x) {
+        const int q = quot(t, rnk), k = 1 + t - q * nk;
         const bool xw = q < n1;
         const int side = xw ? (q >= n0) : (q >= n2);
         const int p = q - (xw ? (side ? n0 : 0) : (side ? n2 : n1));
@@ -222,7 +234,8 @@ __device__ __forceinline__ void ghost_rows(int Nxg, int Nyg, int per, int Nzg, u
 }
 
 // The same two rows at a time (arrays of even pitch): f(place of the pair in
-// the ghost column, the nearest, the second; x wall; side; first row).
+// the ghost column, the nearest, the second; i + j of the nearest; x wall;
+// side; first row).
 template <bool THREE, typename F>
 __device__ __forceinline__ void ghost_pairs(int Nxg, int Nyg, int per, const Reg& r, const TileGeo& g, F f) {
     const int jlo = THREE ? max(r.sa, 2) : 1, jhi = THREE ? min(r.sb, Nyg - 1) : 1;
@@ -231,17 +244,18 @@ __device__ __forceinline__ void ghost_pairs(int Nxg, int Nyg, int per, const Reg
     const int n0 = !per && r.ra == 1 ? nx : 0, n1 = n0 + (!per && r.rb == Nxg ? nx : 0);
     const int n2 = n1 + (THREE && r.sa == 1 ? ny : 0), n3 = n2 + (THREE && r.sb == Nyg ? ny : 0);
     const int row = row_slot(g, 1);
+    const float rnp = recip(g.np);
     for (int t = threadIdx.x; t < n3 * g.np; t += blockDim.x) {
-        const int q = (int)div32((uint32_t)t, g.mnp, g.snp), k = 2 * (t - q * g.np);
+        const int q = quot(t, rnp), k = 2 * (t - q * g.np);
         const bool xw = q < n1;
         const int side = xw ? (q >= n0) : (q >= n2);
         const int p = q - (xw ? (side ? n0 : 0) : (side ? n2 : n1));
         if (xw) {
             const int d = side ? -1 : 1, li = (side ? Nxg : 1) - r.ra, o = row_slot(g, jlo + p - r.sa) + k;
-            f(o + col_slot(g, li), o + col_slot(g, li + d), o + col_slot(g, li + 2 * d), true, side, k);
+            f(o + col_slot(g, li), o + col_slot(g, li + d), o + col_slot(g, li + 2 * d), li + d + r.ra + jlo + p, true, side, k);
         } else {
             const int d = side ? -row : row, s = slot(g, ilo + p - r.ra, (side ? Nyg : 1) - r.sa) + k;
-            f(s, s + d, s + 2 * d, false, side, k);
+            f(s, s + d, s + 2 * d, ilo + p + (side ? Nyg - 1 : 2), false, side, k);
         }
     }
 }
@@ -271,8 +285,9 @@ __device__ __forceinline__ void restrict_tile(const LevelDev<T>& F, const LevelD
     const int nx = chi - clo + 1, ny = dhi - dlo + 1;
     constexpr int P = 4;
     const int part = threadIdx.x % P;
+    const float rnx = recip(nx);
     for (int cq = threadIdx.x / P; cq < nx * ny; cq += blockDim.x / P) {
-        const int cj = cq / nx, ic = clo + cq - cj * nx, jc = dlo + cj;
+        const int cj = quot(cq, rnx), ic = clo + cq - cj * nx, jc = dlo + cj;
         T* const ro = rc + (int64_t)Ncz * ((ic - 1) + Cc.Nxg * (jc - 1));
         T* const zo = zero ? zero + (ro - rc) : nullptr;
         const bool ghost = (!per && (ic == 1 || ic == Cc.Nxg)) || (THREE && (jc == 1 || jc == Cc.Nyg));
@@ -344,10 +359,26 @@ __device__ __forceinline__ void restrict_tile(const LevelDev<T>& F, const LevelD
     }
 }
 
+// A level's right-hand side as the kernels read it: of the level's own type, or
+// for the finest level the solver's FP64 vector times *scale (null: 1), which
+// saves a pass that scales and converts it.
+template <typename TB>
+struct Rhs {
+    const TB* p;
+    const double* scale;
+};
+template <typename T, typename TB>
+__device__ __forceinline__ T rhs_value(TB v, double s) {
+    if constexpr (sizeof(TB) == 8) return T(s * v);
+    else return v;
+}
+
 // Accessor of stage_up (sweep_n).
-template <typename T, bool THREE, bool VEC>
+template <typename T, typename TB, bool THREE, bool VEC>
 struct UpAcc {
-    const T *b, *x, *xc;        // at column 1 of the region's first row, and the coarse field, at the thread's k
+    const TB* b;                // at column 1 of the region's first row and the thread's k
+    double scale;
+    const T *x, *xc;            // likewise; the coarse field at the thread's k
     T *xs, *bs;
     const LevelDev<T>& F;
     const LevelDev<T>& Cc;
@@ -355,63 +386,70 @@ struct UpAcc {
     int ra, sa, k;
     bool first, last;           // this k is the bottom row / ends in the free-surface row
     template <int N>
-    __device__ __forceinline__ void avg(T* o, const T* c0, const T* c1, int i0, int i1) const {
-        T a[N], e[N];
-        get<N>(a, c0 + i0);
-        get<N>(e, c0 + i1);
-#pragma unroll
-        for (int n = 0; n < N; ++n) o[n] = a[n] + e[n];
-        if (THREE) {
-            get<N>(a, c1 + i0);
-            get<N>(e, c1 + i1);
-        }
-#pragma unroll
-        for (int n = 0; n < N; ++n) o[n] = THREE ? T(0.25) * (o[n] + (a[n] + e[n])) : T(0.5) * o[n];
-    }
-    // v: N values of x, then N of b
-    template <int N>
-    __device__ __forceinline__ void ld(T* v, int c, int q) const {
-        const int i = gcol(ra + c, F.Nxg, F.per), j = sa + q;
-        const int e = F.Nzg * (i - 1 + F.Nxg * q);
-        get<N>(v, x + e);
-        get<N>(v + N, b + e);
-        if ((!F.per && (i == 1 || i == F.Nxg)) || (THREE && (j == 1 || j == F.Nyg))) return;
-        const int Ncz = Cc.Nzg;
-        int i0 = Cc.xc ? 1 + ((i - 2) >> 1) : i - 1;   // 0-based coarse columns
-        int i1 = Cc.xc ? i0 + (i & 1) : i0;
+    struct Val { T x[N]; TB b[N]; T c[THREE ? 4 : 2][N]; };
+    // the coarse columns around fine column i (0-based, in values), row j's two
+    __device__ __forceinline__ void coarse_cols(int i, int& i0, int& i1) const {
+        i0 = Cc.xc ? 1 + ((i - 2) >> 1) : i - 1;
+        i1 = Cc.xc ? i0 + (i & 1) : i0;
         if (F.per && i1 == Cc.Nxg - 2) i1 = 1;
-        i0 *= Ncz;
-        i1 *= Ncz;
-        const int j0 = !THREE ? 0 : (Cc.yc ? 1 + ((j - 2) >> 1) : j - 1);
-        const T* const c0 = xc + Ncz * Cc.Nxg * j0;
-        const T* const c1 = c0 + (THREE && Cc.yc && (j & 1) ? Ncz * Cc.Nxg : 0);
-        T d[N];
-        if (!Cc.zc) {
-            avg<N>(d, c0, c1, i0, i1);
-            if (!first) v[0] += d[0];
-            if (N == 2) { if (!last) v[N - 1] += d[N - 1]; }
-            else if (last && !first) v[0] -= d[0];
-            return;
+        i0 *= Cc.Nzg;
+        i1 *= Cc.Nzg;
+    }
+    __device__ __forceinline__ void coarse_rows(int j, const T*& c0, const T*& c1) const {
+        const int nrow = Cc.Nzg * Cc.Nxg, j0 = !THREE ? 0 : (Cc.yc ? 1 + ((j - 2) >> 1) : j - 1);
+        c0 = xc + nrow * j0;
+        c1 = c0 + (THREE && Cc.yc && (j & 1) ? nrow : 0);
+    }
+    template <int N>
+    __device__ __forceinline__ void ld(Val<N>& v, int c, int q) const {
+        const int i = gcol(ra + c, F.Nxg, F.per);
+        const int e = F.Nzg * (i - 1 + F.Nxg * q);
+        get<N>(v.x, x + e);
+        get<N>(v.b, b + e);
+        if (Cc.zc) return;      // (uniform) the sigma form loads in st
+        int i0, i1;             // in range on ghost columns too
+        coarse_cols(i, i0, i1);
+        const T *c0, *c1;
+        coarse_rows(sa + q, c0, c1);
+        get<N>(v.c[0], c0 + i0);
+        get<N>(v.c[1], c0 + i1);
+        if constexpr (THREE) {
+            get<N>(v.c[2], c1 + i0);
+            get<N>(v.c[3], c1 + i1);
         }
+    }
+    template <int N>
+    __device__ __forceinline__ void st(int c, int q, const Val<N>& v) const {
+        const int i = gcol(ra + c, F.Nxg, F.per), j = sa + q;
+        const bool ghost = (!F.per && (i == 1 || i == F.Nxg)) || (THREE && (j == 1 || j == F.Nyg));
+        T xv[N], bv[N];
 #pragma unroll
         for (int n = 0; n < N; ++n) {
-            const int kk = k + n;
-            if (kk < 1 || kk > F.Nzg - 2) continue;
-            const int z0 = __ldg(F.piz + 2 * kk) - 1, z1 = __ldg(F.piz + 2 * kk + 1) - 1;
-            avg<1>(d, c0 + z0, c1 + z0, i0, i1);
-            v[n] += __ldg(F.pwz + 2 * kk) * d[0];
-            const T w1 = __ldg(F.pwz + 2 * kk + 1);
-            if (w1 != T(0)) {
-                avg<1>(d, c0 + z1, c1 + z1, i0, i1);
-                v[n] += w1 * d[0];
+            xv[n] = v.x[n];
+            bv[n] = rhs_value<T>(v.b[n], scale);
+            if (!Cc.zc) {
+                T d = v.c[0][n] + v.c[1][n];
+                if constexpr (THREE) d = T(0.25) * (d + (v.c[2][n] + v.c[3][n]));
+                else d = T(0.5) * d;
+                if (!ghost && !(first && n == 0) && !(last && n == N - 1)) xv[n] += d;
+            } else if (!ghost && k + n >= 1 && k + n <= F.Nzg - 2) {
+                int i0, i1;
+                coarse_cols(i, i0, i1);
+                const T *c0, *c1;
+                coarse_rows(j, c0, c1);
+                auto avg = [&](int z) -> T {
+                    const T d = c0[i0 + z] + c0[i1 + z];
+                    return THREE ? T(0.25) * (d + (c1[i0 + z] + c1[i1 + z])) : T(0.5) * d;
+                };
+                const int kk = k + n;
+                const T w1 = __ldg(F.pwz + 2 * kk + 1);
+                xv[n] += __ldg(F.pwz + 2 * kk) * avg(__ldg(F.piz + 2 * kk) - 1);
+                if (w1 != T(0)) xv[n] += w1 * avg(__ldg(F.piz + 2 * kk + 1) - 1);
             }
         }
-    }
-    template <int N>
-    __device__ __forceinline__ void st(int c, int q, const T* v) const {
         const int s = slot(g, c, q);
-        put<N, VEC>(xs + s, v);
-        put<N, VEC>(bs + s, v + N);
+        put<N, VEC>(xs + s, xv);
+        put<N, VEC>(bs + s, bv);
     }
 };
 
@@ -420,58 +458,67 @@ struct UpAcc {
 // point, in sigma by the level's table where the coarse grid is coarsened
 // there too; ghost columns, bottom and free-surface rows take no correction)
 // in xs and the right-hand side in bs.
-template <bool THREE, bool VEC, typename T>
+template <bool THREE, bool VEC, typename T, typename TB>
 __device__ __forceinline__ void stage_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileGeo& g, const Reg& r,
-                                         const T* __restrict__ b, const T* __restrict__ xin, const T* __restrict__ xc,
-                                         T* xs, T* bs) {
+                                         const TB* __restrict__ b, const double* __restrict__ bscale,
+                                         const T* __restrict__ xin, const T* __restrict__ xc, T* xs, T* bs) {
     const int64_t o = (int64_t)F.Nzg * F.Nxg * (r.sa - 1);
-    sweep<2, T, 2>(r.W, r.H, F.Nzg, [&](int k) {
+    const double scale = bscale ? *bscale : 1.0;
+    sweep<2>(r.W, r.H, F.Nzg, [&](int k) {
         const int end = k + ((F.Nzg & 1) == 0 ? 1 : 0);
-        return UpAcc<T, THREE, VEC>{b + o + k, xin + o + k, xc + (Cc.zc ? 0 : k), xs + k, bs + k, F, Cc, g, r.ra, r.sa, k,
-                                    k == 0, end == F.Nzg - 1};
+        return UpAcc<T, TB, THREE, VEC>{b + o + k, scale, xin + o + k, xc + (Cc.zc ? 0 : k), xs + k, bs + k, F, Cc, g,
+                                        r.ra, r.sa, k, k == 0, end == F.Nzg - 1};
     });
 }
 
-// Accessor of stage_down (sweep_n).
-template <typename T, bool THREE, bool VEC>
+// Accessor of stage_down (sweep_n); INPLACE: the right-hand side goes where the
+// iterate will be.
+template <typename T, typename TB, bool THREE, bool VEC, bool INPLACE>
 struct DownAcc {
-    const T* b;                 // at the thread's k
+    const TB* b;                // at column 1 of the region's first row and the thread's k
+    double scale;
     T *xs, *bs;
     const TileGeo& g;
     const T (*gx)[3], (*gy)[3];
     int ra, sa, Nxg, Nyg, per, nz;
     bool first;                 // this k is the bottom row
+    bool wall;                  // the region touches a wall
     template <int N>
-    __device__ __forceinline__ void ld(T* v, int c, int q) const {
-        get<N>(v, b + nz * (gcol(ra + c, Nxg, per) - 1 + Nxg * q));
+    struct Val { TB b[N]; };
+    template <int N>
+    __device__ __forceinline__ void ld(Val<N>& v, int c, int q) const {
+        get<N>(v.b, b + nz * (gcol(ra + c, Nxg, per) - 1 + Nxg * q));
     }
     template <int N>
-    __device__ __forceinline__ void st(int c, int q, const T* v) const {
+    __device__ __forceinline__ void st(int c, int q, const Val<N>& v) const {
         const int s = slot(g, c, q), i = ra + c, j = sa + q;
-        put<N, VEC>(bs + s, v);
-        T x[N];
+        T bv[N], x[N];
 #pragma unroll
-        for (int n = 0; n < N; ++n) x[n] = T(0);
+        for (int n = 0; n < N; ++n) { bv[n] = rhs_value<T>(v.b[n], scale); x[n] = INPLACE ? bv[n] : T(0); }
+        if (!INPLACE) put<N, VEC>(bs + s, bv);
         const bool x0 = !per && i == 1, x1 = !per && i == Nxg, y0 = THREE && j == 1, y1 = THREE && j == Nyg;
-        if (x0 || x1 || y0 || y1) {
+        if (wall && (x0 || x1 || y0 || y1)) {
             const T w = (x0 || x1) && (y0 || y1) ? T(1) : (gx ? (x0 || x1 ? gx[x1][2] : gy[y1][2]) : T(0));
 #pragma unroll
-            for (int n = 0; n < N; ++n) x[n] = first && n == 0 ? v[n] : w * v[n];
+            for (int n = 0; n < N; ++n) x[n] = first && n == 0 ? bv[n] : w * bv[n];
         }
         put<N, VEC>(xs + s, x);
     }
 };
 
-// Stage the right-hand side in bs and in xs the zero iterate with its identity
-// rows (corner columns, level 1 of the ghost columns: b) and, gx[w][2] and
-// gy[w][2] being one over the ghost weight of wall w, its ghost rows relaxed
-// (null: left at zero).
-template <bool THREE, bool VEC, typename T>
+// Stage the right-hand side in bs and in xs the zero iterate (INPLACE: in xs
+// the right-hand side) with the identity rows (corner columns, level 1 of the
+// ghost columns: b) and, gx[w][2] and gy[w][2] being one over the ghost weight
+// of wall w, the ghost rows relaxed (null: left at zero).
+template <bool THREE, bool VEC, bool INPLACE, typename T, typename TB>
 __device__ __forceinline__ void stage_down(const LevelDev<T>& F, const TileGeo& g, const Reg& r,
-                                           const T* __restrict__ b, T* xs, T* bs, const T (*gx)[3], const T (*gy)[3]) {
+                                           const TB* __restrict__ b, const double* __restrict__ bscale, T* xs, T* bs,
+                                           const T (*gx)[3], const T (*gy)[3]) {
     const int64_t o = (int64_t)F.Nzg * F.Nxg * (r.sa - 1);
-    sweep<4, T, 1>(r.W, r.H, F.Nzg, [&](int k) {
-        return DownAcc<T, THREE, VEC>{b + o + k, xs + k, bs + k, g, gx, gy, r.ra, r.sa, F.Nxg, F.Nyg, F.per, F.Nzg, k == 0};
+    const double scale = bscale ? *bscale : 1.0;
+    sweep<4>(r.W, r.H, F.Nzg, [&](int k) {
+        return DownAcc<T, TB, THREE, VEC, INPLACE>{b + o + k, scale, xs + k, bs + k, g, gx, gy, r.ra, r.sa, F.Nxg, F.Nyg, F.per,
+                                          F.Nzg, k == 0, at_wall(F.Nxg, F.Nyg, F.per, r, THREE)};
     });
 }
 
@@ -483,18 +530,20 @@ struct CoreAcc {
     const TileGeo& g;
     int c0, q0, nz, Nxg;
     template <int N>
-    __device__ __forceinline__ void ld(T* v, int c, int q) const {
+    struct Val { T x[N]; };
+    template <int N>
+    __device__ __forceinline__ void ld(Val<N>& v, int c, int q) const {
         const T* const p = xs + slot(g, c + c0, q + q0);
         if constexpr (N == 2 && VEC) {
-            get<2>(v, p);
+            get<2>(v.x, p);
         } else {
 #pragma unroll
-            for (int n = 0; n < N; ++n) v[n] = p[n];
+            for (int n = 0; n < N; ++n) v.x[n] = p[n];
         }
     }
     template <int N>
-    __device__ __forceinline__ void st(int c, int q, const T* v) const {
-        put<N, true>(out + nz * (c + Nxg * q), v);
+    __device__ __forceinline__ void st(int c, int q, const Val<N>& v) const {
+        put<N, true>(out + nz * (c + Nxg * q), v.x);
     }
 };
 
@@ -505,7 +554,7 @@ __device__ __forceinline__ void write_core(const LevelDev<T>& F, const Reg& r, c
                                            T* __restrict__ out) {
     const int Nzg = F.Nzg, Nxg = F.Nxg, H = r.jb - r.ja + 1;
     T* const o = out + (int64_t)Nzg * ((r.ia - 1) + (int64_t)Nxg * (r.ja - 1));
-    sweep<4, T, 1>(r.ib - r.ia + 1, H, Nzg, [&](int k) {
+    sweep<4>(r.ib - r.ia + 1, H, Nzg, [&](int k) {
         return CoreAcc<T, VEC>{xs + k, o + k, g, r.ia - r.ra, r.ja - r.sa, Nzg, Nxg};
     });
     if (F.per && bx == 0)
@@ -536,30 +585,35 @@ __device__ __forceinline__ void uni_off(const UniTab<T>& u, const T* xp, int l, 
     }
 }
 
+// Rows of a column whose sums are formed together: enough loads in flight,
+// few enough for the registers of two blocks per SM (18 rows at once spill).
+__host__ __device__ constexpr int uni_chunk(int nzg) { return nzg == 0 ? 8 : (nzg <= 10 ? (nzg + 1) / 2 * 2 : 6); }
+
 // Rows 2..Nzg-1 of the column at xp bottom to top, then its bottom row and
 // its free-surface row: x_k = (b_k - off_k - up_k x_{k+1}) id_k - g_k x_{k-1}.
-// All rows' sums are formed before the first new value is stored, so their
+// A chunk's sums are formed before its first new value is stored, so their
 // loads are in flight together and only the chain's one multiply-add per row
 // is serial. off(k, o): the neighbour columns' part of rows k, k + 1; ZERO: the
 // column's own old iterate is zero.
 template <int NZG, bool ZERO, typename T, typename OFF>
 __device__ __forceinline__ void uni_column(const UniTab<T>& u, int nzg, T* xp, const T* bp, OFF off) {
     const int Nzg = NZG > 0 ? NZG : nzg;
-    constexpr int CH = NZG > 0 ? (NZG + 1) / 2 * 2 : 8;   // rows per chunk
+    constexpr int CH = uni_chunk(NZG);
     const T b1 = bp[0];
     T xprev = ZERO ? b1 * u.t6 : (b1 - u.t0 * xp[1] - u.t1 * xp[2]) * u.t6;
     T x2 = 0, x3 = 0;
+#pragma unroll
     for (int k0 = 0; k0 < Nzg; k0 += CH) {
         T q[CH], xo[CH + 1];
         if (!ZERO) {
 #pragma unroll
             for (int m = 0; m < CH; m += 2)
-                if (NZG > 0 || k0 + m < Nzg) { const auto v = pair_at(xp + k0 + m); xo[m] = v.x; xo[m + 1] = v.y; }
-            xo[CH] = NZG == 0 && k0 + CH < Nzg ? xp[k0 + CH] : T(0);
+                if (k0 + m < Nzg) { const auto v = pair_at(xp + k0 + m); xo[m] = v.x; xo[m + 1] = v.y; }
+            xo[CH] = k0 + CH < Nzg ? xp[k0 + CH] : T(0);
         }
 #pragma unroll
         for (int m = 0; m < CH; m += 2) {
-            if (NZG == 0 && k0 + m >= Nzg) continue;
+            if (k0 + m >= Nzg) continue;
             const auto v = pair_at(bp + k0 + m);
             T o[2];
             off(k0 + m, o);
@@ -583,53 +637,175 @@ __device__ __forceinline__ void uni_column(const UniTab<T>& u, int nzg, T* xp, c
         }
 #pragma unroll
         for (int m = 0; m < CH; m += 2)
-            if (NZG > 0 || k0 + m < Nzg) put_pair(xp + k0 + m, q[m], q[m + 1]);   // the free-surface row: b
+            if (k0 + m < Nzg) put_pair(xp + k0 + m, q[m], q[m + 1]);   // the free-surface row: b
     }
     xp[0] = (b1 - u.t0 * x2 - u.t1 * x3) * u.t6;
 }
 
-// Replace the right-hand side of the column's rows 2..Nzg-1 by the residual.
-template <bool THREE, int NZG, typename T>
-__device__ __forceinline__ void uni_residual(const UniTab<T>& u, int nzg, const T* xp, T* bp, int l, int r, int row) {
-    const int Nzg = NZG > 0 ? NZG : nzg;
-    constexpr int CH = NZG > 0 ? (NZG + 1) / 2 * 2 : 8;
-    T xm = 0;
-    for (int k0 = 0; k0 < Nzg; k0 += CH) {
-        T x[CH + 2];            // rows k0 - 1 .. k0 + CH
-        x[0] = xm;
-#pragma unroll
-        for (int m = 0; m < CH; m += 2)
-            if (NZG > 0 || k0 + m < Nzg) { const auto v = pair_at(xp + k0 + m); x[m + 1] = v.x; x[m + 2] = v.y; }
-        x[CH + 1] = NZG == 0 && k0 + CH < Nzg ? xp[k0 + CH] : T(0);
-        xm = x[CH];
-#pragma unroll
-        for (int m = 0; m < CH; m += 2) {
-            if (NZG == 0 && k0 + m >= Nzg) continue;
-            const auto v = pair_at(bp + k0 + m);
-            T q[2] = {v.x, v.y}, o[2];
-            uni_off<THREE>(u, xp, l, r, row, k0 + m, o);
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                const int k = k0 + m + n, i = m + n + 1;
-                if (k >= 1 && k < Nzg - 1) q[n] -= o[n] + u.lo[k] * x[i - 1] + u.up[k] * x[i + 1] + u.dg[k] * x[i];
-            }
-            put_pair(bp + k0 + m, q[0], q[1]);
+// Down, in place: xs holds b and is overwritten by the iterate column by
+// column -- from x = 0 a colour-0 column reads no column but ghosts, a colour-1
+// column only colour-0 and ghost columns -- and then by the residual, which
+// follows from what changed after a row was solved, so b is not needed again:
+//   colour 1: -up x_{k+1};  colour 0: that and -w x of its colour-1
+//   neighbours; next to a wall, the change of the ghost value; in row 2 the
+//   second update of the bottom row.
+// Colour 0's residual first (it reads colour 1's iterate), then colour 1's
+// (its own column only).
+
+// Colour 0 (FIRST) or 1 of the smoothing step, at distance <= 3 or 2.
+template <bool THREE, int NZG, bool FIRST, typename T>
+__device__ __forceinline__ void uni_first(const LevelDev<T>& F, const UniTab<T>& u, const TileGeo& g, const Reg& r, T* xs) {
+    const int Nxg = F.Nxg, Nyg = F.Nyg, per = F.per, row = row_slot(g, 1);
+    colour_columns<THREE>(Nxg, Nyg, per, r, 2, FIRST ? 0 : 1, FIRST ? 3 : 2, [&](int i, int j) {
+        const int li = i - r.ra, l = near_l(g, li), h = near_r(g, li);
+        T* const xp = xs + slot(g, li, j - r.sa);
+        if (!FIRST) {
+            uni_column<NZG, true>(u, F.Nzg, xp, xp, [&](int k, T* o) { uni_off<THREE>(u, xp, l, h, row, k, o); });
+            return;
         }
-    }
+        const bool el = !per && i == 2, er = !per && i == Nxg - 1, ed = THREE && j == 2, eu = THREE && j == Nyg - 1;
+        if (el || er || ed || eu) {
+            uni_column<NZG, true>(u, F.Nzg, xp, xp, [&](int k, T* o) {
+                o[0] = o[1] = T(0);
+                auto add = [&](bool on, T w, int at) {
+                    if (!on) return;
+                    const auto v = pair_at(xp + at + k);
+                    o[0] += w * v.x;
+                    o[1] += w * v.y;
+                };
+                add(el, u.wxl, l);
+                add(er, u.wxr, h);
+                add(ed, u.wyd, -row);
+                add(eu, u.wyu, row);
+            });
+        } else {
+            uni_column<NZG, true>(u, F.Nzg, xp, xp, [&](int, T* o) { o[0] = o[1] = T(0); });
+        }
+    });
 }
 
-// One smoothing step on the staged iterate: colour c at distance <= d - c,
-// the ghost rows relaxed before, between and after. ZERO: the iterate is zero
-// and its ghost rows are relaxed; colour 0 then reads no neighbour columns but
-// ghosts, so it may reach the region's edge.
-template <bool THREE, int NZG, bool ZERO, typename T>
+// The columns of one colour at distance <= 1: residual in place.
+template <bool THREE, int NZG, bool FIRST, typename T>
+__device__ __forceinline__ void uni_residual(const LevelDev<T>& F, const UniTab<T>& u, const TileGeo& g, const Reg& r,
+                                             T* xs) {
+    const int Nxg = F.Nxg, Nyg = F.Nyg, per = F.per, row = row_slot(g, 1), Nzg = NZG > 0 ? NZG : F.Nzg;
+    constexpr int CH = uni_chunk(NZG);
+    // add(k, q): the side terms of rows k, k + 1
+    auto column = [&](T* xp, auto add) {
+        const T c2 = u.lo[1] * u.t6 * (u.t0 * xp[1] + u.t1 * xp[2]);   // the bottom row's second update
+#pragma unroll
+        for (int k0 = 0; k0 < Nzg; k0 += CH) {
+            T x[CH + 1], q[CH];
+#pragma unroll
+            for (int m = 0; m < CH; m += 2)
+                if (k0 + m < Nzg) { const auto v = pair_at(xp + k0 + m); x[m] = v.x; x[m + 1] = v.y; }
+            x[CH] = k0 + CH < Nzg ? xp[k0 + CH] : T(0);
+#pragma unroll
+            for (int m = 0; m < CH; m += 2) {
+                if (k0 + m >= Nzg) continue;
+                T o[2] = {T(0), T(0)};
+                add(k0 + m, o);
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    const int k = k0 + m + n;
+                    q[m + n] = x[m + n];
+                    if (k >= 1 && k < Nzg - 1) q[m + n] = o[n] - u.up[k] * x[m + n + 1] + (k == 1 ? c2 : T(0));
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < CH; m += 2)
+                if (k0 + m < Nzg) put_pair(xp + k0 + m, q[m], q[m + 1]);
+        }
+    };
+    colour_columns<THREE>(Nxg, Nyg, per, r, 2, FIRST ? 0 : 1, 1, [&](int i, int j) {
+        const int li = i - r.ra, l = near_l(g, li), h = near_r(g, li);
+        T* const xp = xs + slot(g, li, j - r.sa);
+        const bool el = !per && i == 2, er = !per && i == Nxg - 1, ed = THREE && j == 2, eu = THREE && j == Nyg - 1;
+        if (el || er || ed || eu) {
+            column(xp, [&](int k, T* o) {
+                // a ghost neighbour moved by -(wa x_near + wb x_second) / wg since the row was solved
+                auto side = [&](bool wall, T w, const T* gw, int at, int opposite) {
+                    if (wall) {
+                        const auto v = pair_at(xp + k);
+                        const T c = w * gw[2];
+                        T d0 = gw[0] * v.x, d1 = gw[0] * v.y;
+                        if (FIRST) { const auto z = pair_at(xp + opposite + k); d0 += gw[1] * z.x; d1 += gw[1] * z.y; }
+                        o[0] += c * d0;
+                        o[1] += c * d1;
+                    } else if (FIRST) {
+                        const auto z = pair_at(xp + at + k);
+                        o[0] -= w * z.x;
+                        o[1] -= w * z.y;
+                    }
+                };
+                side(el, u.wxl, u.gx[0], l, h);
+                side(er, u.wxr, u.gx[1], h, l);
+                if (THREE) {
+                    side(ed, u.wyd, u.gy[0], -row, row);
+                    side(eu, u.wyu, u.gy[1], row, -row);
+                }
+            });
+        } else if (FIRST) {
+            column(xp, [&](int k, T* o) {
+                uni_off<THREE>(u, xp, l, h, row, k, o);
+                o[0] = -o[0];
+                o[1] = -o[1];
+            });
+        } else {
+            column(xp, [&](int, T*) {});
+        }
+    });
+}
+
+template <typename T, typename TB, bool THREE, int NZG>
+__global__ void __launch_bounds__(kUniThreads, sizeof(T) == 8 ? 2 : 3)
+    k_mg_down_uni(LevelDev<T> F, LevelDev<T> Cc, const TB* __restrict__ b, const double* __restrict__ scale,
+                  T* __restrict__ xout, T* __restrict__ rc, T* __restrict__ zero, const __grid_constant__ UniTab<T> u,
+                  TileGeo g) {
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    T* const xs = reinterpret_cast<T*>(tile_smem);
+    const int bx = blockIdx.x, by = blockIdx.y;
+    const Reg r = region(F.Nxg, F.Nyg, F.per, g, bx, by, THREE);
+    const bool wall = at_wall(F.Nxg, F.Nyg, F.per, r, THREE);
+    stage_down<THREE, true, true>(F, g, r, b, scale, xs, xs, u.gx, u.gy);
+    __syncthreads();
+    // ghost rows: the contribution of the colour just solved
+    auto ghosts = [&](int colour) {
+        if (!wall) return;
+        ghost_pairs<THREE>(F.Nxg, F.Nyg, F.per, r, g, [&](int s, int sa, int sb, int ij, bool xw, int side, int k) {
+            const T* const w = xw ? u.gx[side] : u.gy[side];
+            const bool near = (ij & 1) == colour;
+            const auto v = pair_at(xs + s), a = pair_at(xs + (near ? sa : sb));
+            const T c = (near ? w[0] : w[1]) * w[2];
+            put_pair(xs + s, k == 0 ? v.x : v.x - c * a.x, v.y - c * a.y);   // level 1: an identity row
+        });
+        __syncthreads();
+    };
+    uni_first<THREE, NZG, true>(F, u, g, r, xs);
+    __syncthreads();
+    ghosts(0);
+    uni_first<THREE, NZG, false>(F, u, g, r, xs);
+    __syncthreads();
+    ghosts(1);
+    write_core<THREE, true>(F, r, g, bx, xs, xout);
+    __syncthreads();
+    uni_residual<THREE, NZG, true>(F, u, g, r, xs);
+    __syncthreads();
+    uni_residual<THREE, NZG, false>(F, u, g, r, xs);
+    __syncthreads();
+    restrict_tile<THREE, true>(F, Cc, g, r, bx, xs, rc, zero);
+}
+
+// One smoothing step on the staged iterate: colour c at distance <= 1 - c, the
+// ghost rows relaxed before, between and after.
+template <bool THREE, int NZG, typename T>
 __device__ __forceinline__ void uni_smooth(const LevelDev<T>& F, const UniTab<T>& u, const TileGeo& g, const Reg& r,
-                                           T* xs, const T* bs, int d) {
-    const int Nxg = F.Nxg, Nyg = F.Nyg, per = F.per;
-    const bool wall = at_wall(Nxg, Nyg, per, r, THREE);
+                                           T* xs, const T* bs) {
+    const bool wall = at_wall(F.Nxg, F.Nyg, F.per, r, THREE);
     auto ghosts = [&]() {
         if (!wall) return;
-        ghost_pairs<THREE>(Nxg, Nyg, per, r, g, [&](int s, int sa, int sb, bool xw, int side, int k) {
+        ghost_pairs<THREE>(F.Nxg, F.Nyg, F.per, r, g, [&](int s, int sa, int sb, int, bool xw, int side, int k) {
             const T* const w = xw ? u.gx[side] : u.gy[side];
             const auto b = pair_at(bs + s), a = pair_at(xs + sa), c = pair_at(xs + sb);
             const T v0 = (b.x - w[0] * a.x - w[1] * c.x) * w[2], v1 = (b.y - w[0] * a.y - w[1] * c.y) * w[2];
@@ -637,66 +813,22 @@ __device__ __forceinline__ void uni_smooth(const LevelDev<T>& F, const UniTab<T>
         });
         __syncthreads();
     };
-    if (!ZERO) ghosts();
+    ghosts();
     const int row = row_slot(g, 1);
     for (int colour = 0; colour < 2; ++colour) {
-        colour_columns<THREE>(Nxg, Nyg, per, r, 2, colour, d - colour, [&](int i, int j) {
+        colour_columns<THREE>(F.Nxg, F.Nyg, F.per, r, 2, colour, 1 - colour, [&](int i, int j) {
             const int li = i - r.ra, s = slot(g, li, j - r.sa), l = near_l(g, li), h = near_r(g, li);
             T* const xp = xs + s;
-            if (ZERO && colour == 0) {
-                const bool el = !per && i == 2, er = !per && i == Nxg - 1;
-                const bool ed = THREE && j == 2, eu = THREE && j == Nyg - 1;
-                if (el || er || ed || eu) {
-                    uni_column<NZG, true>(u, F.Nzg, xp, bs + s, [&](int k, T* o) {
-                        o[0] = o[1] = T(0);
-                        auto add = [&](bool on, T w, int at) {
-                            if (!on) return;
-                            const auto v = pair_at(xp + at + k);
-                            o[0] += w * v.x;
-                            o[1] += w * v.y;
-                        };
-                        add(el, u.wxl, l);
-                        add(er, u.wxr, h);
-                        add(ed, u.wyd, -row);
-                        add(eu, u.wyu, row);
-                    });
-                } else {
-                    uni_column<NZG, true>(u, F.Nzg, xp, bs + s, [&](int, T* o) { o[0] = o[1] = T(0); });
-                }
-                return;
-            }
-            uni_column<NZG, ZERO>(u, F.Nzg, xp, bs + s, [&](int k, T* o) { uni_off<THREE>(u, xp, l, h, row, k, o); });
+            uni_column<NZG, false>(u, F.Nzg, xp, bs + s, [&](int k, T* o) { uni_off<THREE>(u, xp, l, h, row, k, o); });
         });
         __syncthreads();
         ghosts();
     }
 }
 
-template <typename T, bool THREE, int NZG>
-__global__ void __launch_bounds__(256, 2) k_mg_down_uni(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
-                                                     T* __restrict__ xout, T* __restrict__ rc, T* __restrict__ zero,
-                                                     const __grid_constant__ UniTab<T> u, TileGeo g) {
-    pdl_entry();
-    extern __shared__ __align__(16) unsigned char tile_smem[];
-    T* const xs = reinterpret_cast<T*>(tile_smem);
-    T* const bs = xs + 2 * g.HW * g.PH * g.NZP;
-    const int bx = blockIdx.x, by = blockIdx.y;
-    const Reg r = region(F.Nxg, F.Nyg, F.per, g, bx, by, THREE);
-    stage_down<THREE, true>(F, g, r, b, xs, bs, u.gx, u.gy);
-    __syncthreads();
-    uni_smooth<THREE, NZG, true>(F, u, g, r, xs, bs, 3);
-    write_core<THREE, true>(F, r, g, bx, xs, xout);
-    const int row = row_slot(g, 1);
-    all_columns<THREE>(F.Nxg, F.Nyg, F.per, r, 1, [&](int i, int j) {
-        const int li = i - r.ra, s = slot(g, li, j - r.sa);
-        uni_residual<THREE, NZG>(u, F.Nzg, xs + s, bs + s, near_l(g, li), near_r(g, li), row);
-    });
-    __syncthreads();
-    restrict_tile<THREE, true>(F, Cc, g, r, bx, bs, rc, zero);
-}
-
-template <typename T, bool THREE, int NZG>
-__global__ void __launch_bounds__(256, 2) k_mg_up_uni(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
+template <typename T, typename TB, bool THREE, int NZG>
+__global__ void __launch_bounds__(256, 2) k_mg_up_uni(LevelDev<T> F, LevelDev<T> Cc, const TB* __restrict__ b,
+                                                   const double* __restrict__ scale,
                                                    const T* __restrict__ xin, const T* __restrict__ xc,
                                                    T* __restrict__ out, const __grid_constant__ UniTab<T> u, TileGeo g) {
     pdl_entry();
@@ -705,9 +837,9 @@ __global__ void __launch_bounds__(256, 2) k_mg_up_uni(LevelDev<T> F, LevelDev<T>
     T* const bs = xs + 2 * g.HW * g.PH * g.NZP;
     const int bx = blockIdx.x, by = blockIdx.y;
     const Reg r = region(F.Nxg, F.Nyg, F.per, g, bx, by, THREE);
-    stage_up<THREE, true>(F, Cc, g, r, b, xin, xc, xs, bs);
+    stage_up<THREE, true>(F, Cc, g, r, b, scale, xin, xc, xs, bs);
     __syncthreads();
-    uni_smooth<THREE, NZG, false>(F, u, g, r, xs, bs, 1);
+    uni_smooth<THREE, NZG>(F, u, g, r, xs, bs);
     write_core<THREE, true>(F, r, g, bx, xs, out);
 }
 
@@ -804,9 +936,10 @@ __device__ __forceinline__ void cross_pass(const LevelDev<T>& F, const RowTab<T>
     const int ka = 1 + 2 * rr, kb = ka + 1;
     const int kac = min(ka, Nzg - 1), kbc = min(kb, Nzg - 1);
     const int nrow = row_slot(g, 1);
+    const float rni = recip(ni);
     for (int base = (threadIdx.x >> 5) * per_warp; base < total; base += step) {
         const int q = base + lane / S;
-        const int tq = min(q, total - 1), tj = tq / ni, j = jlo + tj * js;
+        const int tq = min(q, total - 1), tj = quot(tq, rni), j = jlo + tj * js;
         const int par = four ? colour & 1 : (colour + j) & 1;
         int i = RES ? ilo + tq - tj * ni : ilo + ((ilo ^ par) & 1) + 2 * (tq - tj * ni);
         const bool act = q < total && i <= ihi;
@@ -916,7 +1049,7 @@ __device__ __forceinline__ void cross_bottoms(const LevelDev<T>& F, const RowTab
 template <typename T, bool THREE>
 __device__ __forceinline__ void cross_ghosts(const LevelDev<T>& F, const RowTab<T>& t, const Reg& r, const TileGeo& g,
                                              const CrossTile<T>& w, int ncolor, int post, int pre) {
-    ghost_rows<THREE>(F.Nxg, F.Nyg, 0, F.Nzg, F.mz32, F.sz32, r, g, [&](int s, int sa, int sb, int ni, int nj, bool xw,
+    ghost_rows<THREE>(F.Nxg, F.Nyg, 0, F.Nzg, r, g, [&](int s, int sa, int sb, int ni, int nj, bool xw,
                                                                         int side) {
         auto has = [&](int i, int j, int colour) {
             return ncolor == 4 ? ((i & 1) == (colour & 1) && (j & 1) == (colour >> 1)) : ((i + j) & 1) == colour;
@@ -953,8 +1086,9 @@ __device__ __forceinline__ CrossTile<T> cross_arrays(const TileGeo& g, T* sm) {
 }
 template <bool THREE, typename T>
 __device__ __forceinline__ void stage_cf(const LevelDev<T>& F, const TileGeo& g, const Reg& r, T* cf) {
+    const float rw = recip(r.W);
     for (int q = threadIdx.x; q < r.W * r.H; q += blockDim.x) {
-        const int lj = q / r.W, li = q - lj * r.W;
+        const int lj = quot(q, rw), li = q - lj * r.W;
         T a, b, c, d;
         load_cf(F.cf, (int64_t)(r.ra + li - 1) + (int64_t)F.Nxg * (r.sa + lj - 1), a, b, c, d);
         T* const o = cf + 4 * ((lj * 2 + (li & 1)) * g.HW + (li >> 1));
@@ -964,6 +1098,7 @@ __device__ __forceinline__ void stage_cf(const LevelDev<T>& F, const TileGeo& g,
 
 template <typename T, bool THREE, int S>
 __global__ void __launch_bounds__(kCrossThreads) k_mg_down_cross(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
+                                                       const double* __restrict__ scale,
                                                                  T* __restrict__ xout, T* __restrict__ rc,
                                                                  T* __restrict__ zero,
                                                                  const __grid_constant__ RowTab<T> t, TileGeo g) {
@@ -973,7 +1108,7 @@ __global__ void __launch_bounds__(kCrossThreads) k_mg_down_cross(LevelDev<T> F, 
     const int nc = F.ncolor, bx = blockIdx.x, by = blockIdx.y;
     const Reg r = region(F.Nxg, F.Nyg, 0, g, bx, by, THREE);
     stage_cf<THREE>(F, g, r, w.cf);
-    stage_down<THREE, false>(F, g, r, b, w.xs, w.bs, (const T(*)[3])nullptr, (const T(*)[3])nullptr);
+    stage_down<THREE, false, false>(F, g, r, b, scale, w.xs, w.bs, (const T(*)[3])nullptr, (const T(*)[3])nullptr);
     __syncthreads();
     cross_bottoms<T, THREE, true>(F, t, g, r, w, g.halo);
     cross_smooth<T, THREE, S>(F, t, g, r, w, nc + 2, 2);
@@ -985,6 +1120,7 @@ __global__ void __launch_bounds__(kCrossThreads) k_mg_down_cross(LevelDev<T> F, 
 
 template <typename T, bool THREE, int S>
 __global__ void __launch_bounds__(kCrossThreads) k_mg_up_cross(LevelDev<T> F, LevelDev<T> Cc, const T* __restrict__ b,
+                                                       const double* __restrict__ scale,
                                                                const T* __restrict__ xin, const T* __restrict__ xc,
                                                                T* __restrict__ out,
                                                                const __grid_constant__ RowTab<T> t, TileGeo g) {
@@ -994,7 +1130,7 @@ __global__ void __launch_bounds__(kCrossThreads) k_mg_up_cross(LevelDev<T> F, Le
     const int nc = F.ncolor, bx = blockIdx.x, by = blockIdx.y;
     const Reg r = region(F.Nxg, F.Nyg, 0, g, bx, by, THREE);
     stage_cf<THREE>(F, g, r, w.cf);
-    stage_up<THREE, false>(F, Cc, g, r, b, xin, xc, w.xs, w.bs);
+    stage_up<THREE, false>(F, Cc, g, r, b, scale, xin, xc, w.xs, w.bs);
     __syncthreads();
     cross_bottoms<T, THREE, false>(F, t, g, r, w, nc + 1);
     cross_smooth<T, THREE, S>(F, t, g, r, w, nc, 0);
@@ -1010,7 +1146,7 @@ inline int tile_pitch(int nzg, bool cross) { return cross ? nzg | 1 : ((nzg + 1)
 
 // Cores, slots and shared memory of a launch over all its tiles.
 template <typename T>
-void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross) {
+void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross, bool down) {
     const bool three = L.Nyg > 1;
     auto cores = [](int n, int c, int& nt, int& q, int& rem, int& most) {
         nt = (n + c - 1) / c;
@@ -1024,14 +1160,14 @@ void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross) {
     else { g.nty = 1; g.qy = 1; g.remy = 0; g.cy = 1; }
     g.NZP = tile_pitch(L.Nzg, cross);
     g.np = (L.Nzg + 1) / 2;
-    div_magic32((uint32_t)g.np, g.mnp, g.snp);
     int W = 0, H = 0;
     for (int bx = 0; bx < g.ntx; ++bx) W = std::max(W, region(L.Nxg, L.Nyg, L.per, g, bx, 0, three).W);
     for (int by = 0; by < g.nty; ++by) H = std::max(H, region(L.Nxg, L.Nyg, L.per, g, 0, by, three).H);
     g.HW = (W + 1) / 2;
     g.PH = H;
     const size_t cols = (size_t)2 * g.HW * g.PH;
-    g.smem = (cols * g.NZP * 2 + (cross ? 4 * cols : 0)) * sizeof(T);   // iterate, right-hand side, coefficients
+    // iterate, right-hand side (uniform levels on the way down: in one place), coefficients
+    g.smem = (cols * g.NZP * (cross || !down ? 2 : 1) + (cross ? 4 * cols : 0)) * sizeof(T);
 }
 
 }  // namespace
@@ -1045,16 +1181,16 @@ void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
     static const int line[][2] = {{64, 1}, {32, 1}, {16, 1}};
     const int (*cand)[2] = three ? (cross ? cross3 : uni3) : line;
     const int ncand = three && cross ? 4 : 3;
-    auto pick = [&](TileGeo& g, int halo) {
+    auto pick = [&](TileGeo& g, int halo, bool down) {
         g.halo = halo;
         bool found = false;
         TileGeo best{};
         for (int q = 0; q < ncand; ++q) {
-            size_geo(L, g, cand[q][0], cand[q][1], cross);
+            size_geo(L, g, cand[q][0], cand[q][1], cross, down);
             if (g.smem > kTileSmemMax || (g.smem > kTileSmemTwo && q + 1 < ncand)) continue;
             const int lanes = cross ? (L.Nzg <= 10 ? 4 : (L.Nzg <= 18 ? 8 : 16)) : 1;
             const int cols = (g.cx + 2 * halo) * (three ? g.cy + 2 * halo : 1) / L.ncolor * lanes;
-            g.threads = std::max(256, std::min(cross ? kCrossThreads : 256, (cols + 31) / 32 * 32));
+            g.threads = std::max(256, std::min(cross ? kCrossThreads : (down ? kUniThreads : 256), (cols + 31) / 32 * 32));
             found = true;
             best = g;
             if (g.ntx * g.nty >= 148) break;
@@ -1064,7 +1200,7 @@ void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
     };
     if (t.mode == kTileNone) return;
     const int nc = L.ncolor;
-    if (!pick(t.down, cross ? nc + 3 : 3) || !pick(t.up, cross ? nc + 2 : 2)) t.mode = kTileNone;
+    if (!pick(t.down, cross ? nc + 3 : 3, true) || !pick(t.up, cross ? nc + 2 : 2, false)) t.mode = kTileNone;
 }
 
 namespace {
@@ -1079,87 +1215,100 @@ void allow_smem(K kernel, std::atomic<unsigned long long>& set) {
     }
 }
 
-template <typename T, bool THREE, int NZG>
-void down_uni(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, T* xs, T* rc, T* zero,
+template <typename T, typename TB, bool THREE, int NZG>
+void down_uni(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, Rhs<TB> b, T* xs, T* rc, T* zero,
               cudaStream_t st) {
     static std::atomic<unsigned long long> set{0ull};
     const TileGeo& g = t.down;
-    allow_smem(k_mg_down_uni<T, THREE, NZG>, set);
-    launch_k(k_mg_down_uni<T, THREE, NZG>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc,
-             b, xs, rc, zero, t.u, g);
+    allow_smem(k_mg_down_uni<T, TB, THREE, NZG>, set);
+    launch_k(k_mg_down_uni<T, TB, THREE, NZG>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem,
+             st, F, Cc, b.p, b.scale, xs, rc, zero, t.u, g);
 }
-template <typename T, bool THREE, int NZG>
-void up_uni(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, const T* xs, const T* xc,
+template <typename T, typename TB, bool THREE, int NZG>
+void up_uni(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, Rhs<TB> b, const T* xs, const T* xc,
             T* out, cudaStream_t st) {
     static std::atomic<unsigned long long> set{0ull};
     const TileGeo& g = t.up;
-    allow_smem(k_mg_up_uni<T, THREE, NZG>, set);
-    launch_k(k_mg_up_uni<T, THREE, NZG>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc, b,
-             xs, xc, out, t.u, g);
+    allow_smem(k_mg_up_uni<T, TB, THREE, NZG>, set);
+    launch_k(k_mg_up_uni<T, TB, THREE, NZG>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem,
+             st, F, Cc, b.p, b.scale, xs, xc, out, t.u, g);
 }
-template <typename T, bool THREE, int S>
-void down_cross(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, T* xs, T* rc, T* zero,
+template <typename T, typename TB, bool THREE, int S>
+void down_cross(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, Rhs<TB> b, T* xs, T* rc, T* zero,
                 cudaStream_t st) {
     static std::atomic<unsigned long long> set{0ull};
     const TileGeo& g = t.down;
     allow_smem(k_mg_down_cross<T, THREE, S>, set);
-    launch_k(k_mg_down_cross<T, THREE, S>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc,
-             b, xs, rc, zero, t.r, g);
+    launch_k(k_mg_down_cross<T, THREE, S>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st,
+             F, Cc, b.p, b.scale, xs, rc, zero, t.r, g);
 }
-template <typename T, bool THREE, int S>
-void up_cross(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, const T* xs, const T* xc,
+template <typename T, typename TB, bool THREE, int S>
+void up_cross(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, Rhs<TB> b, const T* xs, const T* xc,
               T* out, cudaStream_t st) {
     static std::atomic<unsigned long long> set{0ull};
     const TileGeo& g = t.up;
     allow_smem(k_mg_up_cross<T, THREE, S>, set);
-    launch_k(k_mg_up_cross<T, THREE, S>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F, Cc, b,
-             xs, xc, out, t.r, g);
+    launch_k(k_mg_up_cross<T, THREE, S>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st, F,
+             Cc, b.p, b.scale, xs, xc, out, t.r, g);
 }
-}  // namespace
 
 // Uniform levels: the level counts of the decks' usual Nz unrolled. Cross
 // levels (FP64): the lanes per column, two rows each.
-#define OW3D_TILE(way, ...)                                                \
-    do {                                                                   \
-        if (t.mode == kTileUniform) {                                      \
-            if (F.Nyg > 1) {                                               \
-                if (F.Nzg == 18) way##_uni<T, true, 18>(__VA_ARGS__);      \
-                else if (F.Nzg == 10) way##_uni<T, true, 10>(__VA_ARGS__); \
-                else way##_uni<T, true, 0>(__VA_ARGS__);                   \
-            } else {                                                       \
-                if (F.Nzg == 10) way##_uni<T, false, 10>(__VA_ARGS__);     \
-                else way##_uni<T, false, 0>(__VA_ARGS__);                  \
-            }                                                              \
-        } else if constexpr (sizeof(T) == 8) {                             \
-            if (F.Nyg > 1) {                                               \
-                if (F.Nzg <= 10) way##_cross<T, true, 4>(__VA_ARGS__);     \
-                else if (F.Nzg <= 18) way##_cross<T, true, 8>(__VA_ARGS__); \
-                else way##_cross<T, true, 16>(__VA_ARGS__);                \
-            } else {                                                       \
-                if (F.Nzg <= 10) way##_cross<T, false, 4>(__VA_ARGS__);    \
-                else if (F.Nzg <= 18) way##_cross<T, false, 8>(__VA_ARGS__); \
-                else way##_cross<T, false, 16>(__VA_ARGS__);               \
-            }                                                              \
-        }                                                                  \
+#define OW3D_TILE(way, ...)                                                    \
+    do {                                                                       \
+        if (t.mode == kTileUniform) {                                          \
+            if (F.Nyg > 1) {                                                   \
+                if (F.Nzg == 18) way##_uni<T, TB, true, 18>(__VA_ARGS__);      \
+                else if (F.Nzg == 10) way##_uni<T, TB, true, 10>(__VA_ARGS__); \
+                else way##_uni<T, TB, true, 0>(__VA_ARGS__);                   \
+            } else {                                                           \
+                if (F.Nzg == 10) way##_uni<T, TB, false, 10>(__VA_ARGS__);     \
+                else way##_uni<T, TB, false, 0>(__VA_ARGS__);                  \
+            }                                                                  \
+        } else if constexpr (sizeof(T) == 8) {                                 \
+            if (F.Nyg > 1) {                                                   \
+                if (F.Nzg <= 10) way##_cross<T, TB, true, 4>(__VA_ARGS__);     \
+                else if (F.Nzg <= 18) way##_cross<T, TB, true, 8>(__VA_ARGS__); \
+                else way##_cross<T, TB, true, 16>(__VA_ARGS__);                \
+            } else {                                                           \
+                if (F.Nzg <= 10) way##_cross<T, TB, false, 4>(__VA_ARGS__);    \
+                else if (F.Nzg <= 18) way##_cross<T, TB, false, 8>(__VA_ARGS__); \
+                else way##_cross<T, TB, false, 16>(__VA_ARGS__);               \
+            }                                                                  \
+        }                                                                      \
     } while (0)
 
-template <typename T>
-void launch_tile_down(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, T* xs, T* rc,
-                      T* zero, cudaStream_t st) {
+template <typename T, typename TB>
+void down(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, Rhs<TB> b, T* xs, T* rc, T* zero,
+          cudaStream_t st) {
     OW3D_TILE(down, F, Cc, t, b, xs, rc, zero, st);
 }
-template <typename T>
-void launch_tile_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, const T* xs,
-                    const T* xc, T* out, cudaStream_t st) {
+template <typename T, typename TB>
+void up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, Rhs<TB> b, const T* xs, const T* xc, T* out,
+        cudaStream_t st) {
     OW3D_TILE(up, F, Cc, t, b, xs, xc, out, st);
+}
+}  // namespace
+
+template <typename T>
+void launch_tile_down(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const double* src,
+                      const double* scale, T* xs, T* rc, T* zero, cudaStream_t st) {
+    if (src) down<T, double>(F, Cc, t, Rhs<double>{src, scale}, xs, rc, zero, st);
+    else down<T, T>(F, Cc, t, Rhs<T>{F.bv, nullptr}, xs, rc, zero, st);
+}
+template <typename T>
+void launch_tile_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const double* src,
+                    const double* scale, const T* xs, const T* xc, T* out, cudaStream_t st) {
+    if (src) up<T, double>(F, Cc, t, Rhs<double>{src, scale}, xs, xc, out, st);
+    else up<T, T>(F, Cc, t, Rhs<T>{F.bv, nullptr}, xs, xc, out, st);
 }
 
 #define OW3D_INST(T)                                                                                              \
     template void tile_geometry<T>(const LevelDev<T>&, TileLevel<T>&);                                            \
-    template void launch_tile_down<T>(const LevelDev<T>&, const LevelDev<T>&, const TileLevel<T>&, const T*, T*,  \
-                                      T*, T*, cudaStream_t);                                                      \
-    template void launch_tile_up<T>(const LevelDev<T>&, const LevelDev<T>&, const TileLevel<T>&, const T*,        \
-                                    const T*, const T*, T*, cudaStream_t);
+    template void launch_tile_down<T>(const LevelDev<T>&, const LevelDev<T>&, const TileLevel<T>&, const double*, \
+                                      const double*, T*, T*, T*, cudaStream_t);                                   \
+    template void launch_tile_up<T>(const LevelDev<T>&, const LevelDev<T>&, const TileLevel<T>&, const double*,   \
+                                    const double*, const T*, const T*, T*, cudaStream_t);
 OW3D_INST(double)
 OW3D_INST(float)
 #undef OW3D_INST

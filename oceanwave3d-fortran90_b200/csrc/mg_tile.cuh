@@ -36,8 +36,7 @@ struct RowTab {
 // PH rows.
 struct TileGeo {
     int cx, cy, ntx, nty, qx, remx, qy, remy, halo, HW, PH, NZP, threads;
-    uint32_t mnp;             // division by the row pairs of a column (div32)
-    int snp, np;
+    int np;                   // row pairs of a column
     size_t smem;
 };
 
@@ -54,15 +53,18 @@ struct TileLevel {
 template <typename T>
 void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t);
 
+// The right-hand side of both: the level's own (F.bv) when src is null, else
+// src * *scale (scale null: 1), rounded to the level's type.
+//
 // Pre-smoothing from x = 0 (one step), residual and restriction of level F
 // into rc (level Cc's right-hand side); the smoothed iterate goes to xs.
 // zero: iterate of level Cc to clear, or null.
 template <typename T>
-void launch_tile_down(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, T* xs, T* rc,
-                      T* zero, cudaStream_t st);
+void launch_tile_down(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const double* src,
+                      const double* scale, T* xs, T* rc, T* zero, cudaStream_t st);
 // Correction xs + P xc and one post-smoothing step, into out (not xs).
 template <typename T>
-void launch_tile_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const T* b, const T* xs,
-                    const T* xc, T* out, cudaStream_t st);
+void launch_tile_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t, const double* src,
+                    const double* scale, const T* xs, const T* xc, T* out, cudaStream_t st);
 
 }  // namespace ow3d

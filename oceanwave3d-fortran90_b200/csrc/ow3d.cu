@@ -522,12 +522,11 @@ void run_precond(ow3d_handle* H, MgSet<T>& S, const double* src, const double* d
     LevelDev<T>* lev = S.lev.data();
     const int L = (int)S.lev.size();
     LevelDev<T>& F = lev[L - 1];
-    launch_scale_copy_dev<T>(src, dscale, S.fine_b, F.N, H->st);
     F.xv = out;
     if (S.table.lex)  // the recursion to the coarsest level, as the reference runs it
-        launch_mg_vcycle<T>(lev, L, S.coarse_inv, 0, H->p.nu1, H->p.nu2, H->p.maxit, S.table, H->st);
+        launch_mg_vcycle<T>(lev, L, src, dscale, S.coarse_inv, 0, H->p.nu1, H->p.nu2, H->p.maxit, S.table, H->st);
     else
-        launch_mg_vcycle<T>(lev, L, S.dense_op, S.dense_level, H->p.nu1, H->p.nu2, H->p.maxit, S.table, H->st);
+        launch_mg_vcycle<T>(lev, L, src, dscale, S.dense_op, S.dense_level, H->p.nu1, H->p.nu2, H->p.maxit, S.table, H->st);
 }
 
 // Apply M^{-1} to src (times *dscale) into the FP64 vector dst.

@@ -255,8 +255,8 @@ struct LevelTable {
 
 // M: dense operator of level ld (the coarsest level's inverse when ld = 0).
 template <typename T>
-void launch_mg_vcycle(LevelDev<T>* lev, int nlev, const T* M, int ld, int nu1, int nu2, int maxit,
-                      LevelTable<T>& pack, cudaStream_t st);
+void launch_mg_vcycle(LevelDev<T>* lev, int nlev, const double* src, const double* scale, const T* M, int ld, int nu1,
+                      int nu2, int maxit, LevelTable<T>& pack, cudaStream_t st);
 template <typename T>
 void launch_mg_subcycle(LevelDev<T>* lev, int nlev, int l, int ld, const T* M, int nu1, int nu2,
                         LevelTable<T>& pack, cudaStream_t st);
