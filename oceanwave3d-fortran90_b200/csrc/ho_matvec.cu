@@ -136,10 +136,10 @@ __device__ __forceinline__ void band_col(int64_t q, int Nxg, int Nyg, bool all, 
 // point of whole columns. sp, sx, sy: the block's shared phi, d/dx and d/dy of
 // this thread's column, level by level. All threads of the block call it;
 // those without a point (on false) only join the barrier.
-template <bool THREE, typename TIN>
+template <bool THREE, typename TIN, typename ZT>
 __device__ void ho_point_general(const HoGrid& g, const Surface& s, const TIN* __restrict__ phi, double scale,
-                                 const double* __restrict__ b, double* __restrict__ y, int mode, int i, int j,
-                                 int k, bool on, double* sp, double* sx, double* sy) {
+                                 const double* __restrict__ b, double* __restrict__ y, int mode, const ZT& zt,
+                                 bool centred, int i, int j, int k, bool on, double* sp, double* sx, double* sy) {
     const int Nxg = g.Nxg, Nyg = g.Nyg, Nzg = g.Nzg;
     auto P = [&](int kk, int ii, int jj) -> double {   // 1-based
         return (double)__ldg(phi + (int64_t)(kk - 1) + (int64_t)Nzg * ((int64_t)(ii - 1) + (int64_t)Nxg * (jj - 1)));
@@ -178,6 +178,14 @@ __device__ void ho_point_general(const HoGrid& g, const Surface& s, const TIN* _
         // (ConstructTableCrossDerivatives.f90:173-186,231-235)
         const int wsx = g.per ? i - 3 : win_start(i, Nxg);
         double dx = 0, dxx = 0, dy = 0, dyy = 0;
+        if (centred && i > kBand && i <= Nxg - kBand) {   // the common stencil, from the constant bank
+#pragma unroll
+            for (int m = 0; m < kHoRank; ++m) {
+                const double q = P(k, i - 3 + m, j);
+                dx += zt.cx[0][m] * q;
+                dxx += zt.cx[1][m] * q;
+            }
+        } else
 #pragma unroll
         for (int m = 0; m < kHoRank; ++m) {
             const double q = P(k, g.per ? wrap_x(wsx + m, Nxg) : wsx + m, j);
@@ -191,6 +199,14 @@ __device__ void ho_point_general(const HoGrid& g, const Surface& s, const TIN* _
         }
         if (THREE) {
             const int wsy = win_start(j, Nyg);
+            if (centred && j > kBand && j <= Nyg - kBand) {
+#pragma unroll
+                for (int m = 0; m < kHoRank; ++m) {
+                    const double q = P(k, i, j - 3 + m);
+                    dy += zt.cy[0][m] * q;
+                    dyy += zt.cy[1][m] * q;
+                }
+            } else
 #pragma unroll
             for (int m = 0; m < kHoRank; ++m) {
                 const double q = P(k, i, wsy + m);
@@ -344,7 +360,7 @@ __global__ void __launch_bounds__(THREE ? 256 : 256, 2)
         if (on) band_col(q, Nxg, Nyg, all != 0, i, j);
         extern __shared__ __align__(16) unsigned char smraw[];
         double* const sp = reinterpret_cast<double*>(smraw) + c * Nzg;
-        ho_point_general<THREE, TIN>(g, s, phi, scale, b, y, mode, i, j, k, on, sp, sp + blockDim.x,
+        ho_point_general<THREE, TIN>(g, s, phi, scale, b, y, mode, zt, all > 1, i, j, k, on, sp, sp + blockDim.x,
                                      sp + 2 * blockDim.x);
         return;
     }
@@ -453,7 +469,7 @@ void launch_impl(const HoGrid& g, const Surface& s, const TIN* phi, const double
         attr_set.fetch_or(bit, std::memory_order_relaxed);
     }
     launch_k(k_ho_matvec<NZG, THREE, TIN>, dim3(band_blocks + tiles), dim3(threads), smem, st, 
-        g, s, phi, scale, b, y, mode, zt, band_blocks, nband, split ? 0 : 1, tiles_x);
+        g, s, phi, scale, b, y, mode, zt, band_blocks, nband, split ? 0 : (uniform && !g.per ? 2 : 1), tiles_x);
 }
 
 template <bool THREE, typename TIN>

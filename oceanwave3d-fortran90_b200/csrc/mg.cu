@@ -825,11 +825,13 @@ void launch_mg_vcycle(LevelDev<T>* lev, int nlev, const double* src, const doubl
     bool fine = tiles && tiled(pack, nlev - 1, ld);
     if (nlev - 1 <= lc)
         for (int q = ld + 1; q < nlev; ++q) fine = fine && tiled(pack, q, ld);
-    if (!fine) {
+    // (sloping FP32 levels read a vector of their own type)
+    const bool direct = fine && (sizeof(T) == 8 || pack.tile[nlev - 1].mode == kTileUniform);
+    if (!direct) {
         launch_scale_copy_dev<T>(src, scale, F.bv, F.N, st);
-        launch_fill<T>(F.xv, T(0), F.N, st);
         src = scale = nullptr;
     }
+    if (!fine) launch_fill<T>(F.xv, T(0), F.N, st);
     for (int it = 1; it <= maxit; ++it) {
         if (nlev == 1 && it > 1) break;
         vcycle(lev, nlev - 1, nlev - 1, lc, ld, M, nu1, nu2, tiles, pack, st, src, scale);

@@ -57,9 +57,14 @@ __device__ __forceinline__ void load_bt8(const float* bt, int64_t c, float* o) {
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
 }
 
+// Index of point (k, i, j) in the level's vectors, and of column (i, j).
 template <typename T>
 __device__ __forceinline__ int64_t IX(const LevelDev<T>& L, int k, int i, int j) {
-    return (int64_t)(k - 1) + (int64_t)L.Nzg * ((int64_t)(i - 1) + (int64_t)L.Nxg * (j - 1));
+    return (int64_t)(k - 1) + (int64_t)L.Nzg * ((int64_t)(i - 1) + (int64_t)L.pitch * (j - 1));
+}
+template <typename T>
+__device__ __forceinline__ int64_t IC(const LevelDev<T>& L, int i, int j) {
+    return (int64_t)(i - 1) + (int64_t)L.pitch * (j - 1);
 }
 // stencil tables are read-only for the whole solve
 template <typename T>
@@ -297,7 +302,8 @@ __device__ __forceinline__ void residual_point(const LevelDev<T>& L, int64_t p) 
 template <typename T, bool THREE>
 __device__ __forceinline__ T bottom_value(const LevelDev<T>& L, const T* X, const T* B, int64_t c, int i, int j, T x2,
                                           T x3) {
-    const int Nzg = L.Nzg, Nxg = L.Nxg;
+    const int Nzg = L.Nzg, Nxg = L.pitch;
+    const int64_t a = IC(L, i, j);
     const T hx = L.hx[c];
     const T hy = THREE ? L.hy[c] : T(0);
     T ih, ca, cb, c3;
@@ -306,15 +312,22 @@ __device__ __forceinline__ T bottom_value(const LevelDev<T>& L, const T* X, cons
     const T s2 = omb * ca, s4 = THREE ? omb * cb : T(0);
     const T f = THREE ? (ih + hx * s2 + hy * s4) : (ih + hx * s2);
     const T dz = sz(L, 1, 2, 1) * x2 + sz(L, 1, 2, 2) * x3;
-    T dx = sx(L, 1, i, 0) * X[(c - 1) * Nzg + 1] + sx(L, 1, i, 1) * x2;
-    dx += sx(L, 1, i, 2) * X[(c + 1) * Nzg + 1];
+    T dx = sx(L, 1, i, 0) * X[(a - 1) * Nzg + 1] + sx(L, 1, i, 1) * x2;
+    dx += sx(L, 1, i, 2) * X[(a + 1) * Nzg + 1];
     T off = f * dz + hx * dx;
     if (THREE) {
-        T dy = sy(L, 1, j, 0) * X[(c - Nxg) * Nzg + 1] + sy(L, 1, j, 1) * x2;
-        dy += sy(L, 1, j, 2) * X[(c + Nxg) * Nzg + 1];
+        T dy = sy(L, 1, j, 0) * X[(a - Nxg) * Nzg + 1] + sy(L, 1, j, 1) * x2;
+        dy += sy(L, 1, j, 2) * X[(a + Nxg) * Nzg + 1];
         off += hy * dy;
     }
-    return (B[c * Nzg] - off) / (f * sz(L, 1, 2, 0));
+    return (B[a * Nzg] - off) / (f * sz(L, 1, 2, 0));
+}
+
+template <typename T, bool THREE>
+__device__ __forceinline__ void bottom_column(const LevelDev<T>& L, int i, int j) {
+    T* const X = L.xv;
+    const int64_t c = (int64_t)(i - 1) + (int64_t)L.Nxg * (j - 1), a = IC(L, i, j);
+    X[a * L.Nzg] = bottom_value<T, THREE>(L, X, L.bv, c, i, j, X[a * L.Nzg + 1], X[a * L.Nzg + 2]);
 }
 
 // Level-1 pass item q (levels with mixed-derivative terms relax their level-1
@@ -333,8 +346,7 @@ __device__ __forceinline__ void bottom_item(const LevelDev<T>& L, int64_t q) {
     if (q < nint) {
         const int64_t tj = q / nxi;
         const int i = 2 + (int)(q - tj * nxi), j = THREE ? 2 + (int)tj : 1;
-        const int64_t c = (int64_t)(i - 1) + (int64_t)L.Nxg * (j - 1);
-        X[c * L.Nzg] = bottom_value<T, THREE>(L, X, L.bv, c, i, j, X[c * L.Nzg + 1], X[c * L.Nzg + 2]);
+        bottom_column<T, THREE>(L, i, j);
         return;
     }
     q -= nint;
@@ -387,47 +399,28 @@ __device__ __forceinline__ RowConst<T> row_const(const LevelDev<T>& L) {
     return c;
 }
 
+// The task of column (i, j) for its segment (act false: the segment joins the
+// warp's shuffles and stores nothing).
 template <typename T, bool THREE, int S, bool CROSS>
-__device__ void colour_warp(const LevelDev<T>& L, int colour, int base, const RowConst<T>& rk) {
+__device__ __forceinline__ void colour_col1(const LevelDev<T>& L, int i, int j, bool act, const RowConst<T>& rk) {
     const int Nxg = L.Nxg, Nyg = L.Nyg, Nzg = L.Nzg, R = Nzg - 2;
     const int lane = threadIdx.x & 31, r = lane & (S - 1);
-    const int nxi = Nxg - 2 - L.per, nyi = THREE ? Nyg - 2 : 1;
-    // columns of this colour: every other i (and every other j with 4 colours)
-    const bool four = (L.ncolor == 4);
-    const int ni = (nxi + 1) / 2;
-    const int nj = four ? (nyi + 1) / 2 : nyi;
-    const int total = ni * nj;                // columns of one colour (< 2^31)
     const unsigned segmask = 0xffffffffu;   // the whole warp runs the scan together
     T* const X = L.xv;
     const T* const B = L.bv;
-
-    const int q = base + (lane / S);
-    bool act = q < total;
-    int i = 2, j = THREE ? 2 : 1;
-    if (act) {
-        const int tj = q / ni, ti = q - tj * ni;   // 32-bit division
-        if (four) {
-            j = THREE ? 2 + 2 * tj + (colour >> 1) : 1;
-            i = 2 + 2 * ti + (colour & 1);
-        } else {
-            j = THREE ? 2 + tj : 1;
-            i = 2 + 2 * ti + ((colour + j) & 1);    // (i + j) & 1 == colour
-        }
-        act = (i <= Nxg - 1 - L.per) && (!THREE || j <= Nyg - 1);
-    }
     const bool rowact = act && (r < R);
     const int k = r + 2;
     // the column's base; neighbours and rows are 32-bit offsets from it
     // (every level has fewer than 2^31 points)
     const int c = (i - 1) + Nxg * (j - 1);
-    T* const xc = X + (int64_t)c * Nzg;
-    const T* const bc = B + (int64_t)c * Nzg;
-    const int ox = Nzg, oy = Nzg * Nxg;
+    T* const xc = X + IC(L, i, j) * Nzg;
+    const T* const bc = B + IC(L, i, j) * Nzg;
+    const int ox = Nzg, oy = Nzg * L.pitch;
     // the column borders a ghost column (ghost relaxation before or after it,
     // and the corner columns)
     const bool edge = act && (i <= 3 || i >= Nxg - 2 || (THREE && (j <= 3 || j >= Nyg - 2)));
 
-    auto colidx = [&](int ii, int jj) -> int64_t { return (int64_t)(ii - 1) + (int64_t)Nxg * (jj - 1); };
+    auto colidx = [&](int ii, int jj) -> int64_t { return IC(L, ii, jj); };
     // Relax ghost column cg: Neumann rows k = 2..Nzg with the 3-point stencil
     // wa x(ca) + wb x(cb) + wg x(cg) = b, identity row k = 1. With post set,
     // the value of this column (ca if own == 1, cb if own == 2) is the lane's
@@ -603,6 +596,34 @@ __device__ void colour_warp(const LevelDev<T>& L, int colour, int base, const Ro
     if (edge) ghosts(true, xn, xfs);
 }
 
+template <typename T, bool THREE, int S, bool CROSS>
+__device__ void colour_warp(const LevelDev<T>& L, int colour, int base, const RowConst<T>& rk) {
+    const int Nxg = L.Nxg, Nyg = L.Nyg;
+    const int lane = threadIdx.x & 31;
+    const int nxi = Nxg - 2 - L.per, nyi = THREE ? Nyg - 2 : 1;
+    // columns of this colour: every other i (and every other j with 4 colours)
+    const bool four = (L.ncolor == 4);
+    const int ni = (nxi + 1) / 2;
+    const int nj = four ? (nyi + 1) / 2 : nyi;
+    const int total = ni * nj;                // columns of one colour (< 2^31)
+
+    const int q = base + (lane / S);
+    bool act = q < total;
+    int i = 2, j = THREE ? 2 : 1;
+    if (act) {
+        const int tj = q / ni, ti = q - tj * ni;   // 32-bit division
+        if (four) {
+            j = THREE ? 2 + 2 * tj + (colour >> 1) : 1;
+            i = 2 + 2 * ti + (colour & 1);
+        } else {
+            j = THREE ? 2 + tj : 1;
+            i = 2 + 2 * ti + ((colour + j) & 1);    // (i + j) & 1 == colour
+        }
+        act = (i <= Nxg - 1 - L.per) && (!THREE || j <= Nyg - 1);
+    }
+    colour_col1<T, THREE, S, CROSS>(L, i, j, act, rk);
+}
+
 // Row constants of row k (clamped to the interior rows 2..Nzg-1).
 template <typename T>
 __device__ __forceinline__ RowConst<T> row_const_k(const LevelDev<T>& L, int k) {
@@ -643,12 +664,12 @@ __device__ __forceinline__ void colour_col2(const LevelDev<T>& L, int i, int j, 
     const bool va = act && ka <= Nzg - 1, vb = act && kb <= Nzg - 1;
     const int last = (R - 1) / 2;           // lane holding row Nzg-1 (the free surface follows it)
     const int c = (i - 1) + Nxg * (j - 1);
-    T* const xc = X + (int64_t)c * Nzg;
+    T* const xc = X + IC(L, i, j) * Nzg;
     const T* const bc = br;
     const int ox = Nzg;
     const bool edge = !TILE && act && (i <= 3 || i >= Nxg - 2 || (THREE && (j <= 3 || j >= Nyg - 2)));
 
-    auto colidx = [&](int ii, int jj) -> int64_t { return (int64_t)(ii - 1) + (int64_t)Nxg * (jj - 1); };
+    auto colidx = [&](int ii, int jj) -> int64_t { return IC(L, ii, jj); };
     // ghost column cg: Neumann rows of this lane's levels, wa x(ca) + wb x(cb) + wg x(cg) = b;
     // with post set, the value of this column (ca if own == 1, cb if own == 2)
     // is the lane's new one
@@ -942,7 +963,7 @@ __device__ void restrict_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const
         const int kf = 2 + (kc - 2) * (1 + zcz), ifn = 2 + (ic - 2) * (1 + xcz), jf = gy ? 2 + (jc - 2) * (1 + ycz) : 1;
         // fine values by 32-bit offsets from (kf, ifn, jf) (levels have < 2^31 points)
         const T* rb = rf + IX(F, kf, ifn, jf);
-        const int fox = F.Nzg, foy = F.Nzg * F.Nxg;
+        const int fox = F.Nzg, foy = F.Nzg * F.pitch;
         auto R = [&](int k, int i, int j) -> T { return rb[(k - kf) + (i - ifn) * fox + (j - jf) * foy]; };
         if (kf == F.Nzg) { rc[p] = R(kf, ifn, jf); return; }
         // x-weighted value at (k, ifn, j) (raw on ghost rows and outside 2..Nzf)
@@ -976,12 +997,11 @@ __device__ void restrict_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const
 // value is the weighted sum over (at most) 2 x 2 x 2 coarse points with the
 // fine level's per-direction tables. The free-surface row, the bottom ghost
 // row and the ghost columns are not touched.
+// prolong_value adds the correction of fine point (kf, ifn, jf) to *x.
 template <typename T>
-__device__ void prolong_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* xc, T* xf, int64_t p) {
+__device__ __forceinline__ void prolong_value(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* xc, T* x, int kf,
+                                              int ifn, int jf) {
     const int gy = (F.Nyg > 1) ? 1 : 0;
-    int kf, ifn, jf;
-    int64_t cfl;
-    decomp(F, p, kf, cfl, ifn, jf);
     if (kf == 1 || kf == F.Nzg || ifn == 1 || ifn == F.Nxg || (gy && (jf == 1 || jf == F.Nyg))) return;
     if (F.per && ifn == F.Nxg - 1) return;   // periodic x: the repeated column stays zero
     const int2 zi = __ldg(reinterpret_cast<const int2*>(F.piz) + (kf - 1));
@@ -1006,7 +1026,14 @@ __device__ void prolong_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const 
     };
     T v = wz0 * Py(zi.x);
     if (wz1 != T(0)) v += wz1 * Py(zi.y);
-    xf[p] += v;
+    *x += v;
+}
+template <typename T>
+__device__ void prolong_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* xc, T* xf, int64_t p) {
+    int kf, ifn, jf;
+    int64_t cfl;
+    decomp(F, p, kf, cfl, ifn, jf);
+    prolong_value(F, Cc, xc, xf + p, kf, ifn, jf);
 }
 
 // Coarsest level, row r of x = A^{-1} b.

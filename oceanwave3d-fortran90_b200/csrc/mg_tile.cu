@@ -32,7 +32,7 @@ namespace ow3d {
 namespace {
 using namespace mgdev;
 
-constexpr int kCrossThreads = 512, kUniThreads = 320;
+constexpr int kCrossThreads = 512, kUniThreads = 320, kOrderedThreads = 512;
 constexpr size_t kTileSmemMax = 220 * 1024, kTileSmemTwo = 112 * 1024;
 
 // Core and staged region of a block, 1-based columns; on a periodic level i
@@ -367,6 +367,19 @@ struct Rhs {
     const TB* p;
     const double* scale;
 };
+// Sums and products kept apart (the ordered form's transfers).
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return a * b; }
+__device__ __forceinline__ double add_rn(double a, double b) { return a + b; }
+
+// Place of column (c, q) of the region: by column parity (slot), or FLAT: row
+// by row, as the ordered cross form keeps it.
+template <bool FLAT>
+__device__ __forceinline__ int tile_slot(const TileGeo& g, int c, int q) {
+    return FLAT ? (2 * g.HW * q + c) * g.NZP : slot(g, c, q);
+}
+
 template <typename T, typename TB>
 __device__ __forceinline__ T rhs_value(TB v, double s) {
     if constexpr (sizeof(TB) == 8) return T(s * v);
@@ -374,7 +387,7 @@ __device__ __forceinline__ T rhs_value(TB v, double s) {
 }
 
 // Accessor of stage_up (sweep_n).
-template <typename T, typename TB, bool THREE, bool VEC>
+template <typename T, typename TB, bool THREE, bool VEC, bool FLAT>
 struct UpAcc {
     const TB* b;                // at column 1 of the region's first row and the thread's k
     double scale;
@@ -443,11 +456,12 @@ struct UpAcc {
                 };
                 const int kk = k + n;
                 const T w1 = __ldg(F.pwz + 2 * kk + 1);
-                xv[n] += __ldg(F.pwz + 2 * kk) * avg(__ldg(F.piz + 2 * kk) - 1);
-                if (w1 != T(0)) xv[n] += w1 * avg(__ldg(F.piz + 2 * kk + 1) - 1);
+                T d = mul_rn(__ldg(F.pwz + 2 * kk), avg(__ldg(F.piz + 2 * kk) - 1));
+                if (w1 != T(0)) d += w1 * avg(__ldg(F.piz + 2 * kk + 1) - 1);
+                xv[n] = add_rn(xv[n], d);
             }
         }
-        const int s = slot(g, c, q);
+        const int s = tile_slot<FLAT>(g, c, q);
         put<N, VEC>(xs + s, xv);
         put<N, VEC>(bs + s, bv);
     }
@@ -458,7 +472,7 @@ struct UpAcc {
 // point, in sigma by the level's table where the coarse grid is coarsened
 // there too; ghost columns, bottom and free-surface rows take no correction)
 // in xs and the right-hand side in bs.
-template <bool THREE, bool VEC, typename T, typename TB>
+template <bool THREE, bool VEC, bool FLAT, typename T, typename TB>
 __device__ __forceinline__ void stage_up(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileGeo& g, const Reg& r,
                                          const TB* __restrict__ b, const double* __restrict__ bscale,
                                          const T* __restrict__ xin, const T* __restrict__ xc, T* xs, T* bs) {
@@ -466,14 +480,14 @@ __device__ __forceinline__ void stage_up(const LevelDev<T>& F, const LevelDev<T>
     const double scale = bscale ? *bscale : 1.0;
     sweep<2>(r.W, r.H, F.Nzg, [&](int k) {
         const int end = k + ((F.Nzg & 1) == 0 ? 1 : 0);
-        return UpAcc<T, TB, THREE, VEC>{b + o + k, scale, xin + o + k, xc + (Cc.zc ? 0 : k), xs + k, bs + k, F, Cc, g,
+        return UpAcc<T, TB, THREE, VEC, FLAT>{b + o + k, scale, xin + o + k, xc + (Cc.zc ? 0 : k), xs + k, bs + k, F, Cc, g,
                                         r.ra, r.sa, k, k == 0, end == F.Nzg - 1};
     });
 }
 
 // Accessor of stage_down (sweep_n); INPLACE: the right-hand side goes where the
 // iterate will be.
-template <typename T, typename TB, bool THREE, bool VEC, bool INPLACE>
+template <typename T, typename TB, bool THREE, bool VEC, bool INPLACE, bool FLAT>
 struct DownAcc {
     const TB* b;                // at column 1 of the region's first row and the thread's k
     double scale;
@@ -491,7 +505,7 @@ struct DownAcc {
     }
     template <int N>
     __device__ __forceinline__ void st(int c, int q, const Val<N>& v) const {
-        const int s = slot(g, c, q), i = ra + c, j = sa + q;
+        const int s = tile_slot<FLAT>(g, c, q), i = ra + c, j = sa + q;
         T bv[N], x[N];
 #pragma unroll
         for (int n = 0; n < N; ++n) { bv[n] = rhs_value<T>(v.b[n], scale); x[n] = INPLACE ? bv[n] : T(0); }
@@ -510,14 +524,14 @@ struct DownAcc {
 // the right-hand side) with the identity rows (corner columns, level 1 of the
 // ghost columns: b) and, gx[w][2] and gy[w][2] being one over the ghost weight
 // of wall w, the ghost rows relaxed (null: left at zero).
-template <bool THREE, bool VEC, bool INPLACE, typename T, typename TB>
+template <bool THREE, bool VEC, bool INPLACE, bool FLAT, typename T, typename TB>
 __device__ __forceinline__ void stage_down(const LevelDev<T>& F, const TileGeo& g, const Reg& r,
                                            const TB* __restrict__ b, const double* __restrict__ bscale, T* xs, T* bs,
                                            const T (*gx)[3], const T (*gy)[3]) {
     const int64_t o = (int64_t)F.Nzg * F.Nxg * (r.sa - 1);
     const double scale = bscale ? *bscale : 1.0;
     sweep<4>(r.W, r.H, F.Nzg, [&](int k) {
-        return DownAcc<T, TB, THREE, VEC, INPLACE>{b + o + k, scale, xs + k, bs + k, g, gx, gy, r.ra, r.sa, F.Nxg, F.Nyg, F.per,
+        return DownAcc<T, TB, THREE, VEC, INPLACE, FLAT>{b + o + k, scale, xs + k, bs + k, g, gx, gy, r.ra, r.sa, F.Nxg, F.Nyg, F.per,
                                           F.Nzg, k == 0, at_wall(F.Nxg, F.Nyg, F.per, r, THREE)};
     });
 }
@@ -768,7 +782,7 @@ __global__ void __launch_bounds__(kUniThreads, sizeof(T) == 8 ? 2 : 3)
     const int bx = blockIdx.x, by = blockIdx.y;
     const Reg r = region(F.Nxg, F.Nyg, F.per, g, bx, by, THREE);
     const bool wall = at_wall(F.Nxg, F.Nyg, F.per, r, THREE);
-    stage_down<THREE, true, true>(F, g, r, b, scale, xs, xs, u.gx, u.gy);
+    stage_down<THREE, true, true, false>(F, g, r, b, scale, xs, xs, u.gx, u.gy);
     __syncthreads();
     // ghost rows: the contribution of the colour just solved
     auto ghosts = [&](int colour) {
@@ -827,7 +841,7 @@ __device__ __forceinline__ void uni_smooth(const LevelDev<T>& F, const UniTab<T>
 }
 
 template <typename T, typename TB, bool THREE, int NZG>
-__global__ void __launch_bounds__(256, 2) k_mg_up_uni(LevelDev<T> F, LevelDev<T> Cc, const TB* __restrict__ b,
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_mg_up_uni(LevelDev<T> F, LevelDev<T> Cc, const TB* __restrict__ b,
                                                    const double* __restrict__ scale,
                                                    const T* __restrict__ xin, const T* __restrict__ xc,
                                                    T* __restrict__ out, const __grid_constant__ UniTab<T> u, TileGeo g) {
@@ -837,7 +851,7 @@ __global__ void __launch_bounds__(256, 2) k_mg_up_uni(LevelDev<T> F, LevelDev<T>
     T* const bs = xs + 2 * g.HW * g.PH * g.NZP;
     const int bx = blockIdx.x, by = blockIdx.y;
     const Reg r = region(F.Nxg, F.Nyg, F.per, g, bx, by, THREE);
-    stage_up<THREE, true>(F, Cc, g, r, b, scale, xin, xc, xs, bs);
+    stage_up<THREE, true, false>(F, Cc, g, r, b, scale, xin, xc, xs, bs);
     __syncthreads();
     uni_smooth<THREE, NZG>(F, u, g, r, xs, bs);
     write_core<THREE, true>(F, r, g, bx, xs, out);
@@ -1108,7 +1122,7 @@ __global__ void __launch_bounds__(kCrossThreads) k_mg_down_cross(LevelDev<T> F, 
     const int nc = F.ncolor, bx = blockIdx.x, by = blockIdx.y;
     const Reg r = region(F.Nxg, F.Nyg, 0, g, bx, by, THREE);
     stage_cf<THREE>(F, g, r, w.cf);
-    stage_down<THREE, false, false>(F, g, r, b, scale, w.xs, w.bs, (const T(*)[3])nullptr, (const T(*)[3])nullptr);
+    stage_down<THREE, false, false, false>(F, g, r, b, scale, w.xs, w.bs, (const T(*)[3])nullptr, (const T(*)[3])nullptr);
     __syncthreads();
     cross_bottoms<T, THREE, true>(F, t, g, r, w, g.halo);
     cross_smooth<T, THREE, S>(F, t, g, r, w, nc + 2, 2);
@@ -1130,11 +1144,366 @@ __global__ void __launch_bounds__(kCrossThreads) k_mg_up_cross(LevelDev<T> F, Le
     const int nc = F.ncolor, bx = blockIdx.x, by = blockIdx.y;
     const Reg r = region(F.Nxg, F.Nyg, 0, g, bx, by, THREE);
     stage_cf<THREE>(F, g, r, w.cf);
-    stage_up<THREE, false>(F, Cc, g, r, b, scale, xin, xc, w.xs, w.bs);
+    stage_up<THREE, false, false>(F, Cc, g, r, b, scale, xin, xc, w.xs, w.bs);
     __syncthreads();
     cross_bottoms<T, THREE, false>(F, t, g, r, w, nc + 1);
     cross_smooth<T, THREE, S>(F, t, g, r, w, nc, 0);
     write_core<THREE, false>(F, r, g, bx, w.xs, out);
+}
+
+// ------------------------------------------- cross levels in FP32 (ordered)
+//
+// In FP32 another order of the sums moves the steep basins' results by up to
+// 1e-8 (see tile_level in ow3d.cu), so these levels keep every sum of the
+// per-phase kernels (mg_device.cuh) in its order: the bottom rows, residual and
+// restriction are the same functions on the staged tile (the level's
+// description with its vectors' base and pitch replaced by the tile's), the
+// colour tasks the same operations with the difference's weights at hand. The
+// results are the per-phase kernels' bit for bit. TWO: the form of
+// the column task that levels above the fused coarse kernel's size take there
+// (two rows per lane), else one row per lane.
+using LevelF = LevelDev<float>;
+
+// The tile's level: F with vectors xs and bs of the region.
+__device__ __forceinline__ void tile_view(LevelF& L, const LevelF& F, const TileGeo& g, const Reg& r, float* xs,
+                                          float* bs) {
+    if (threadIdx.x == 0) {
+        L = F;
+        L.pitch = 2 * g.HW;
+        const int64_t o = (int64_t)F.Nzg * ((r.ra - 1) + (int64_t)L.pitch * (r.sa - 1));
+        L.xv = xs - o;
+        L.bv = bs - o;
+        L.rv = bs - o;
+    }
+}
+
+// Every point of the columns ilo..ihi x jlo..jhi of the region: f(place in the
+// staged vectors, place in the level's vectors, k, i, j), all 1-based.
+template <typename F_>
+__device__ __forceinline__ void box_points(const LevelF& F, const TileGeo& g, const Reg& r, int ilo, int ihi, int jlo,
+                                           int jhi, F_ f) {
+    const int Nzg = F.Nzg, len = (ihi - ilo + 1) * Nzg;
+    for (int j = jlo + threadIdx.x / 32; j <= jhi; j += blockDim.x / 32) {
+        const int s0 = (2 * g.HW * (j - r.sa) + ilo - r.ra) * Nzg, p0 = Nzg * ((ilo - 1) + F.Nxg * (j - 1));
+#pragma unroll 2
+        for (int e = threadIdx.x % 32; e < len; e += 32) {
+            const int c = (int)div32((uint32_t)e, F.mz32, F.sz32);
+            f(s0 + e, p0 + e, e - c * Nzg + 1, ilo + c, j);
+        }
+    }
+}
+
+// The mixed-derivative sums of a row, in the per-phase kernels' order: over
+// three planes (x: y planes, y: x planes) and three levels the two outer
+// columns of the centred difference. Its centre weight is zero (checked at
+// set-up), so the terms the general form adds for the centre column change
+// nothing. p: the row in the column's staged values; oa, ob: offsets along the
+// difference and across the planes; w: its weights. sh: in row 2 next to a
+// wall, the shift of the level below the bottom's stencil off the ghost column
+// (weights e); the own column's term there goes to lo, times f = 2 s2 or 2 s4
+// (JOIN), or into the sum like the others.
+template <bool PLANES, bool JOIN>
+__device__ __forceinline__ float mixed_sum(const float* w, const float* e, int sh, const float* p, float z0, float z1,
+                                           float z2, int oa, int ob, float f, float& lo) {
+    float xz = 0;
+#pragma unroll
+    for (int b = PLANES ? -1 : 0; b <= (PLANES ? 1 : 0); ++b)
+#pragma unroll
+        for (int kk = 0; kk < 3; ++kk) {
+            const float* const q = p + b * ob + kk - 1;
+            float dx;
+            if (kk == 0 && sh != 0) {
+                dx = 0;
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    const int a = sh - 1 + m;
+                    if (JOIN && a == 0 && b == 0) lo = __fmaf_rn(__fmul_rn(f, z0), e[m], lo);
+                    else dx = __fmaf_rn(e[m], q[a * oa], dx);
+                }
+            } else {
+                dx = __fmaf_rn(w[2], q[oa], __fmul_rn(w[0], q[-oa]));
+            }
+            xz = __fmaf_rn(kk == 0 ? z0 : (kk == 1 ? z1 : z2), dx, xz);
+        }
+    return xz;
+}
+
+// Row k of a column as the map x_k = q - g x_{k-1} (colour_col1 /
+// colour_col2): x0, xp the old values of rows k, k + 1; shx, shy as above.
+template <bool THREE>
+__device__ __forceinline__ void ordered_row(const RowTab<float>& t, const RowConst<float>& rk, const float* p, float bk,
+                                            float x0, float xp, float ih, float ca, float cb, float c3, int ox, int oy,
+                                            int shx, int shy, float& qo, float& go) {
+    const float xl = p[-ox], xr = p[ox];
+    const float xd = THREE ? p[-oy] : 0.0f, xu = THREE ? p[oy] : 0.0f;
+    const float om = rk.om;
+    const float s2 = om * ca, s4 = THREE ? om * cb : 0.0f;
+    const float s3 = om * c3;
+    const float cz = s2 * s2 + s4 * s4 + ih * ih;
+    float off = t.sx2[0] * xl + t.sx2[2] * xr;
+    float diag = t.sx2[1] + s3 * rk.z1 + cz * rk.zz1;
+    if (THREE) { off += t.sy2[0] * xd + t.sy2[2] * xu; diag += t.sy2[1]; }
+    float lo = s3 * rk.z0 + cz * rk.zz0;
+    const float up = s3 * rk.z2 + cz * rk.zz2;
+    if (s2 != 0.0f) {
+        const float f = 2.0f * s2;
+        off = __fmaf_rn(f, mixed_sum<THREE, true>(t.sx1, t.ex[shx < 0], shx, p, rk.z0, rk.z1, rk.z2, ox, oy, f, lo), off);
+    }
+    if (THREE && s4 != 0.0f) {
+        const float f = 2.0f * s4;
+        off = __fmaf_rn(f, mixed_sum<true, true>(t.sy1, t.ey[shy < 0], shy, p, rk.z0, rk.z1, rk.z2, oy, ox, f, lo), off);
+    }
+    const float id = 1.0f / diag;
+    qo = x0 + (bk - diag * x0 - up * xp - off) * id;
+    go = lo * id;
+}
+
+// A x at row k (2..Nzg-1) of an interior column (lo_interior).
+template <bool THREE>
+__device__ __forceinline__ float ordered_interior(const LevelF& L, const RowTab<float>& t, const float* p, int k, int i,
+                                                  int j, int ox, int oy) {
+    float ih, ca, cb, c3;
+    load_cf(L.cf, (int64_t)(i - 1) + (int64_t)L.Nxg * (j - 1), ih, ca, cb, c3);
+    const float om = 1.0f - __ldg(L.zs + k - 1);
+    const float s2 = om * ca, s4 = THREE ? om * cb : 0.0f;
+    const float s3 = om * c3;
+    const float cz = s2 * s2 + s4 * s4 + ih * ih;
+    float acc = 0;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) acc = __fmaf_rn(t.sx2[m], p[(m - 1) * ox], acc);
+    if (THREE) {
+#pragma unroll
+        for (int m = 0; m < 3; ++m) acc = __fmaf_rn(t.sy2[m], p[(m - 1) * oy], acc);
+    }
+    const float z[3] = {t.z0[k - 1], t.z1[k - 1], t.z2[k - 1]}, y[3] = {t.y0[k - 1], t.y1[k - 1], t.y2[k - 1]};
+    float dz = 0, dzz = 0;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        const float v = p[m - 1];
+        dz = __fmaf_rn(z[m], v, dz);
+        dzz = __fmaf_rn(y[m], v, dzz);
+    }
+    acc += s3 * dz + cz * dzz;
+    const int shx = k != 2 ? 0 : (i == 2 ? 1 : (i == L.Nxg - 1 ? -1 : 0));
+    const int shy = !THREE || k != 2 ? 0 : (j == 2 ? 1 : (j == L.Nyg - 1 ? -1 : 0));
+    float none;
+    if (s2 != 0.0f)
+        acc = __fmaf_rn(2.0f * s2, mixed_sum<THREE, false>(t.sx1, t.ex[shx < 0], shx, p, z[0], z[1], z[2], ox, oy, 0.0f,
+                                                           none), acc);
+    if (THREE && s4 != 0.0f)
+        acc = __fmaf_rn(2.0f * s4, mixed_sum<true, false>(t.sy1, t.ey[shy < 0], shy, p, z[0], z[1], z[2], oy, ox, 0.0f,
+                                                          none), acc);
+    return acc;
+}
+
+// The colour task of column (i, j) (act), S lanes each: colour_col2 (TWO) or
+// colour_col1 on the staged tile.
+template <bool THREE, int S, bool TWO>
+__device__ __forceinline__ void ordered_task(const LevelF& L, const RowTab<float>& t, int i, int j, bool act,
+                                             const RowConst<float>& ra, const RowConst<float>& rb) {
+    const int Nxg = L.Nxg, Nyg = L.Nyg, Nzg = L.Nzg, R = Nzg - 2, lane = threadIdx.x & 31, r = lane & (S - 1);
+    const int ox = Nzg, oy = Nzg * L.pitch;
+    float* const X = L.xv;
+    const float* const B = L.bv;
+    float* const xc = X + IC(L, i, j) * Nzg;
+    const float* const bc = B + IC(L, i, j) * Nzg;
+    const int ka = TWO ? 2 + 2 * r : min(r + 2, Nzg - 1), kb = ka + 1;
+    const bool va = act && (TWO ? ka <= Nzg - 1 : r < R), vb = TWO && act && kb <= Nzg - 1;
+    const int last = TWO ? (R - 1) / 2 : R - 1;
+    const bool edge = act && (i <= 3 || i >= Nxg - 2 || (THREE && (j <= 3 || j >= Nyg - 2)));
+    // ghost column at offset og from the column, the two columns of its stencil
+    // at oa (weight wa) and ob (wb); own: which of them is this column (its new
+    // values are xna, xnb, xfs once post is set)
+    auto relax = [&](int og, int oa, float wa, int ob, float wb, float wg, int own, bool post, float xna, float xnb,
+                     float xfsn) {
+        auto row = [&](int kk, float xo) {
+            const float v1 = (post && own == 1) ? xo : xc[oa + kk - 1];
+            const float v2 = (post && own == 2) ? xo : xc[ob + kk - 1];
+            xc[og + kk - 1] = (bc[og + kk - 1] - (wa * v1 + wb * v2)) / wg;
+        };
+        if (TWO) {
+            if (ka <= Nzg - 1) row(ka, xna);
+            if (kb <= Nzg - 1) row(kb, xnb);
+        } else if (r < R) {
+            row(r + 2, xna);
+        }
+        if (r == last) row(Nzg, xfsn);
+    };
+    auto ghosts = [&](bool post, float xna, float xnb, float xfsn) {
+        // low walls: stencil of position 2, columns 1 (ghost), 2, 3; high walls
+        // of position n - 1, columns n - 2, n - 1, n (ghost)
+        if (i == 2 || (post && i == 3))
+            relax((1 - i) * ox, (2 - i) * ox, t.sx1[1], (3 - i) * ox, t.sx1[2], t.sx1[0], i == 2 ? 1 : 2, post, xna, xnb,
+                  xfsn);
+        if (i == Nxg - 1 || (post && i == Nxg - 2))
+            relax((Nxg - i) * ox, (Nxg - 2 - i) * ox, t.sx1[0], (Nxg - 1 - i) * ox, t.sx1[1], t.sx1[2],
+                  i == Nxg - 1 ? 2 : 1, post, xna, xnb, xfsn);
+        if (THREE) {
+            if (j == 2 || (post && j == 3))
+                relax((1 - j) * oy, (2 - j) * oy, t.sy1[1], (3 - j) * oy, t.sy1[2], t.sy1[0], j == 2 ? 1 : 2, post, xna,
+                      xnb, xfsn);
+            if (j == Nyg - 1 || (post && j == Nyg - 2))
+                relax((Nyg - j) * oy, (Nyg - 2 - j) * oy, t.sy1[0], (Nyg - 1 - j) * oy, t.sy1[1], t.sy1[2],
+                      j == Nyg - 1 ? 2 : 1, post, xna, xnb, xfsn);
+        }
+    };
+    if (edge) {
+        // (corner columns hold b from the staging)
+        ghosts(false, 0.0f, 0.0f, 0.0f);
+    }
+    __syncwarp();
+    float qa = 0, ga = 0, qb = 0, gb = 0, x1 = 0;
+    if (act) {
+        float ih, ca, cb, c3;
+        load_cf(L.cf, (int64_t)(i - 1) + (int64_t)Nxg * (j - 1), ih, ca, cb, c3);
+        const int kra = min(ka, Nzg - 1), krb = min(kb, Nzg - 1);
+        const int shx = kra != 2 ? 0 : (i == 2 ? 1 : (i == Nxg - 1 ? -1 : 0));
+        const int shy = !THREE || kra != 2 ? 0 : (j == 2 ? 1 : (j == Nyg - 1 ? -1 : 0));
+        const float x0a = xc[kra - 1], xpa = xc[kra], xpb = xc[krb];
+        ordered_row<THREE>(t, ra, xc + kra - 1, bc[kra - 1], x0a, xpa, ih, ca, cb, c3, ox, oy, shx, shy, qa, ga);
+        if (TWO)
+            ordered_row<THREE>(t, rb, xc + krb - 1, bc[krb - 1], xpa, xpb, ih, ca, cb, c3, ox, oy, 0, 0, qb, gb);
+        if (!va) { qa = 0; ga = 0; }
+        if (!vb) { qb = 0; gb = 0; }
+        x1 = xc[0];
+    }
+    float xna, xnb = 0;
+    if constexpr (TWO) {
+        float a = 1, bb = 0;
+        if (va) { bb = qa; a = -ga; }
+        if (vb) { bb = qb - gb * bb; a = -gb * a; }
+#pragma unroll
+        for (int d = 1; d < S; d <<= 1) {
+            const float ap = __shfl_up_sync(0xffffffffu, a, d, S);
+            const float bp = __shfl_up_sync(0xffffffffu, bb, d, S);
+            if (r >= d) { bb = a * bp + bb; a = a * ap; }
+        }
+        const float ae = __shfl_up_sync(0xffffffffu, a, 1, S), be = __shfl_up_sync(0xffffffffu, bb, 1, S);
+        const float xin = (r == 0) ? x1 : ae * x1 + be;
+        xna = qa - ga * xin;
+        xnb = qb - gb * xna;
+    } else {
+        float a = -ga, bb = qa;
+#pragma unroll
+        for (int d = 1; d < S; d <<= 1) {
+            const float ap = __shfl_up_sync(0xffffffffu, a, d, S);
+            const float bp = __shfl_up_sync(0xffffffffu, bb, d, S);
+            if (r >= d) { bb = a * bp + bb; a = a * ap; }
+        }
+        xna = a * x1 + bb;
+    }
+    const float xfs = act ? bc[Nzg - 1] : 0.0f;
+    __syncwarp();
+    if (va) xc[ka - 1] = xna;
+    if (vb) xc[kb - 1] = xnb;
+    if (act && r == last) xc[Nzg - 1] = xfs;
+    if (edge) ghosts(true, xna, xnb, xfs);
+}
+
+template <bool THREE>
+__device__ __forceinline__ void ordered_bottoms(const LevelF& L, const Reg& r, int d) {
+    all_columns<THREE>(L.Nxg, L.Nyg, 0, r, d, [&](int i, int j) { bottom_column<float, THREE>(L, i, j); });
+    __syncthreads();
+}
+
+// The colour tasks at distance <= d, one column per segment of S lanes.
+template <bool THREE, int S, bool TWO>
+__device__ __forceinline__ void ordered_colour(const LevelF& L, const RowTab<float>& t, const Reg& r, int colour, int d) {
+    const int Nxg = L.Nxg, Nyg = L.Nyg, Nzg = L.Nzg;
+    const int ilo = max(r.ia - d, 2), ihi = min(r.ib + d, Nxg - 1);
+    int jlo = 1, jhi = 1, js = 1;
+    if (THREE) { jlo = max(r.ja - d, 2); jhi = min(r.jb + d, Nyg - 1); }
+    const bool four = L.ncolor == 4;
+    if (THREE && four) { jlo += (jlo ^ (colour >> 1)) & 1; js = 2; }
+    const int ni = max((ihi - ilo + 2) >> 1, 0), nj = jhi >= jlo ? (jhi - jlo) / js + 1 : 0, total = ni * nj;
+    const int lane = threadIdx.x & 31, rr = lane & (S - 1);
+    const int per_warp = 32 / S, step = (blockDim.x >> 5) * per_warp;
+    const RowConst<float> ra = TWO ? row_const_k<float>(L, 2 + 2 * rr) : row_const<float, S>(L);
+    const RowConst<float> rb = TWO ? row_const_k<float>(L, 3 + 2 * rr) : ra;
+    const float rni = recip(ni);
+    for (int base = (threadIdx.x >> 5) * per_warp; base < total; base += step) {
+        const int q = base + lane / S;
+        int i = 2, j = THREE ? 2 : 1;
+        bool act = q < total;
+        if (act) {
+            const int tj = quot(q, rni);
+            j = jlo + tj * js;
+            const int par = four ? colour & 1 : (colour + j) & 1;
+            i = ilo + ((ilo ^ par) & 1) + 2 * (q - tj * ni);
+            act = i <= ihi;
+        }
+        ordered_task<THREE, S, TWO>(L, t, i, j, act, ra, rb);
+    }
+    __syncthreads();
+}
+
+template <bool THREE, int S, bool TWO>
+__global__ void __launch_bounds__(kOrderedThreads) k_mg_down_ordered(LevelF F, LevelF Cc, const float* __restrict__ b,
+                                                                     float* __restrict__ xout, float* __restrict__ rc,
+                                                                     const __grid_constant__ RowTab<float> t,
+                                                                     TileGeo g) {
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    __shared__ LevelF L;
+    float* const xs = reinterpret_cast<float*>(tile_smem);
+    float* const bs = xs + 2 * g.HW * g.PH * F.Nzg;
+    const int Nxg = F.Nxg, Nyg = F.Nyg, nc = F.ncolor;
+    const Reg r = region(Nxg, Nyg, 0, g, blockIdx.x, blockIdx.y, THREE);
+    tile_view(L, F, g, r, xs, bs);
+    // x = 0; the bottom pass over it sets the ghost columns' level 1 (the
+    // corner columns, which only the column diagonal to them reads, after it
+    // has set them, may hold b already)
+    stage_down<THREE, true, false, true>(F, g, r, b, (const double*)nullptr, xs, bs, (const float(*)[3])nullptr,
+                                         (const float(*)[3])nullptr);
+    __syncthreads();
+    ordered_bottoms<THREE>(L, r, nc + 3);
+    for (int c = 0; c < nc; ++c) ordered_colour<THREE, S, TWO>(L, t, r, c, nc + 2 - c);
+    ordered_bottoms<THREE>(L, r, 2);
+    // the iterate of the core, and at distance <= 1 the residual where the
+    // right-hand side was
+    box_points(F, g, r, max(r.ia - 1, 1), min(r.ib + 1, Nxg), THREE ? max(r.ja - 1, 1) : 1,
+               THREE ? min(r.jb + 1, Nyg) : 1, [&](int s, int p, int k, int i, int j) {
+        if (i >= r.ia && i <= r.ib && j >= r.ja && j <= r.jb) xout[p] = xs[s];
+        float v, dg;
+        if (i == 1 || i == Nxg || (THREE && (j == 1 || j == Nyg))) v = lo_ghost<float, THREE>(L, L.xv, k, i, j, dg);
+        else if (k == F.Nzg) v = xs[s];
+        else if (k == 1) v = lo_bottom<float, THREE>(L, L.xv, i, j, dg);
+        else v = ordered_interior<THREE>(F, t, xs + s, k, i, j, F.Nzg, F.Nzg * 2 * g.HW);
+        bs[s] = bs[s] - v;
+    });
+    __syncthreads();
+    int clo, chi, dlo = 1, dhi = 1;
+    owned(r.ia, r.ib, Nxg, Cc.Nxg, 1 + Cc.xc, 0, clo, chi);
+    if (THREE) owned(r.ja, r.jb, Nyg, Cc.Nyg, 1 + Cc.yc, 0, dlo, dhi);
+    const int Ncz = Cc.Nzg, len = (chi - clo + 1) * Ncz;
+    const float rlen = recip(len);
+    for (int e = threadIdx.x; e < len * (dhi - dlo + 1); e += blockDim.x) {
+        const int q = quot(e, rlen);
+        restrict_item<float>(L, Cc, L.rv, rc, Cc.xv,
+                              (e - q * len) + Ncz * ((clo - 1) + (int64_t)Cc.Nxg * (dlo + q - 1)));
+    }
+}
+
+template <bool THREE, int S, bool TWO>
+__global__ void __launch_bounds__(kOrderedThreads) k_mg_up_ordered(LevelF F, LevelF Cc, const float* __restrict__ b,
+                                                                   const float* __restrict__ xin,
+                                                                   const float* __restrict__ xc,
+                                                                   float* __restrict__ out,
+                                                                   const __grid_constant__ RowTab<float> t, TileGeo g) {
+    pdl_entry();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    __shared__ LevelF L;
+    float* const xs = reinterpret_cast<float*>(tile_smem);
+    float* const bs = xs + 2 * g.HW * g.PH * F.Nzg;
+    const int nc = F.ncolor;
+    const Reg r = region(F.Nxg, F.Nyg, 0, g, blockIdx.x, blockIdx.y, THREE);
+    tile_view(L, F, g, r, xs, bs);
+    stage_up<THREE, true, true>(F, Cc, g, r, b, (const double*)nullptr, xin, xc, xs, bs);
+    __syncthreads();
+    ordered_bottoms<THREE>(L, r, nc + 1);
+    for (int c = 0; c < nc; ++c) ordered_colour<THREE, S, TWO>(L, t, r, c, nc - c);
+    ordered_bottoms<THREE>(L, r, 0);
+    box_points(F, g, r, r.ia, r.ib, r.ja, r.jb, [&](int s, int p, int, int, int) { out[p] = xs[s]; });
 }
 
 // ------------------------------------------------------------ host side
@@ -1143,6 +1512,11 @@ __global__ void __launch_bounds__(kCrossThreads) k_mg_up_cross(LevelDev<T> F, Le
 // column one by one: odd. Uniform levels, two rows at a time: twice an odd
 // number.
 inline int tile_pitch(int nzg, bool cross) { return cross ? nzg | 1 : ((nzg + 1) / 2 | 1) * 2; }
+
+// Whether the per-phase kernels take the level's columns with two rows per lane
+// (the levels above the fused coarse kernel's size).
+template <typename T>
+bool two_rows(const LevelDev<T>& L) { return L.N > g_coop_max_points.load(std::memory_order_relaxed); }
 
 // Cores, slots and shared memory of a launch over all its tiles.
 template <typename T>
@@ -1158,7 +1532,8 @@ void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross, bool
     cores(L.per ? L.Nxg - 3 : L.Nxg, cx, g.ntx, g.qx, g.remx, g.cx);
     if (three) cores(L.Nyg, cy, g.nty, g.qy, g.remy, g.cy);
     else { g.nty = 1; g.qy = 1; g.remy = 0; g.cy = 1; }
-    g.NZP = tile_pitch(L.Nzg, cross);
+    const bool ordered = cross && sizeof(T) == 4;
+    g.NZP = ordered ? L.Nzg : tile_pitch(L.Nzg, cross);
     g.np = (L.Nzg + 1) / 2;
     int W = 0, H = 0;
     for (int bx = 0; bx < g.ntx; ++bx) W = std::max(W, region(L.Nxg, L.Nyg, L.per, g, bx, 0, three).W);
@@ -1167,7 +1542,7 @@ void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross, bool
     g.PH = H;
     const size_t cols = (size_t)2 * g.HW * g.PH;
     // iterate, right-hand side (uniform levels on the way down: in one place), coefficients
-    g.smem = (cols * g.NZP * (cross || !down ? 2 : 1) + (cross ? 4 * cols : 0)) * sizeof(T);
+    g.smem = (cols * g.NZP * (cross || !down ? 2 : 1) + (cross && !ordered ? 4 * cols : 0)) * sizeof(T);
 }
 
 }  // namespace
@@ -1177,10 +1552,10 @@ void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
     const bool three = L.Nyg > 1, cross = t.mode == kTileCross;
     // The largest core that leaves room for two blocks per SM, on levels with
     // at least a tile per SM of that size; smaller levels take smaller cores.
-    static const int uni3[][2] = {{32, 8}, {16, 8}, {8, 4}}, cross3[][2] = {{16, 16}, {16, 8}, {8, 8}, {4, 4}};
+    static const int uni3[][2] = {{32, 8}, {16, 8}, {8, 4}}, cross3[][2] = {{16, 16}, {16, 8}, {8, 8}};
     static const int line[][2] = {{64, 1}, {32, 1}, {16, 1}};
     const int (*cand)[2] = three ? (cross ? cross3 : uni3) : line;
-    const int ncand = three && cross ? 4 : 3;
+    const int ncand = 3;
     auto pick = [&](TileGeo& g, int halo, bool down) {
         g.halo = halo;
         bool found = false;
@@ -1188,9 +1563,11 @@ void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
         for (int q = 0; q < ncand; ++q) {
             size_geo(L, g, cand[q][0], cand[q][1], cross, down);
             if (g.smem > kTileSmemMax || (g.smem > kTileSmemTwo && q + 1 < ncand)) continue;
-            const int lanes = cross ? (L.Nzg <= 10 ? 4 : (L.Nzg <= 18 ? 8 : 16)) : 1;
+            int lanes = cross ? (L.Nzg <= 10 ? 4 : (L.Nzg <= 18 ? 8 : 16)) : 1;
+            if (cross && sizeof(T) == 4 && !two_rows(L)) lanes *= 2;
             const int cols = (g.cx + 2 * halo) * (three ? g.cy + 2 * halo : 1) / L.ncolor * lanes;
-            g.threads = std::max(256, std::min(cross ? kCrossThreads : (down ? kUniThreads : 256), (cols + 31) / 32 * 32));
+            const int most = cross ? kCrossThreads : (down ? kUniThreads : 256);
+            g.threads = std::min(most, std::max(256, (cols + 31) / 32 * 32));
             found = true;
             best = g;
             if (g.ntx * g.nty >= 148) break;
@@ -1199,8 +1576,9 @@ void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
         return found;
     };
     if (t.mode == kTileNone) return;
-    const int nc = L.ncolor;
-    if (!pick(t.down, cross ? nc + 3 : 3, true) || !pick(t.up, cross ? nc + 2 : 2, false)) t.mode = kTileNone;
+    // (the ordered form's first bottom pass reads one column further)
+    const int nc = L.ncolor, extra = sizeof(T) == 4 ? 1 : 0;
+    if (!pick(t.down, cross ? nc + 3 + extra : 3, true) || !pick(t.up, cross ? nc + 2 : 2, false)) t.mode = kTileNone;
 }
 
 namespace {
@@ -1252,30 +1630,68 @@ void up_cross(const LevelDev<T>& F, const LevelDev<T>& Cc, const TileLevel<T>& t
              Cc, b.p, b.scale, xs, xc, out, t.r, g);
 }
 
+template <bool THREE, int S, bool TWO>
+void down_ordered(const LevelF& F, const LevelF& Cc, const TileLevel<float>& t, Rhs<float> b, float* xs, float* rc, float*,
+                  cudaStream_t st) {
+    static std::atomic<unsigned long long> set{0ull};
+    const TileGeo& g = t.down;
+    allow_smem(k_mg_down_ordered<THREE, S, TWO>, set);
+    launch_k(k_mg_down_ordered<THREE, S, TWO>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem,
+             st, F, Cc, b.p, xs, rc, t.r, g);
+}
+template <bool THREE, int S, bool TWO>
+void up_ordered(const LevelF& F, const LevelF& Cc, const TileLevel<float>& t, Rhs<float> b, const float* xs,
+                const float* xc, float* out, cudaStream_t st) {
+    static std::atomic<unsigned long long> set{0ull};
+    const TileGeo& g = t.up;
+    allow_smem(k_mg_up_ordered<THREE, S, TWO>, set);
+    launch_k(k_mg_up_ordered<THREE, S, TWO>, dim3((unsigned)g.ntx, (unsigned)g.nty), dim3((unsigned)g.threads), g.smem, st,
+             F, Cc, b.p, xs, xc, out, t.r, g);
+}
+
 // Uniform levels: the level counts of the decks' usual Nz unrolled. Cross
-// levels (FP64): the lanes per column, two rows each.
-#define OW3D_TILE(way, ...)                                                    \
-    do {                                                                       \
-        if (t.mode == kTileUniform) {                                          \
-            if (F.Nyg > 1) {                                                   \
-                if (F.Nzg == 18) way##_uni<T, TB, true, 18>(__VA_ARGS__);      \
-                else if (F.Nzg == 10) way##_uni<T, TB, true, 10>(__VA_ARGS__); \
-                else way##_uni<T, TB, true, 0>(__VA_ARGS__);                   \
-            } else {                                                           \
-                if (F.Nzg == 10) way##_uni<T, TB, false, 10>(__VA_ARGS__);     \
-                else way##_uni<T, TB, false, 0>(__VA_ARGS__);                  \
-            }                                                                  \
-        } else if constexpr (sizeof(T) == 8) {                                 \
-            if (F.Nyg > 1) {                                                   \
-                if (F.Nzg <= 10) way##_cross<T, TB, true, 4>(__VA_ARGS__);     \
+// levels: the lanes per column (FP64, and FP32 with two rows per lane: two
+// rows each; else one).
+#define OW3D_TILE(way, ...)                                                     \
+    do {                                                                        \
+        if (t.mode == kTileUniform) {                                           \
+            if (F.Nyg > 1) {                                                    \
+                if (F.Nzg == 18) way##_uni<T, TB, true, 18>(__VA_ARGS__);       \
+                else if (F.Nzg == 10) way##_uni<T, TB, true, 10>(__VA_ARGS__);  \
+                else way##_uni<T, TB, true, 0>(__VA_ARGS__);                    \
+            } else {                                                            \
+                if (F.Nzg == 10) way##_uni<T, TB, false, 10>(__VA_ARGS__);      \
+                else way##_uni<T, TB, false, 0>(__VA_ARGS__);                   \
+            }                                                                   \
+        } else if constexpr (sizeof(T) == 8) {                                  \
+            if (F.Nyg > 1) {                                                    \
+                if (F.Nzg <= 10) way##_cross<T, TB, true, 4>(__VA_ARGS__);      \
                 else if (F.Nzg <= 18) way##_cross<T, TB, true, 8>(__VA_ARGS__); \
-                else way##_cross<T, TB, true, 16>(__VA_ARGS__);                \
-            } else {                                                           \
-                if (F.Nzg <= 10) way##_cross<T, TB, false, 4>(__VA_ARGS__);    \
+                else way##_cross<T, TB, true, 16>(__VA_ARGS__);                 \
+            } else {                                                            \
+                if (F.Nzg <= 10) way##_cross<T, TB, false, 4>(__VA_ARGS__);     \
                 else if (F.Nzg <= 18) way##_cross<T, TB, false, 8>(__VA_ARGS__); \
-                else way##_cross<T, TB, false, 16>(__VA_ARGS__);               \
-            }                                                                  \
-        }                                                                      \
+                else way##_cross<T, TB, false, 16>(__VA_ARGS__);                \
+            }                                                                   \
+        } else if constexpr (sizeof(TB) == 4) {                                 \
+            if (F.Nyg > 1 && two_rows(F)) {                                     \
+                if (F.Nzg <= 10) way##_ordered<true, 4, true>(__VA_ARGS__);     \
+                else if (F.Nzg <= 18) way##_ordered<true, 8, true>(__VA_ARGS__); \
+                else way##_ordered<true, 16, true>(__VA_ARGS__);                \
+            } else if (F.Nyg > 1) {                                             \
+                if (F.Nzg <= 10) way##_ordered<true, 8, false>(__VA_ARGS__);    \
+                else if (F.Nzg <= 18) way##_ordered<true, 16, false>(__VA_ARGS__); \
+                else way##_ordered<true, 32, false>(__VA_ARGS__);               \
+            } else if (two_rows(F)) {                                           \
+                if (F.Nzg <= 10) way##_ordered<false, 4, true>(__VA_ARGS__);    \
+                else if (F.Nzg <= 18) way##_ordered<false, 8, true>(__VA_ARGS__); \
+                else way##_ordered<false, 16, true>(__VA_ARGS__);               \
+            } else {                                                            \
+                if (F.Nzg <= 10) way##_ordered<false, 8, false>(__VA_ARGS__);   \
+                else if (F.Nzg <= 18) way##_ordered<false, 16, false>(__VA_ARGS__); \
+                else way##_ordered<false, 32, false>(__VA_ARGS__);              \
+            }                                                                   \
+        }                                                                       \
     } while (0)
 
 template <typename T, typename TB>

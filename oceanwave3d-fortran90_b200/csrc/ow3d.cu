@@ -175,11 +175,12 @@ int upload(ow3d_handle* H, T** p, const std::vector<double>& v) {
 // interior columns, checked value by value). Uniform: no mixed-derivative
 // terms and the same coefficients in every interior column (flat bottom) -- a
 // varying depth given without its slopes keeps the per-phase kernels. Cross:
-// mixed-derivative terms, walls, FP64 only: in FP32 another order of the sums
-// moves the steep basins' results by up to 1e-8 (65x33x9 shoal, which stops at
-// the matvec limit: 2e-9; two-dimensional 65x17 and 257x17 flumes: 1e-9), in
-// FP64 by 1e-12. Flat levels move by 1e-11 at most in FP32. Periodic levels
-// with an odd period (the two colours would meet at its ends) have none.
+// mixed-derivative terms, walls. In FP32 another order of the sums moves the
+// steep basins' results by up to 1e-8 (65x33x9 shoal, which stops at the matvec
+// limit: 2e-9; two-dimensional 65x17 and 257x17 flumes: 1e-9), in FP64 by
+// 1e-12, so the FP32 cross kernels keep the per-phase kernels' order; flat
+// levels move by 1e-11 at most in FP32. Periodic levels with an odd period
+// (the two colours would meet at its ends) have none.
 template <typename T>
 TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vector<double>& cf,
                         const std::vector<double>& bt) {
@@ -204,7 +205,9 @@ TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vec
         gy[1][0] = sy(1, ny - 1, 1); gy[1][1] = sy(1, ny - 1, 0); gy[1][2] = 1.0 / sy(1, ny - 1, 2);
     }
     if (d.cross) {
-        if (d.per || d.ncolor != (three ? 4 : 2) || sizeof(T) != 8) return t;
+        if (d.per || d.ncolor != (three ? 4 : 2)) return t;
+        // (the ordered FP32 kernels leave out the centre of the first difference)
+        if (sizeof(T) == 4 && (sx(1, 2, 1) != 0.0 || (three && sy(1, 2, 1) != 0.0))) return t;
         t.mode = kTileCross;
         RowTab<T>& r = t.r;
         for (int k = 1; k <= h.Nzg; ++k) {
@@ -261,6 +264,7 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
         const LevelHost& h = H->G.levels[l];
         LevelDev<T>& d = S.lev[l];
         d.Nx = h.Nx; d.Ny = h.Ny; d.Nz = h.Nz; d.Nxg = h.Nxg; d.Nyg = h.Nyg; d.Nzg = h.Nzg;
+        d.pitch = h.Nxg;
         d.N = (int64_t)h.Nxg * h.Nyg * h.Nzg;
         d.ncolor = h.ncolor; d.xc = h.xc; d.yc = h.yc; d.zc = h.zc;
         d.per = H->G.per;

@@ -119,6 +119,7 @@ template <typename T>
 struct LevelDev {
     int Nx, Ny, Nz;         // interior counts
     int Nxg, Nyg, Nzg;
+    int pitch;              // columns per row of xv, bv and rv: Nxg, or a staged tile's width
     int64_t N;
     int ncolor;             // 2 or 4 (multicolour column Gauss-Seidel)
     int cross;              // mixed-derivative terms present (h_x or h_y nonzero on the level)
