@@ -1194,36 +1194,47 @@ __device__ __forceinline__ void box_points(const LevelF& F, const TileGeo& g, co
 }
 
 // The mixed-derivative sums of a row, in the per-phase kernels' order: over
-// three planes (x: y planes, y: x planes) and three levels the two outer
-// columns of the centred difference. Its centre weight is zero (checked at
-// set-up), so the terms the general form adds for the centre column change
-// nothing. p: the row in the column's staged values; oa, ob: offsets along the
-// difference and across the planes; w: its weights. sh: in row 2 next to a
-// wall, the shift of the level below the bottom's stencil off the ghost column
-// (weights e); the own column's term there goes to lo, times f = 2 s2 or 2 s4
-// (JOIN), or into the sum like the others.
+// three planes (x: y planes, y: x planes) and three levels the three columns of
+// the centred difference (w; its centre weight is zero up to rounding, and
+// where it is exactly zero, cw false, its terms change nothing and are left
+// out). p: the row in the column's staged values; oa, ob: offsets along the
+// difference and across the planes. sh: in row 2 next to a wall, the shift of
+// the level below the bottom's stencil off the ghost column (weights e). JOIN:
+// the own column's terms go to lo, dg, up, times f = 2 s2 or 2 s4 (top: row
+// Nzg-1, whose upper one does not), else into the sum like the others.
 template <bool PLANES, bool JOIN>
-__device__ __forceinline__ float mixed_sum(const float* w, const float* e, int sh, const float* p, float z0, float z1,
-                                           float z2, int oa, int ob, float f, float& lo) {
+__device__ __forceinline__ float mixed_sum(const float* w, const float* e, int sh, bool cw, bool top, const float* p,
+                                           float z0, float z1, float z2, int oa, int ob, float f, float& lo, float& dg,
+                                           float& up) {
     float xz = 0;
 #pragma unroll
     for (int b = PLANES ? -1 : 0; b <= (PLANES ? 1 : 0); ++b)
 #pragma unroll
         for (int kk = 0; kk < 3; ++kk) {
             const float* const q = p + b * ob + kk - 1;
+            const float z = kk == 0 ? z0 : (kk == 1 ? z1 : z2);
             float dx;
             if (kk == 0 && sh != 0) {
                 dx = 0;
 #pragma unroll
                 for (int m = 0; m < 3; ++m) {
                     const int a = sh - 1 + m;
-                    if (JOIN && a == 0 && b == 0) lo = __fmaf_rn(__fmul_rn(f, z0), e[m], lo);
+                    if (JOIN && a == 0 && b == 0) lo = __fmaf_rn(__fmul_rn(f, z), e[m], lo);
                     else dx = __fmaf_rn(e[m], q[a * oa], dx);
                 }
             } else {
-                dx = __fmaf_rn(w[2], q[oa], __fmul_rn(w[0], q[-oa]));
+                dx = __fmul_rn(w[0], q[-oa]);
+                if (cw) {
+                    if (JOIN && b == 0 && !(kk == 2 && top)) {
+                        float& c = kk == 0 ? lo : (kk == 1 ? dg : up);
+                        c = __fmaf_rn(__fmul_rn(f, z), w[1], c);
+                    } else {
+                        dx = __fmaf_rn(w[1], q[0], dx);
+                    }
+                }
+                dx = __fmaf_rn(w[2], q[oa], dx);
             }
-            xz = __fmaf_rn(kk == 0 ? z0 : (kk == 1 ? z1 : z2), dx, xz);
+            xz = __fmaf_rn(z, dx, xz);
         }
     return xz;
 }
@@ -1233,7 +1244,7 @@ __device__ __forceinline__ float mixed_sum(const float* w, const float* e, int s
 template <bool THREE>
 __device__ __forceinline__ void ordered_row(const RowTab<float>& t, const RowConst<float>& rk, const float* p, float bk,
                                             float x0, float xp, float ih, float ca, float cb, float c3, int ox, int oy,
-                                            int shx, int shy, float& qo, float& go) {
+                                            int shx, int shy, bool top, float& qo, float& go) {
     const float xl = p[-ox], xr = p[ox];
     const float xd = THREE ? p[-oy] : 0.0f, xu = THREE ? p[oy] : 0.0f;
     const float om = rk.om;
@@ -1244,14 +1255,16 @@ __device__ __forceinline__ void ordered_row(const RowTab<float>& t, const RowCon
     float diag = t.sx2[1] + s3 * rk.z1 + cz * rk.zz1;
     if (THREE) { off += t.sy2[0] * xd + t.sy2[2] * xu; diag += t.sy2[1]; }
     float lo = s3 * rk.z0 + cz * rk.zz0;
-    const float up = s3 * rk.z2 + cz * rk.zz2;
+    float up = s3 * rk.z2 + cz * rk.zz2;
     if (s2 != 0.0f) {
         const float f = 2.0f * s2;
-        off = __fmaf_rn(f, mixed_sum<THREE, true>(t.sx1, t.ex[shx < 0], shx, p, rk.z0, rk.z1, rk.z2, ox, oy, f, lo), off);
+        off = __fmaf_rn(f, mixed_sum<THREE, true>(t.sx1, t.ex[shx < 0], shx, t.sx1[1] != 0.0f, top, p, rk.z0, rk.z1,
+                                                  rk.z2, ox, oy, f, lo, diag, up), off);
     }
     if (THREE && s4 != 0.0f) {
         const float f = 2.0f * s4;
-        off = __fmaf_rn(f, mixed_sum<true, true>(t.sy1, t.ey[shy < 0], shy, p, rk.z0, rk.z1, rk.z2, oy, ox, f, lo), off);
+        off = __fmaf_rn(f, mixed_sum<true, true>(t.sy1, t.ey[shy < 0], shy, t.sy1[1] != 0.0f, top, p, rk.z0, rk.z1, rk.z2,
+                                                 oy, ox, f, lo, diag, up), off);
     }
     const float id = 1.0f / diag;
     qo = x0 + (bk - diag * x0 - up * xp - off) * id;
@@ -1288,11 +1301,11 @@ __device__ __forceinline__ float ordered_interior(const LevelF& L, const RowTab<
     const int shy = !THREE || k != 2 ? 0 : (j == 2 ? 1 : (j == L.Nyg - 1 ? -1 : 0));
     float none;
     if (s2 != 0.0f)
-        acc = __fmaf_rn(2.0f * s2, mixed_sum<THREE, false>(t.sx1, t.ex[shx < 0], shx, p, z[0], z[1], z[2], ox, oy, 0.0f,
-                                                           none), acc);
+        acc = __fmaf_rn(2.0f * s2, mixed_sum<THREE, false>(t.sx1, t.ex[shx < 0], shx, t.sx1[1] != 0.0f, false, p, z[0],
+                                                           z[1], z[2], ox, oy, 0.0f, none, none, none), acc);
     if (THREE && s4 != 0.0f)
-        acc = __fmaf_rn(2.0f * s4, mixed_sum<true, false>(t.sy1, t.ey[shy < 0], shy, p, z[0], z[1], z[2], oy, ox, 0.0f,
-                                                          none), acc);
+        acc = __fmaf_rn(2.0f * s4, mixed_sum<true, false>(t.sy1, t.ey[shy < 0], shy, t.sy1[1] != 0.0f, false, p, z[0],
+                                                          z[1], z[2], oy, ox, 0.0f, none, none, none), acc);
     return acc;
 }
 
@@ -1360,9 +1373,11 @@ __device__ __forceinline__ void ordered_task(const LevelF& L, const RowTab<float
         const int shx = kra != 2 ? 0 : (i == 2 ? 1 : (i == Nxg - 1 ? -1 : 0));
         const int shy = !THREE || kra != 2 ? 0 : (j == 2 ? 1 : (j == Nyg - 1 ? -1 : 0));
         const float x0a = xc[kra - 1], xpa = xc[kra], xpb = xc[krb];
-        ordered_row<THREE>(t, ra, xc + kra - 1, bc[kra - 1], x0a, xpa, ih, ca, cb, c3, ox, oy, shx, shy, qa, ga);
+        ordered_row<THREE>(t, ra, xc + kra - 1, bc[kra - 1], x0a, xpa, ih, ca, cb, c3, ox, oy, shx, shy,
+                           kra == Nzg - 1, qa, ga);
         if (TWO)
-            ordered_row<THREE>(t, rb, xc + krb - 1, bc[krb - 1], xpa, xpb, ih, ca, cb, c3, ox, oy, 0, 0, qb, gb);
+            ordered_row<THREE>(t, rb, xc + krb - 1, bc[krb - 1], xpa, xpb, ih, ca, cb, c3, ox, oy, 0, 0, krb == Nzg - 1,
+                               qb, gb);
         if (!va) { qa = 0; ga = 0; }
         if (!vb) { qb = 0; gb = 0; }
         x1 = xc[0];

@@ -206,8 +206,6 @@ TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vec
     }
     if (d.cross) {
         if (d.per || d.ncolor != (three ? 4 : 2)) return t;
-        // (the ordered FP32 kernels leave out the centre of the first difference)
-        if (sizeof(T) == 4 && (sx(1, 2, 1) != 0.0 || (three && sy(1, 2, 1) != 0.0))) return t;
         t.mode = kTileCross;
         RowTab<T>& r = t.r;
         for (int k = 1; k <= h.Nzg; ++k) {

@@ -77,6 +77,14 @@ def test_periodic(ow3d, n):
     _compare(ow3d, p, geo, 0)
 
 
+@pytest.mark.parametrize("n", [(65, 65, 17), (129, 33, 13), (257, 65, 17)])
+def test_slope_rounded_centre_weight(ow3d, n):
+    """Spacings at which the centred difference's centre weight is not exactly
+    zero (1e-16 of the others): its terms are part of the per-phase sums."""
+    p, geo = cases.bump_3d(Nx=n[0], Ny=n[1], Nz=n[2], Lx=0.1 * (n[0] - 1), Ly=0.1 * (n[1] - 1))
+    _compare(ow3d, p, geo, 1, slope=True)
+
+
 def test_varying_depth_without_slopes(ow3d):
     """No tile form: the per-phase kernels either way, bitwise."""
     p, geo = cases.bump_3d(Nx=65, Ny=33, Nz=9, Lx=6.5, Ly=4.0)
