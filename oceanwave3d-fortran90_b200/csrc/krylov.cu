@@ -77,7 +77,7 @@ __device__ bool last_block_reduce(double* partial, int nv, int nblocks, unsigned
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned int t = atomicAdd(counter, 1u);
-        amlast = (t == gridDim.x - 1);
+        amlast = (t == gridDim.x * gridDim.y - 1);
     }
     __syncthreads();
     if (!amlast) return false;
@@ -141,36 +141,35 @@ __global__ void __launch_bounds__(kThreads) k_norm_init(const double* __restrict
     }
 }
 
-// Upper-triangular solve R y = g for the current k, one warp: R and g in shared
-// memory, lane l holding the right-hand sides of rows l and l + 32; each step
-// fixes one unknown and the lanes subtract its column. (One thread reading R
-// from memory: 18-32 us at 16-22 columns, a chain of loads.)
+// Upper-triangular solve R y = g for the current k: the block brings R and g to
+// shared memory, one thread runs the rows' chain of multiply-adds there. (The
+// same chain on R in memory, load after load: 18-32 us at 16-22 columns; the
+// columns subtracted by a warp's lanes would be shorter still, but in another
+// order of sums, which a preconditioner in FP32 magnifies.)
 // With in_basis set (left preconditioning), the coefficients of the vectors
 // the Arnoldi steps multiplied are taken to the final basis, y <- T y, so
 // that the update is x += sum_i y_i v_i.
 __global__ void __launch_bounds__(kThreads) k_backsolve(KrylovState* ks, int in_basis) {
     pdl_entry();
-    __shared__ double R[kMaxKrylov + 1][kMaxKrylov + 1], y[kMaxKrylov + 1];
+    __shared__ double R[kMaxKrylov + 1][kMaxKrylov + 1], y[kMaxKrylov + 1];   // R[row][column]
     __shared__ int kk;
     const int k0 = ks->k, tid = threadIdx.x;
     for (int t = tid; t < k0 * k0; t += blockDim.x) {
         const int c = t / k0, r = t - c * k0;
-        R[c][r] = r <= c ? ks->R[c][r] : 0.0;
+        if (r <= c) R[r][c] = ks->R[c][r];
+        if (c == 0) y[r] = ks->g[r];
     }
     __syncthreads();
-    if (tid < 32) {
+    if (tid == 0) {
         int k = k0;
         while (k > 0 && R[k - 1][k - 1] == 0.0) --k;
-        const int r0 = tid, r1 = tid + 32;
-        double g0 = r0 < k ? ks->g[r0] : 0.0, g1 = r1 < k ? ks->g[r1] : 0.0;
-        const double i0 = r0 < k ? 1.0 / R[r0][r0] : 0.0, i1 = r1 < k ? 1.0 / R[r1][r1] : 0.0;
         for (int i = k - 1; i >= 0; --i) {
-            const double v = __shfl_sync(0xffffffffu, i < 32 ? g0 * i0 : g1 * i1, i & 31);
-            if (r0 < i) g0 -= R[i][r0] * v;
-            if (r1 < i) g1 -= R[i][r1] * v;
-            if (tid == 0) y[i] = v;
+            double t = y[i];
+#pragma unroll 4
+            for (int j = i + 1; j < k; ++j) t -= R[i][j] * y[j];
+            y[i] = t / R[i][i];
         }
-        if (tid == 0) kk = k;
+        kk = k;
     }
     __syncthreads();
     const int k = kk;
@@ -229,10 +228,14 @@ __global__ void k_krylov_reset(KrylovState* ks) {
 
 // The scalar work of a step runs in the warp that ends a kernel's last block,
 // with its columns in shared memory: lane l takes entries l and l + 32, and
-// only the chain of rotations is serial, on registers' distance instead of a
-// chain of loads from the state in memory.
+// only the sums and the chain of rotations are serial, on shared memory
+// instead of a chain of loads from the state in memory.
+// The order of every FP64 sum here and in the reductions below is part of the
+// method's results in the mixed precision form: a change of rounding in the
+// last place of a coefficient reaches the FP32 preconditioner's input and
+// comes out at 1e-9 to 5e-9 of a small sloping flume's surface.
 struct ColScratch {
-    double h[kMaxKrylov + 2], cs[kMaxKrylov + 1], sn[kMaxKrylov + 1], scale[kMaxKrylov + 2];
+    double h[kMaxKrylov + 2], cs[kMaxKrylov + 1], sn[kMaxKrylov + 1], sig[kMaxKrylov + 1], hq[kMaxKrylov + 1];
 };
 
 // One warp: rotate the unrotated column col of H (w.h[0..col+1]) with
@@ -275,27 +278,33 @@ __device__ double dcgs_rotate(KrylovState* ks, ColScratch& w, int col, double g0
 // solution is a combination of those vectors).
 __device__ void dcgs_column(KrylovState* ks, ColScratch& w, int j, const double* res) {
     const int lane = threadIdx.x & 31;
-    double sig[2] = {0.0, 0.0}, sc[2] = {0.0, 0.0};
-    double g0 = 0.0, scj = ks->scale[j];
-    if (j >= 1) {
-        g0 = ks->gsave[j - 1];
-        double ss = 0.0;
+    double sig[2] = {0.0, 0.0}, sc[2] = {0.0, 0.0}, hq[2] = {0.0, 0.0};
+    double g0 = 0.0, scj = ks->scale[j], ss = 0.0, corr = 0.0;
+    if (j >= 1) g0 = ks->gsave[j - 1];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int i = lane + 32 * q;
-            if (i < j) {
-                sc[q] = ks->scale[i];
-                const double h = ks->H[j - 1][i];
-                if (i < j - 1) { w.cs[i] = ks->cs[i]; w.sn[i] = ks->sn[i]; }
-                sig[q] = sc[q] * res[2 * i];
-                ks->T[j][i] = scj * sig[q];
-                // complete column j-1: W_{j-1} = sum (h + sigma) q_i + nu q_j
-                ks->H[j - 1][i] = h + sig[q];
-                w.h[i] = h + sig[q];
-                ss += sig[q] * sig[q];
-            }
+    for (int q = 0; q < 2; ++q) {
+        const int i = lane + 32 * q;
+        if (i < j) {
+            sc[q] = ks->scale[i];
+            const double h = ks->H[j - 1][i];
+            if (i < j - 1) { w.cs[i] = ks->cs[i]; w.sn[i] = ks->sn[i]; }
+            sig[q] = __dmul_rn(sc[q], res[2 * i]);
+            hq[q] = __dmul_rn(sc[q], res[2 * i + 1]);
+            w.sig[i] = sig[q];
+            w.hq[i] = hq[q];
+            ks->T[j][i] = scj * sig[q];
+            // complete column j-1: W_{j-1} = sum (h + sigma) q_i + nu q_j
+            ks->H[j - 1][i] = w.h[i] = __dadd_rn(h, sig[q]);
         }
-        ss = warp_sum(ss);
+    }
+    __syncwarp();
+#pragma unroll 4
+    for (int i = 0; i < j; ++i) {
+        const double si = w.sig[i];
+        ss = __fma_rn(si, si, ss);
+        corr = __fma_rn(si, w.hq[i], corr);
+    }
+    if (j >= 1) {
         const double nu = sqrt(fmax(res[2 * j] - ss, 0.0));
         if (lane == 0) {
             ks->T[j][j] = scj * nu;
@@ -309,19 +318,15 @@ __device__ void dcgs_column(KrylovState* ks, ColScratch& w, int j, const double*
     } else if (lane == 0) {
         ks->T[0][0] = 1.0;   // scale_0 V_0 is final: v_0
     }
-    double corr = 0.0;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const int i = lane + 32 * q;
         if (i < j) {
-            const double hq = sc[q] * res[2 * i + 1];
-            ks->H[j][i] = hq;
-            corr += sig[q] * hq;
-            ks->coefB[i] = hq * sc[q];
+            ks->H[j][i] = hq[q];
+            ks->coefB[i] = hq[q] * sc[q];
             ks->coefA[i] = sig[q] * sc[q];
         }
     }
-    corr = warp_sum(corr);
     if (lane == 0) {
         const double hj = (j >= 1 ? res[2 * j + 1] - corr : res[2 * j + 1]) * scj;
         ks->H[j][j] = hj;
@@ -330,20 +335,24 @@ __device__ void dcgs_column(KrylovState* ks, ColScratch& w, int j, const double*
 }
 
 // Reduction: res[2v] = <V_v, V_j>, res[2v+1] = <V_v, W> for v <= j. The
-// vectors are cut into chunks of E * blockDim.x element pairs; a block takes
-// chunks in turn, keeps its thread's E pairs of V_j and W in registers, and
-// streams every V_v of the chunk once (so each vector is read from memory once
-// per step), G vectors' loads in flight together. The warp sums of G vectors'
-// 2 G values fold into each other (warp_sums), and a warp adds them to its own
+// vectors are cut into chunks of kDotE * blockDim.x element pairs; a block takes
+// chunks in turn, keeps its thread's kDotE pairs of V_j and W in registers, and
+// streams the V_v of the chunk, kDotG vectors' loads in flight together. The
+// warp sums of kDotG vectors' 2 kDotG values fold into each other (warp_sums:
+// 9 shuffles for four vectors instead of 40), and a warp adds them to its own
 // shared-memory slots; the block's slots become partial[u * gridDim.x + b];
 // the last block reduces the partials in a fixed order and runs dcgs_column.
-// E = G = 4 streams long vectors; short ones, whose few chunks leave most SMs
-// idle and whose time is the latency of the groups one after another, take
-// E = 1, G = 8.
-template <int E, int G>
-__global__ void __launch_bounds__(kThreads) k_dcgs_reduce(const double* __restrict__ V, int64_t ldv, int j,
+// Long vectors take one block per chunk, which reads every vector from memory
+// once per step. Short ones, whose few chunks leave most SMs idle and whose
+// time is the latency of the groups one after another, split the groups over
+// gridDim.y blocks, which read V_j and W again (from L2); the sums are the same.
+constexpr int kDotE = 4;
+constexpr int kDotG = 4;
+
+__global__ void __launch_bounds__(kThreads, 2) k_dcgs_reduce(const double* __restrict__ V, int64_t ldv, int j,
                                                           const double* __restrict__ W, int64_t n, double* partial,
                                                           unsigned int* counter, KrylovState* ks) {
+    constexpr int E = kDotE, G = kDotG;
     pdl_entry();
     if (ks->done) return;
     __shared__ double acc[2 * kMaxDots + 2 * G][kThreads / 32];
@@ -369,7 +378,7 @@ __global__ void __launch_bounds__(kThreads) k_dcgs_reduce(const double* __restri
         // the older basis vectors are read once per pass, so they are streamed
         // (evict-first) rather than let them push the multigrid levels and
         // their coefficient tables out of L2 before the next V-cycle
-        for (int v0 = 0; v0 <= j; v0 += G) {
+        for (int v0 = blockIdx.y * G; v0 <= j; v0 += gridDim.y * G) {
             double2 x[G][E];
 #pragma unroll
             for (int g = 0; g < G; ++g) {
@@ -401,6 +410,7 @@ __global__ void __launch_bounds__(kThreads) k_dcgs_reduce(const double* __restri
     }
     __syncthreads();
     for (int u = threadIdx.x; u < nv; u += blockDim.x) {
+        if ((u / (2 * G)) % gridDim.y != blockIdx.y) continue;
         double t = 0;
         for (int w = 0; w < nw; ++w) t += acc[u][w];
         partial[(int64_t)u * gridDim.x + blockIdx.x] = t;
@@ -494,24 +504,17 @@ __global__ void k_solve_log(const KrylovState* ks, SolveLog* out) {
 
 }  // namespace
 
-// Vectors of at most this many element pairs take the short form of the
-// reduction: fewer than four chunks of the long form per SM.
-constexpr int64_t kShortPairs = 4ll * 148 * 4 * kThreads;
-
 void launch_dcgs_reduce(const double* V, int64_t ldv, int j, const double* W, int64_t n, const DotScratch& sc,
                         KrylovState* ks, cudaStream_t st) {
-    // one block per chunk, at most two per SM (enough loads in flight, and the
-    // last block's sum over the blocks grows with them); 2(j+1) partial rows
-    const int64_t n2 = (n + 1) / 2;
-    const bool brief = n2 <= kShortPairs;
-    const int64_t chunk = (int64_t)(brief ? 1 : 4) * kThreads;
-    int64_t nb = std::min<int64_t>((n2 + chunk - 1) / chunk, std::min(sc.nblocks, 2 * 148));
+    // one block per chunk up to the scratch's blocks; 2(j+1) partial rows
+    const int64_t chunk = (int64_t)kDotE * kThreads, chunks = ((n + 1) / 2 + chunk - 1) / chunk;
+    int64_t nb = std::min<int64_t>(chunks, sc.nblocks);
     nb = std::min<int64_t>(nb, ((int64_t)(kMaxKrylov + 2) * sc.nblocks) / (2 * (j + 1)));   // scratch rows
     if (nb < 1) nb = 1;
-    if (brief)
-        launch_k(k_dcgs_reduce<1, 8>, dim3((unsigned)nb), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial, sc.counter, ks);
-    else
-        launch_k(k_dcgs_reduce<4, 4>, dim3((unsigned)nb), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial, sc.counter, ks);
+    // groups side by side while all blocks fit on the chip at once, two per SM
+    const int64_t ny = std::max<int64_t>(1, std::min<int64_t>((j + kDotG) / kDotG, 2 * 148 / nb));
+    launch_k(k_dcgs_reduce, dim3((unsigned)nb, (unsigned)ny), dim3(kThreads), 0, st, V, ldv, j, W, n, sc.partial,
+             sc.counter, ks);
 }
 
 // Blocks of a pass over n2 items with one partial sum per block.

@@ -266,9 +266,7 @@ __device__ __forceinline__ void dense_rows(int n, const T* __restrict__ M, const
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r = warp; r < n; r += nwarps) {
         const T* row = M + r * n;
-        T acc[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) acc[u] = 0;
+        T s = 0;
         for (int c = lane; c < n; c += 32 * U) {
             T m[U], v[U];
 #pragma unroll
@@ -278,13 +276,8 @@ __device__ __forceinline__ void dense_rows(int n, const T* __restrict__ M, const
                 v[u] = q < n ? b[q] : T(0);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) acc[u] += m[u] * v[u];
+            for (int u = 0; u < U; ++u) s += m[u] * v[u];
         }
-#pragma unroll
-        for (int o = U / 2; o > 0; o >>= 1)
-#pragma unroll
-            for (int u = 0; u < o; ++u) acc[u] += acc[u + o];
-        T s = acc[0];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) x[r] = s;
