@@ -1565,27 +1565,34 @@ void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross, bool
 template <typename T>
 void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
     const bool three = L.Nyg > 1, cross = t.mode == kTileCross;
-    // The largest core that leaves room for two blocks per SM, on levels with
-    // at least a tile per SM of that size; smaller levels take smaller cores.
-    static const int uni3[][2] = {{32, 8}, {16, 8}, {8, 4}}, cross3[][2] = {{16, 16}, {16, 8}, {8, 8}};
+    // Of the cores that leave room for two blocks per SM, the one of least
+    // waves x (columns of a tile with its halo + 200): a tile's time is its
+    // columns' share of the staging and the phases plus the phases' latency,
+    // worth some 200 columns. Levels of few tiles so take smaller cores, and
+    // large ones the largest that fits (way up at 1025x257x17 FP64: 16x8 80 us,
+    // 24x8 70 us; one level below, 561 tiles of 16x8 21 us, 374 of 24x8 23 us).
+    static const int uni3[][2] = {{32, 8}, {24, 8}, {16, 8}, {8, 4}}, cross3[][2] = {{16, 16}, {16, 8}, {8, 8}};
     static const int line[][2] = {{64, 1}, {32, 1}, {16, 1}};
     const int (*cand)[2] = three ? (cross ? cross3 : uni3) : line;
-    const int ncand = 3;
+    const int ncand = three && !cross ? 4 : 3;
     auto pick = [&](TileGeo& g, int halo, bool down) {
         g.halo = halo;
         bool found = false;
+        int64_t least = 0;
         TileGeo best{};
         for (int q = 0; q < ncand; ++q) {
             size_geo(L, g, cand[q][0], cand[q][1], cross, down);
-            if (g.smem > kTileSmemMax || (g.smem > kTileSmemTwo && q + 1 < ncand)) continue;
+            if (g.smem > kTileSmemMax || (g.smem > kTileSmemTwo && (found || q + 1 < ncand))) continue;
             int lanes = cross ? (L.Nzg <= 10 ? 4 : (L.Nzg <= 18 ? 8 : 16)) : 1;
             if (cross && sizeof(T) == 4 && !two_rows(L)) lanes *= 2;
             const int cols = (g.cx + 2 * halo) * (three ? g.cy + 2 * halo : 1) / L.ncolor * lanes;
             const int most = cross ? kCrossThreads : (down ? kUniThreads : 256);
             g.threads = std::min(most, std::max(256, (cols + 31) / 32 * 32));
+            const int64_t waves = (g.ntx * g.nty + 2 * 148 - 1) / (2 * 148), cost = waves * (2 * g.HW * g.PH + 200);
+            if (found && cost >= least) continue;
             found = true;
+            least = cost;
             best = g;
-            if (g.ntx * g.nty >= 148) break;
         }
         g = best;
         return found;

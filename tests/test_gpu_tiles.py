@@ -63,6 +63,14 @@ def test_slope(ow3d, n, precision):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [(513, 65, 17), (513, 129, 9)])
+def test_flat_wide_cores(ow3d, n, precision):
+    """Levels that take the 24x8 and 32x8 cores."""
+    p, geo = cases.bump_3d(Nx=n[0], Ny=n[1], Nz=n[2], Lx=0.1 * n[0], Ly=0.13 * n[1], amp=0.0)
+    _compare(ow3d, p, dict(h=geo["h"]), precision)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("n", LINE)
 def test_flume(ow3d, n, precision):
     p, geo = cases.slope_2d(Nx=n[0], Nz=n[1], L=0.1 * n[0], MGmaxgrids=n[2])
