@@ -12,15 +12,21 @@
 //                   <= 2, residual at <= 1; up 2.
 //   cross levels    down nc + 3: bottom rows at <= nc + 3, colour c at
 //                   <= nc + 2 - c, bottom rows again at <= 2, residual at <= 1;
-//                   up nc + 2.
+//                   up nc + 2. (FP32: one more on the way down.)
 // The arithmetic per row is the colour pass's (mg_device.cuh) up to the order
-// of the sums.
+// of the sums, on FP32 cross levels in the same order.
+//
+// What bounds them: the latency of the phases, not bytes. On a B200, per level
+// and V-cycle: 1025x257x17 FP64 flat 125 us (55 down, 70 up) against about 300
+// of the per-phase kernels, FP32 83 us; a 97x49x9 level 14 us; sloping 257x33x9
+// FP64 50 us, FP32 56 us. All levels of a V-cycle below 160000 points: 41 us
+// (97x49x9), 125 us (257x33x9) against 180 and 345 us in the cooperative kernel.
 //
 // On uniform levels one thread solves one column bottom to top: the sums over
 // neighbour columns do not depend on the row below, only
 // x_k = q_k - g_k x_{k-1} is a chain. On cross levels, whose rows cost an
-// order more, the lanes of a segment share a column. Columns lie in shared memory with an odd
-// pitch and the columns of one parity of i side by side, so that the threads
+// order more, the lanes of a segment share a column. Columns lie in shared
+// memory with an odd pitch and the columns of one parity of i side by side, so that the threads
 // of a warp, which take every other column, meet no bank conflict.
 #include "mg_tile.cuh"
 #include "mg_device.cuh"

@@ -15,7 +15,8 @@ the round (from the step times measured in the previous round), so small
 simulations are not held back by large ones. Each simulation's coarse
 multigrid levels run in one thread-block cluster (ow3d_set_coarse_cluster)
 rather than a cooperative grid over every SM, so that the coarse cycles of
-the simulations overlap too. A request is admitted as soon as it has arrived, a slot is
+the simulations overlap too (levels with a tile form run as plain launches
+and overlap either way). A request is admitted as soon as it has arrived, a slot is
 free and its estimated device memory (ow3d_estimate_bytes) fits in what the
 running simulations leave of the memory budget; finished simulations release
 their handle (and memory) at the end of the round in which they finish.
