@@ -357,10 +357,10 @@ __global__ void __launch_bounds__(THREE ? 256 : 256, 2)
         const int64_t q = (int64_t)blockIdx.x * cpb + c;
         const bool on = c < cpb && q < nband;
         int i = 1, j = 1;
-        if (on) band_col(q, Nxg, Nyg, all != 0, i, j);
+        if (on) band_col(q, Nxg, Nyg, (all & 1) != 0, i, j);
         extern __shared__ __align__(16) unsigned char smraw[];
         double* const sp = reinterpret_cast<double*>(smraw) + c * Nzg;
-        ho_point_general<THREE, TIN>(g, s, phi, scale, b, y, mode, zt, all > 1, i, j, k, on, sp, sp + blockDim.x,
+        ho_point_general<THREE, TIN>(g, s, phi, scale, b, y, mode, zt, (all & 2) != 0, i, j, k, on, sp, sp + blockDim.x,
                                      sp + 2 * blockDim.x);
         return;
     }
@@ -469,7 +469,7 @@ void launch_impl(const HoGrid& g, const Surface& s, const TIN* phi, const double
         attr_set.fetch_or(bit, std::memory_order_relaxed);
     }
     launch_k(k_ho_matvec<NZG, THREE, TIN>, dim3(band_blocks + tiles), dim3(threads), smem, st, 
-        g, s, phi, scale, b, y, mode, zt, band_blocks, nband, split ? 0 : (uniform && !g.per ? 2 : 1), tiles_x);
+        g, s, phi, scale, b, y, mode, zt, band_blocks, nband, (split ? 0 : 1) + (uniform && !g.per ? 2 : 0), tiles_x);
 }
 
 template <bool THREE, typename TIN>

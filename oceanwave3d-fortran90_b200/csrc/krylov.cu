@@ -70,7 +70,10 @@ __device__ void block_store_partials(const double* acc, int nv, double* partial,
 // The last block to finish sums the partials: warp w reduces vectors
 // v = w, w + nwarps, ...; lane l adds blocks l, l+32, ... in order and the
 // warp tree combines the lanes (a fixed order: deterministic results).
-// Returns true in that block.
+// Returns true in that block. G vectors a warp at a time, U L2 loads of each in
+// flight per lane: <1, 20> takes the one sum of a pass over the grid's at most
+// 592 blocks in one round.
+template <int G, int U>
 __device__ bool last_block_reduce(double* partial, int nv, int nblocks, unsigned int* counter, double* out) {
     __shared__ bool amlast;
     __threadfence();
@@ -83,27 +86,29 @@ __device__ bool last_block_reduce(double* partial, int nv, int nblocks, unsigned
     if (!amlast) return false;
     __threadfence();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // three vectors a warp, four L2 loads of each in flight per lane
-    for (int v0 = wid; v0 < nv; v0 += 3 * nw) {
-        double s[3] = {0.0, 0.0, 0.0};
-        for (int b = lane; b < nblocks; b += 4 * 32) {
-            double q[3][4];
+    for (int v0 = wid; v0 < nv; v0 += G * nw) {
+        double s[G];
 #pragma unroll
-            for (int g = 0; g < 3; ++g)
+        for (int g = 0; g < G; ++g) s[g] = 0.0;
+        for (int b = lane; b < nblocks; b += U * 32) {
+            double q[G][U];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
                     const int v = v0 + g * nw, bb = b + 32 * u;
                     q[g][u] = v < nv && bb < nblocks ? __ldcg(partial + (int64_t)v * nblocks + bb) : 0.0;
                 }
 #pragma unroll
-            for (int g = 0; g < 3; ++g)
+            for (int g = 0; g < G; ++g)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) s[g] += q[g][u];
+                for (int u = 0; u < U; ++u) s[g] += q[g][u];
         }
 #pragma unroll
-        for (int g = 0; g < 3; ++g) s[g] = warp_sum(s[g]);
+        for (int g = 0; g < G; ++g) s[g] = warp_sum(s[g]);
         if (lane == 0)
-            for (int g = 0; g < 3; ++g)
+#pragma unroll
+            for (int g = 0; g < G; ++g)
                 if (v0 + g * nw < nv) out[v0 + g * nw] = s[g];
     }
     __syncthreads();
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(kThreads) k_norm_init(const double* __restrict
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += stride) acc[0] += v[t] * v[t];
     block_store_partials(acc, 1, partial, nblocks);
     __shared__ double res[1];
-    if (last_block_reduce(partial, 1, nblocks, counter, res)) {
+    if (last_block_reduce<1, 20>(partial, 1, nblocks, counter, res)) {
         if (threadIdx.x == 0) {
             const double beta = sqrt(res[0]);
             ks->beta = beta;
@@ -416,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_dcgs_reduce(const double* __res
         partial[(int64_t)u * gridDim.x + blockIdx.x] = t;
     }
     __shared__ double res[2 * kMaxDots];
-    if (!last_block_reduce(partial, nv, gridDim.x, counter, res)) return;
+    if (!last_block_reduce<3, 4>(partial, nv, gridDim.x, counter, res)) return;
     __shared__ ColScratch scratch;
     if (wid == 0) dcgs_column(ks, scratch, j, res);
 }
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(kThreads) k_dcgs_update(double* __restrict__ V
     }
     block_store_partials(acc, 1, partial, nblocks);
     __shared__ double res[1];
-    if (!last_block_reduce(partial, 1, nblocks, counter, res)) return;
+    if (!last_block_reduce<1, 20>(partial, 1, nblocks, counter, res)) return;
     __shared__ ColScratch w;
     if (threadIdx.x >= 32) return;
     const int lane = threadIdx.x;
