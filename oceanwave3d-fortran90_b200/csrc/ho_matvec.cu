@@ -24,8 +24,8 @@
 //    per point (k fastest, whole columns per block) reading phi from global
 //    memory, per-position stencils from the tables; the horizontal
 //    derivatives of a column's levels meet in shared memory before its rows
-//    are formed. These blocks come first in the grid so that they start early
-//    and overlap the tiles. Grids of fewer tiles than SMs run wholly this way:
+//    are formed. These short blocks come last in the grid and fill the tiles'
+//    last wave. Grids of fewer tiles than SMs run wholly this way:
 //    a tile's thread walks its levels one after another, which a small grid
 //    has too few warps to hide (one thread per column in the bands, and tiles
 //    at any size: 23 us at 257x33x9, 11 us at 513x9).
@@ -352,9 +352,10 @@ __global__ void __launch_bounds__(THREE ? 256 : 256, 2)
     const int Nxg = g.Nxg, Nyg = g.Nyg, Nzg = NZG > 0 ? NZG : g.Nzg;
     const double scale = dscale ? *dscale : 1.0;
     const int tid = threadIdx.x;
-    if ((int)blockIdx.x < band_blocks) {
+    const int tiles = (int)gridDim.x - band_blocks;
+    if ((int)blockIdx.x >= tiles) {
         const int cpb = blockDim.x / Nzg, c = tid / Nzg, k = tid - c * Nzg + 1;   // whole columns per block
-        const int64_t q = (int64_t)blockIdx.x * cpb + c;
+        const int64_t q = (int64_t)((int)blockIdx.x - tiles) * cpb + c;
         const bool on = c < cpb && q < nband;
         int i = 1, j = 1;
         if (on) band_col(q, Nxg, Nyg, (all & 1) != 0, i, j);
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(THREE ? 256 : 256, 2)
     extern __shared__ __align__(16) unsigned char smraw[];
     TIN* const sm = reinterpret_cast<TIN*>(smraw);
     const int NZP = Nzg | 1;   // odd column pitch
-    const int t = (int)blockIdx.x - band_blocks;
+    const int t = (int)blockIdx.x;
     const int ty_ = t / tiles_x, tx_ = t - ty_ * tiles_x;
     const int i0 = kBand + 1 + tx_ * BX;
     const int j0 = THREE ? kBand + 1 + ty_ * BY : 1;
