@@ -64,6 +64,16 @@ int ow3d_test_set_pdl(int on);
 /* 0: every multigrid level takes the per-phase kernels, 1 (default): levels
  * that have a tile form (mg_tile.cu) take it. Returns the previous value. */
 int ow3d_test_set_tiles(int on);
+/* The form that multigrid level `level` (0 = coarsest) of such a simulation
+ * takes in the fused tile kernels, in the precision of p (host only): mode 0
+ * none (the per-phase kernels), 1 uniform, 2 cross; where it has one, the tile
+ * geometry of its two launches, 10 values each: tiles in x and y, the largest
+ * core in x and y, halo, column slots per parity and row, rows, column pitch,
+ * threads, bytes of shared memory. nlevels: levels of the hierarchy. The
+ * outputs may be null. (Level 0 and the levels of the dense operator are not
+ * launched as tiles.) */
+int ow3d_test_tile_form(const ow3d_params* p, const double* h, const double* hx, const double* hxx, const double* hy,
+                        const double* hyy, int level, int* nlevels, int* mode, int* down, int* up);
 long long ow3d_test_set_tail_max_points(long long points);
 int ow3d_test_set_tail_cluster(int blocks);
 

@@ -74,6 +74,8 @@ def lib():
         L.ow3d_test_set_tail_cluster.argtypes = [_C.c_int]
         L.ow3d_test_set_pdl.argtypes = [_C.c_int]
         L.ow3d_test_set_tiles.argtypes = [_C.c_int]
+        I = _C.POINTER(_C.c_int)
+        L.ow3d_test_tile_form.argtypes = [_C.c_void_p, D, D, D, D, D, _C.c_int, I, I, I, I]
         L.ow3d_test_set_colour_prefetch.argtypes = [_C.c_int]
         L.ow3d_test_graph_count.argtypes = [_C.c_void_p]
         L.ow3d_test_step_graph_count.argtypes = [_C.c_void_p]

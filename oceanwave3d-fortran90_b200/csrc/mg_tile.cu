@@ -1545,7 +1545,7 @@ void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross, bool
     const bool three = L.Nyg > 1;
     auto cores = [](int n, int c, int& nt, int& q, int& rem, int& most) {
         nt = (n + c - 1) / c;
-        if (n / nt < 3) nt = n / 3;      // n >= 4 columns on every level
+        if (n / nt < 3) nt = n / 3;      // n >= 4: of a periodic level the distinct columns (tile_level)
         q = n / nt;
         rem = n - q * nt;
         most = q + (rem > 0 ? 1 : 0);

@@ -180,7 +180,8 @@ int upload(ow3d_handle* H, T** p, const std::vector<double>& v) {
 // limit: 2e-9; two-dimensional 65x17 and 257x17 flumes: 1e-9), in FP64 by
 // 1e-12, so the FP32 cross kernels keep the per-phase kernels' order; flat
 // levels move by 1e-11 at most in FP32. Periodic levels with an odd period
-// (the two colours would meet at its ends) have none.
+// (the two colours would meet at its ends) have none, nor has a period of two
+// columns (a core holds three or more).
 template <typename T>
 TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vector<double>& cf,
                         const std::vector<double>& bt) {
@@ -223,7 +224,7 @@ TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vec
         tile_geometry(d, t);
         return t;
     }
-    if (d.ncolor != 2 || (d.per && (nx - 3) % 2 != 0)) return t;
+    if (d.ncolor != 2 || (d.per && ((nx - 3) % 2 != 0 || nx - 3 < 4))) return t;
     const size_t q0 = 1 + (size_t)nx * (jlo - 1);
     for (int j = jlo; j <= jhi; ++j)
         for (int i = 2; i <= ihi; ++i) {
@@ -253,6 +254,60 @@ TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vec
     return t;
 }
 
+// A level's sizes and switches.
+template <typename T>
+void level_shape(const LevelHost& h, int per, LevelDev<T>& d) {
+    d.Nx = h.Nx; d.Ny = h.Ny; d.Nz = h.Nz; d.Nxg = h.Nxg; d.Nyg = h.Nyg; d.Nzg = h.Nzg;
+    d.pitch = h.Nxg;
+    d.N = (int64_t)h.Nxg * h.Nyg * h.Nzg;
+    d.ncolor = h.ncolor; d.xc = h.xc; d.yc = h.yc; d.zc = h.zc;
+    d.per = per;
+    d.cross = 0;
+    for (size_t q = 0; q < h.hx.size(); ++q) if (h.hx[q] != 0.0 || h.hy[q] != 0.0) { d.cross = 1; break; }
+}
+
+// Per column, the coefficients of the interior rows (cf, 4 values) and of the
+// bottom row (bt, 8 values).
+void level_coefs(const LevelHost& h, std::vector<double>& cf, std::vector<double>& bt) {
+    const bool three = h.Nyg > 1;   // 2-D levels ignore any y-derivatives of h
+    cf.resize(4 * h.h.size());
+    for (size_t q = 0; q < h.h.size(); ++q) {
+        const double ih = 1.0 / h.h[q];
+        const double hyq = three ? h.hy[q] : 0.0, hyyq = three ? h.hyy[q] : 0.0;
+        cf[4 * q + 0] = ih;
+        cf[4 * q + 1] = h.hx[q] * ih;
+        cf[4 * q + 2] = hyq * ih;
+        cf[4 * q + 3] = (h.hxx[q] + hyyq) * ih - 2.0 * (h.hx[q] * h.hx[q] + hyq * hyq) * ih * ih;
+    }
+    // bottom row (k = 1) of column (i, j): f Dz(x)|_2 + h_x Dx(x)|_2 + h_y Dy(x)|_2
+    // with f = 1/h + h_x s2 + h_y s4 at sigma_2 (BuildLinearSystemMatrix.f90:50-70)
+    bt.assign(8 * h.h.size(), 0.0);
+    const double omb = 1.0 - h.zs[1];
+    const double z0 = h.SZ.w[3 + 0], z1 = h.SZ.w[3 + 1], z2 = h.SZ.w[3 + 2];   // order 1, row 2
+    for (int jj = 1; jj <= h.Nyg; ++jj)
+        for (int ii = 1; ii <= h.Nxg; ++ii) {
+            const size_t q = (size_t)(ii - 1) + (size_t)h.Nxg * (jj - 1);
+            const double ih = 1.0 / h.h[q];
+            const double hxq = h.hx[q], hyq = three ? h.hy[q] : 0.0;
+            const double s2 = omb * (hxq * ih), s4 = omb * (hyq * ih);
+            const double f = three ? (ih + hxq * s2 + hyq * s4) : (ih + hxq * s2);
+            const double* wx = &h.SX.w[(size_t)(ii - 1) * 3];
+            double* o = &bt[8 * q];
+            o[0] = f * z1 + hxq * wx[1];
+            o[1] = f * z2;
+            o[2] = hxq * wx[0];
+            o[3] = hxq * wx[2];
+            if (three) {
+                const double* wy = &h.SY.w[(size_t)(jj - 1) * 3];
+                o[0] += hyq * wy[1];
+                o[4] = hyq * wy[0];
+                o[5] = hyq * wy[2];
+            }
+            o[6] = 1.0 / (f * z0);
+            o[7] = f * z0;
+        }
+}
+
 template <typename T>
 int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
     const int L = (int)H->G.levels.size();
@@ -261,13 +316,7 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
     for (int l = 0; l < L; ++l) {
         const LevelHost& h = H->G.levels[l];
         LevelDev<T>& d = S.lev[l];
-        d.Nx = h.Nx; d.Ny = h.Ny; d.Nz = h.Nz; d.Nxg = h.Nxg; d.Nyg = h.Nyg; d.Nzg = h.Nzg;
-        d.pitch = h.Nxg;
-        d.N = (int64_t)h.Nxg * h.Nyg * h.Nzg;
-        d.ncolor = h.ncolor; d.xc = h.xc; d.yc = h.yc; d.zc = h.zc;
-        d.per = H->G.per;
-        d.cross = 0;
-        for (size_t q = 0; q < h.hx.size(); ++q) if (h.hx[q] != 0.0 || h.hy[q] != 0.0) { d.cross = 1; break; }
+        level_shape(h, H->G.per, d);
         T *sx, *sy, *sz, *zs, *hh, *hx, *hxx, *hy, *hyy;
         TRY(upload(H, &sx, h.SX.w)); TRY(upload(H, &sy, h.SY.w.empty() ? std::vector<double>(1, 0.0) : h.SY.w));
         TRY(upload(H, &sz, h.SZ.w)); TRY(upload(H, &zs, h.zs));
@@ -286,53 +335,11 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
         };
         TRY(upload(H, &ix, recip(h.x))); TRY(upload(H, &iy, recip(h.y))); TRY(upload(H, &iz, recip(h.z)));
         d.ix = ix; d.iy = iy; d.iz = iz;
-        std::vector<double> cf(4 * h.h.size()), bt(8 * h.h.size(), 0.0);
-        {
-            for (size_t q = 0; q < h.h.size(); ++q) {
-                const double ih = 1.0 / h.h[q];
-                const bool three = h.Nyg > 1;   // 2-D levels ignore any y-derivatives of h
-                const double hyq = three ? h.hy[q] : 0.0, hyyq = three ? h.hyy[q] : 0.0;
-                cf[4 * q + 0] = ih;
-                cf[4 * q + 1] = h.hx[q] * ih;
-                cf[4 * q + 2] = hyq * ih;
-                cf[4 * q + 3] = (h.hxx[q] + hyyq) * ih - 2.0 * (h.hx[q] * h.hx[q] + hyq * hyq) * ih * ih;
-            }
-            T* c;
-            TRY(upload(H, &c, cf));
-            d.cf = c;
-        }
-        {
-            // bottom row (k = 1) of column (i, j): f Dz(x)|_2 + h_x Dx(x)|_2 + h_y Dy(x)|_2
-            // with f = 1/h + h_x s2 + h_y s4 at sigma_2 (BuildLinearSystemMatrix.f90:50-70)
-            const bool three = h.Nyg > 1;
-            const double omb = 1.0 - h.zs[1];
-            const double z0 = h.SZ.w[3 + 0], z1 = h.SZ.w[3 + 1], z2 = h.SZ.w[3 + 2];   // order 1, row 2
-            for (int jj = 1; jj <= h.Nyg; ++jj)
-                for (int ii = 1; ii <= h.Nxg; ++ii) {
-                    const size_t q = (size_t)(ii - 1) + (size_t)h.Nxg * (jj - 1);
-                    const double ih = 1.0 / h.h[q];
-                    const double hxq = h.hx[q], hyq = three ? h.hy[q] : 0.0;
-                    const double s2 = omb * (hxq * ih), s4 = omb * (hyq * ih);
-                    const double f = three ? (ih + hxq * s2 + hyq * s4) : (ih + hxq * s2);
-                    const double* wx = &h.SX.w[(size_t)(ii - 1) * 3];
-                    double* o = &bt[8 * q];
-                    o[0] = f * z1 + hxq * wx[1];
-                    o[1] = f * z2;
-                    o[2] = hxq * wx[0];
-                    o[3] = hxq * wx[2];
-                    if (three) {
-                        const double* wy = &h.SY.w[(size_t)(jj - 1) * 3];
-                        o[0] += hyq * wy[1];
-                        o[4] = hyq * wy[0];
-                        o[5] = hyq * wy[2];
-                    }
-                    o[6] = 1.0 / (f * z0);
-                    o[7] = f * z0;
-                }
-            T* btd;
-            TRY(upload(H, &btd, bt));
-            d.bt = btd;
-        }
+        std::vector<double> cf, bt;
+        level_coefs(h, cf, bt);
+        T *cfd, *btd;
+        TRY(upload(H, &cfd, cf)); TRY(upload(H, &btd, bt));
+        d.cf = cfd; d.bt = btd;
         d.mz = div_magic((uint64_t)d.Nzg);
         d.mx = div_magic((uint64_t)d.Nxg);
         div_magic32((uint32_t)d.Nzg, d.mz32, d.sz32);
@@ -2263,6 +2270,32 @@ int ow3d_test_pdamp_setup(const ow3d_params* p, int* i1, int* nd, double* gamPhi
     if (gamEta) std::copy(d.gamEta.begin(), d.gamEta.end(), gamEta);
     if (L) std::copy(d.L.begin(), d.L.end(), L);
     if (Linv) std::copy(d.Linv.begin(), d.Linv.end(), Linv);
+    return OW3D_OK;
+}
+
+int ow3d_test_tile_form(const ow3d_params* p, const double* h, const double* hx, const double* hxx, const double* hy,
+                        const double* hyy, int level, int* nlevels, int* mode, int* down, int* up) {
+    if (!p || !h) return OW3D_ERR_BAD_INPUT;
+    std::string e;
+    GridHost G;
+    if (int r = build_grid(*p, h, hx, hxx, hy, hyy, G, &e)) { g_last_error = e; return r; }
+    if (nlevels) *nlevels = (int)G.levels.size();
+    if (level < 0 || level >= (int)G.levels.size()) return OW3D_ERR_BAD_INPUT;
+    const LevelHost& L = G.levels[(size_t)level];
+    std::vector<double> cf, bt;
+    level_coefs(L, cf, bt);
+    auto form = [&](auto d) {
+        level_shape(L, G.per, d);
+        const auto t = tile_level(L, d, cf, bt);
+        if (mode) *mode = t.mode;
+        auto put = [](const TileGeo& g, int* o) {
+            const int v[] = {g.ntx, g.nty, g.cx, g.cy, g.halo, g.HW, g.PH, g.NZP, g.threads, (int)g.smem};
+            if (o) std::copy(v, v + 10, o);
+        };
+        if (t.mode != kTileNone) { put(t.down, down); put(t.up, up); }
+    };
+    if (p->precision == OW3D_PREC_MIXED) form(LevelDev<float>{});
+    else form(LevelDev<double>{});
     return OW3D_OK;
 }
 
