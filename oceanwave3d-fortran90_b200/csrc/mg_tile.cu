@@ -40,6 +40,7 @@ using namespace mgdev;
 
 constexpr int kCrossThreads = 512, kUniThreads = 320, kOrderedThreads = 512;
 constexpr size_t kTileSmemMax = 220 * 1024, kTileSmemTwo = 112 * 1024;
+constexpr int kTileMaxRows = 65535;   // blocks of a grid in y: longer basins take the per-phase kernels
 
 // Core and staged region of a block, 1-based columns; on a periodic level i
 // runs past the ends and is taken cyclically (gcol).
@@ -1588,6 +1589,7 @@ void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
         TileGeo best{};
         for (int q = 0; q < ncand; ++q) {
             size_geo(L, g, cand[q][0], cand[q][1], cross, down);
+            if (g.nty > kTileMaxRows) continue;
             if (g.smem > kTileSmemMax || (g.smem > kTileSmemTwo && (found || q + 1 < ncand))) continue;
             int lanes = cross ? (L.Nzg <= 10 ? 4 : (L.Nzg <= 18 ? 8 : 16)) : 1;
             if (cross && sizeof(T) == 4 && !two_rows(L)) lanes *= 2;

@@ -15,23 +15,23 @@ NONE, UNIFORM, CROSS = 0, 1, 2
 GEO = ("ntx", "nty", "cx", "cy", "halo", "HW", "PH", "NZP", "threads", "smem")
 
 
-def forms(ow3d, p, geo, precision=0):
-    """Per level (0 = coarsest) the mode and the two launches' geometry."""
+def form(ow3d, p, geo, level, precision=0):
     L = ow3d.lib()
     p.precision = precision
     z = np.zeros_like(geo["h"])
     a = [np.ascontiguousarray(geo.get(k, z), dtype=np.float64) for k in ("h", "hx", "hxx", "hy", "hyy")]
     D = C.POINTER(C.c_double)
     n, mode = C.c_int(), C.c_int()
-    out, l = [], 0
-    while True:
-        down, up = (C.c_int * 10)(), (C.c_int * 10)()
-        r = L.ow3d_test_tile_form(C.byref(p), *[v.ctypes.data_as(D) for v in a], l, C.byref(n), C.byref(mode), down, up)
-        assert r == 0, L.ow3d_last_error()
-        out.append((mode.value, dict(zip(GEO, down)), dict(zip(GEO, up))))
-        l += 1
-        if l == n.value:
-            return out
+    down, up = (C.c_int * 10)(), (C.c_int * 10)()
+    r = L.ow3d_test_tile_form(C.byref(p), *[v.ctypes.data_as(D) for v in a], level, C.byref(n), C.byref(mode), down, up)
+    assert r == 0, L.ow3d_last_error()
+    return n.value, (mode.value, dict(zip(GEO, down)), dict(zip(GEO, up)))
+
+
+def forms(ow3d, p, geo, precision=0):
+    """Per level (0 = coarsest) the mode and the two launches' geometry."""
+    n, f = form(ow3d, p, geo, 0, precision)
+    return [f] + [form(ow3d, p, geo, l, precision)[1] for l in range(1, n)]
 
 
 def periodic(ow3d, nx, nz):
@@ -55,6 +55,20 @@ def test_short_periods(ow3d, n, precision):
         if mode:
             for g in (down, up):
                 assert g["ntx"] * g["cx"] >= m and 3 <= g["cx"]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_long_in_y(ow3d, precision):
+    """524289 points in y: cores of 8 rows would be 65537 blocks in y, past the
+    65535 a launch may have. A launch's tiles stay within that, or the level
+    has no tile form."""
+    for ny, levels in ((524289, 16), (262145, 15)):
+        p, geo = cases.bump_3d(Nx=7, Ny=ny, Nz=7, Lx=0.7, Ly=0.1 * ny, amp=0.0, MGmaxgrids=levels)
+        n, (mode, down, up) = form(ow3d, p, dict(h=geo["h"]), levels - 1, precision)
+        assert n == levels
+        assert mode == (NONE if ny == 524289 else UNIFORM)
+        if mode:
+            assert max(down["nty"], up["nty"]) <= 65535
 
 
 @pytest.mark.gpu
