@@ -170,7 +170,8 @@ int upload(ow3d_handle* H, T** p, const std::vector<double>& v) {
 
 #define TRY(x) do { int r_ = (x); if (r_) return r_; } while (0)
 
-// The form a level takes in the fused tile kernels, and its row constants.
+// The form a level takes in the fused tile kernels, and its row constants. cf,
+// bt, same: level_coefs.
 // Both forms need a uniform grid in x and y (one centred stencil for all
 // interior columns, checked value by value). Uniform: no mixed-derivative
 // terms and the same coefficients in every interior column (flat bottom) -- a
@@ -184,7 +185,7 @@ int upload(ow3d_handle* H, T** p, const std::vector<double>& v) {
 // columns (a core holds three or more).
 template <typename T>
 TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vector<double>& cf,
-                        const std::vector<double>& bt) {
+                        const std::vector<double>& bt, bool same) {
     TileLevel<T> t;
     if (h.Nzg > kTileMaxNzg || h.Nzg < 5) return t;
     const bool three = h.Nyg > 1;
@@ -225,13 +226,8 @@ TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vec
         return t;
     }
     if (d.ncolor != 2 || (d.per && ((nx - 3) % 2 != 0 || nx - 3 < 4))) return t;
+    if (!same) return t;
     const size_t q0 = 1 + (size_t)nx * (jlo - 1);
-    for (int j = jlo; j <= jhi; ++j)
-        for (int i = 2; i <= ihi; ++i) {
-            const size_t q = (size_t)(i - 1) + (size_t)nx * (j - 1);
-            for (int m = 0; m < 4; ++m) if (cf[4 * q + m] != cf[4 * q0 + m]) return t;
-            for (int m = 0; m < 8; ++m) if (bt[8 * q + m] != bt[8 * q0 + m]) return t;
-        }
     for (int m = 2; m < 6; ++m) if (bt[8 * q0 + m] != 0.0) return t;
     t.mode = kTileUniform;
     UniTab<T>& u = t.u;
@@ -267,36 +263,39 @@ void level_shape(const LevelHost& h, int per, LevelDev<T>& d) {
 }
 
 // Per column, the coefficients of the interior rows (cf, 4 values) and of the
-// bottom row (bt, 8 values).
-void level_coefs(const LevelHost& h, std::vector<double>& cf, std::vector<double>& bt) {
+// bottom row (bt, 8 values). Returns whether all interior columns (periodic x:
+// the distinct ones) carry the same: compared as they are formed, column by
+// column, since a pass of its own over the tables costs as much as forming them.
+bool level_coefs(const LevelHost& h, int per, std::vector<double>& cf, std::vector<double>& bt) {
     const bool three = h.Nyg > 1;   // 2-D levels ignore any y-derivatives of h
     cf.resize(4 * h.h.size());
-    for (size_t q = 0; q < h.h.size(); ++q) {
-        const double ih = 1.0 / h.h[q];
-        const double hyq = three ? h.hy[q] : 0.0, hyyq = three ? h.hyy[q] : 0.0;
-        cf[4 * q + 0] = ih;
-        cf[4 * q + 1] = h.hx[q] * ih;
-        cf[4 * q + 2] = hyq * ih;
-        cf[4 * q + 3] = (h.hxx[q] + hyyq) * ih - 2.0 * (h.hx[q] * h.hx[q] + hyq * hyq) * ih * ih;
-    }
-    // bottom row (k = 1) of column (i, j): f Dz(x)|_2 + h_x Dx(x)|_2 + h_y Dy(x)|_2
-    // with f = 1/h + h_x s2 + h_y s4 at sigma_2 (BuildLinearSystemMatrix.f90:50-70)
-    bt.assign(8 * h.h.size(), 0.0);
+    bt.resize(8 * h.h.size());
     const double omb = 1.0 - h.zs[1];
     const double z0 = h.SZ.w[3 + 0], z1 = h.SZ.w[3 + 1], z2 = h.SZ.w[3 + 2];   // order 1, row 2
+    const int jlo = three ? 2 : 1, jhi = three ? h.Nyg - 1 : 1, ihi = per ? h.Nxg - 2 : h.Nxg - 1;
+    const size_t q0 = 1 + (size_t)h.Nxg * (jlo - 1);   // the first interior column
+    bool same = true;
     for (int jj = 1; jj <= h.Nyg; ++jj)
         for (int ii = 1; ii <= h.Nxg; ++ii) {
             const size_t q = (size_t)(ii - 1) + (size_t)h.Nxg * (jj - 1);
             const double ih = 1.0 / h.h[q];
-            const double hxq = h.hx[q], hyq = three ? h.hy[q] : 0.0;
+            const double hxq = h.hx[q], hyq = three ? h.hy[q] : 0.0, hyyq = three ? h.hyy[q] : 0.0;
+            double* const c = &cf[4 * q];
+            c[0] = ih;
+            c[1] = hxq * ih;
+            c[2] = hyq * ih;
+            c[3] = (h.hxx[q] + hyyq) * ih - 2.0 * (hxq * hxq + hyq * hyq) * ih * ih;
+            // bottom row (k = 1) of column (i, j): f Dz(x)|_2 + h_x Dx(x)|_2 + h_y Dy(x)|_2
+            // with f = 1/h + h_x s2 + h_y s4 at sigma_2 (BuildLinearSystemMatrix.f90:50-70)
             const double s2 = omb * (hxq * ih), s4 = omb * (hyq * ih);
             const double f = three ? (ih + hxq * s2 + hyq * s4) : (ih + hxq * s2);
             const double* wx = &h.SX.w[(size_t)(ii - 1) * 3];
-            double* o = &bt[8 * q];
+            double* const o = &bt[8 * q];
             o[0] = f * z1 + hxq * wx[1];
             o[1] = f * z2;
             o[2] = hxq * wx[0];
             o[3] = hxq * wx[2];
+            o[4] = o[5] = 0.0;
             if (three) {
                 const double* wy = &h.SY.w[(size_t)(jj - 1) * 3];
                 o[0] += hyq * wy[1];
@@ -305,7 +304,13 @@ void level_coefs(const LevelHost& h, std::vector<double>& cf, std::vector<double
             }
             o[6] = 1.0 / (f * z0);
             o[7] = f * z0;
+            if (same && ii >= 2 && ii <= ihi && jj >= jlo && jj <= jhi) {
+                const double *c0 = &cf[4 * q0], *o0 = &bt[8 * q0];
+                for (int m = 0; m < 4; ++m) same = same && c[m] == c0[m];
+                for (int m = 0; m < 8; ++m) same = same && o[m] == o0[m];
+            }
         }
+    return same;
 }
 
 template <typename T>
@@ -336,7 +341,7 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
         TRY(upload(H, &ix, recip(h.x))); TRY(upload(H, &iy, recip(h.y))); TRY(upload(H, &iz, recip(h.z)));
         d.ix = ix; d.iy = iy; d.iz = iz;
         std::vector<double> cf, bt;
-        level_coefs(h, cf, bt);
+        const bool same = level_coefs(h, d.per, cf, bt);
         T *cfd, *btd;
         TRY(upload(H, &cfd, cf)); TRY(upload(H, &btd, bt));
         d.cf = cfd; d.bt = btd;
@@ -397,7 +402,7 @@ int build_levels(ow3d_handle* H, MgSet<T>& S, bool alloc_fine_x) {
             TRY(upload(H, &a1, wx_)); TRY(upload(H, &a2, wy_)); TRY(upload(H, &a3, wz_));
             d.pwx = a1; d.pwy = a2; d.pwz = a3;
         }
-        if (l > 0) S.tile[(size_t)l] = tile_level<T>(h, d, cf, bt);
+        if (l > 0) S.tile[(size_t)l] = tile_level<T>(h, d, cf, bt, same);
         T* r;
         TRY(dalloc(H, &r, d.N)); d.rv = r;
         if (l < L - 1) {
@@ -2283,10 +2288,10 @@ int ow3d_test_tile_form(const ow3d_params* p, const double* h, const double* hx,
     if (level < 0 || level >= (int)G.levels.size()) return OW3D_ERR_BAD_INPUT;
     const LevelHost& L = G.levels[(size_t)level];
     std::vector<double> cf, bt;
-    level_coefs(L, cf, bt);
+    const bool same = level_coefs(L, G.per, cf, bt);
     auto form = [&](auto d) {
         level_shape(L, G.per, d);
-        const auto t = tile_level(L, d, cf, bt);
+        const auto t = tile_level(L, d, cf, bt, same);
         if (mode) *mode = t.mode;
         auto put = [](const TileGeo& g, int* o) {
             const int v[] = {g.ntx, g.nty, g.cx, g.cy, g.halo, g.HW, g.PH, g.NZP, g.threads, (int)g.smem};

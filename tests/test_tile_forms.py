@@ -71,6 +71,23 @@ def test_long_in_y(ow3d, precision):
             assert max(down["nty"], up["nty"]) <= 65535
 
 
+@pytest.mark.parametrize("field", ["h", "hxx", "hyy"])
+@pytest.mark.parametrize("at", [(1, 1), (1, -2), (-2, 1), (-2, -2), (16, 20)])
+def test_one_column_differs(ow3d, field, at):
+    """The uniform form needs the same coefficients in every interior column:
+    one that differs, the first, the last or any other, takes it from the
+    level; a ghost column does not."""
+    p, geo = cases.bump_3d(Nx=33, Ny=33, Nz=9, Lx=3.3, Ly=3.3, amp=0.0)
+    geo = {k: np.array(v) for k, v in geo.items()}
+    assert forms(ow3d, p, geo)[-1][0] == UNIFORM
+    f = geo[field].reshape(35, 35)
+    f[0, 0] += 0.1
+    f[-1, 3] += 0.1
+    assert forms(ow3d, p, geo)[-1][0] == UNIFORM
+    f[at] += 1e-12
+    assert forms(ow3d, p, geo)[-1][0] == NONE
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", SHORT)
 def test_short_periods_match_oracle(ow3d, oracle, n):
