@@ -399,28 +399,47 @@ __device__ __forceinline__ RowConst<T> row_const(const LevelDev<T>& L) {
     return c;
 }
 
-// The task of column (i, j) for its segment (act false: the segment joins the
-// warp's shuffles and stores nothing).
 template <typename T, bool THREE, int S, bool CROSS>
-__device__ __forceinline__ void colour_col1(const LevelDev<T>& L, int i, int j, bool act, const RowConst<T>& rk) {
+__device__ void colour_warp(const LevelDev<T>& L, int colour, int base, const RowConst<T>& rk) {
     const int Nxg = L.Nxg, Nyg = L.Nyg, Nzg = L.Nzg, R = Nzg - 2;
     const int lane = threadIdx.x & 31, r = lane & (S - 1);
+    const int nxi = Nxg - 2 - L.per, nyi = THREE ? Nyg - 2 : 1;
+    // columns of this colour: every other i (and every other j with 4 colours)
+    const bool four = (L.ncolor == 4);
+    const int ni = (nxi + 1) / 2;
+    const int nj = four ? (nyi + 1) / 2 : nyi;
+    const int total = ni * nj;                // columns of one colour (< 2^31)
     const unsigned segmask = 0xffffffffu;   // the whole warp runs the scan together
     T* const X = L.xv;
     const T* const B = L.bv;
+
+    const int q = base + (lane / S);
+    bool act = q < total;
+    int i = 2, j = THREE ? 2 : 1;
+    if (act) {
+        const int tj = q / ni, ti = q - tj * ni;   // 32-bit division
+        if (four) {
+            j = THREE ? 2 + 2 * tj + (colour >> 1) : 1;
+            i = 2 + 2 * ti + (colour & 1);
+        } else {
+            j = THREE ? 2 + tj : 1;
+            i = 2 + 2 * ti + ((colour + j) & 1);    // (i + j) & 1 == colour
+        }
+        act = (i <= Nxg - 1 - L.per) && (!THREE || j <= Nyg - 1);
+    }
     const bool rowact = act && (r < R);
     const int k = r + 2;
     // the column's base; neighbours and rows are 32-bit offsets from it
     // (every level has fewer than 2^31 points)
     const int c = (i - 1) + Nxg * (j - 1);
-    T* const xc = X + IC(L, i, j) * Nzg;
-    const T* const bc = B + IC(L, i, j) * Nzg;
-    const int ox = Nzg, oy = Nzg * L.pitch;
+    T* const xc = X + (int64_t)c * Nzg;
+    const T* const bc = B + (int64_t)c * Nzg;
+    const int ox = Nzg, oy = Nzg * Nxg;
     // the column borders a ghost column (ghost relaxation before or after it,
     // and the corner columns)
     const bool edge = act && (i <= 3 || i >= Nxg - 2 || (THREE && (j <= 3 || j >= Nyg - 2)));
 
-    auto colidx = [&](int ii, int jj) -> int64_t { return IC(L, ii, jj); };
+    auto colidx = [&](int ii, int jj) -> int64_t { return (int64_t)(ii - 1) + (int64_t)Nxg * (jj - 1); };
     // Relax ghost column cg: Neumann rows k = 2..Nzg with the 3-point stencil
     // wa x(ca) + wb x(cb) + wg x(cg) = b, identity row k = 1. With post set,
     // the value of this column (ca if own == 1, cb if own == 2) is the lane's
@@ -596,34 +615,6 @@ __device__ __forceinline__ void colour_col1(const LevelDev<T>& L, int i, int j, 
     if (edge) ghosts(true, xn, xfs);
 }
 
-template <typename T, bool THREE, int S, bool CROSS>
-__device__ void colour_warp(const LevelDev<T>& L, int colour, int base, const RowConst<T>& rk) {
-    const int Nxg = L.Nxg, Nyg = L.Nyg;
-    const int lane = threadIdx.x & 31;
-    const int nxi = Nxg - 2 - L.per, nyi = THREE ? Nyg - 2 : 1;
-    // columns of this colour: every other i (and every other j with 4 colours)
-    const bool four = (L.ncolor == 4);
-    const int ni = (nxi + 1) / 2;
-    const int nj = four ? (nyi + 1) / 2 : nyi;
-    const int total = ni * nj;                // columns of one colour (< 2^31)
-
-    const int q = base + (lane / S);
-    bool act = q < total;
-    int i = 2, j = THREE ? 2 : 1;
-    if (act) {
-        const int tj = q / ni, ti = q - tj * ni;   // 32-bit division
-        if (four) {
-            j = THREE ? 2 + 2 * tj + (colour >> 1) : 1;
-            i = 2 + 2 * ti + (colour & 1);
-        } else {
-            j = THREE ? 2 + tj : 1;
-            i = 2 + 2 * ti + ((colour + j) & 1);    // (i + j) & 1 == colour
-        }
-        act = (i <= Nxg - 1 - L.per) && (!THREE || j <= Nyg - 1);
-    }
-    colour_col1<T, THREE, S, CROSS>(L, i, j, act, rk);
-}
-
 // Row constants of row k (clamped to the interior rows 2..Nzg-1).
 template <typename T>
 __device__ __forceinline__ RowConst<T> row_const_k(const LevelDev<T>& L, int k) {
@@ -664,12 +655,12 @@ __device__ __forceinline__ void colour_col2(const LevelDev<T>& L, int i, int j, 
     const bool va = act && ka <= Nzg - 1, vb = act && kb <= Nzg - 1;
     const int last = (R - 1) / 2;           // lane holding row Nzg-1 (the free surface follows it)
     const int c = (i - 1) + Nxg * (j - 1);
-    T* const xc = X + IC(L, i, j) * Nzg;
+    T* const xc = X + (int64_t)c * Nzg;
     const T* const bc = br;
     const int ox = Nzg;
     const bool edge = !TILE && act && (i <= 3 || i >= Nxg - 2 || (THREE && (j <= 3 || j >= Nyg - 2)));
 
-    auto colidx = [&](int ii, int jj) -> int64_t { return IC(L, ii, jj); };
+    auto colidx = [&](int ii, int jj) -> int64_t { return (int64_t)(ii - 1) + (int64_t)Nxg * (jj - 1); };
     // ghost column cg: Neumann rows of this lane's levels, wa x(ca) + wb x(cb) + wg x(cg) = b;
     // with post set, the value of this column (ca if own == 1, cb if own == 2)
     // is the lane's new one
@@ -997,11 +988,12 @@ __device__ void restrict_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const
 // value is the weighted sum over (at most) 2 x 2 x 2 coarse points with the
 // fine level's per-direction tables. The free-surface row, the bottom ghost
 // row and the ghost columns are not touched.
-// prolong_value adds the correction of fine point (kf, ifn, jf) to *x.
 template <typename T>
-__device__ __forceinline__ void prolong_value(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* xc, T* x, int kf,
-                                              int ifn, int jf) {
+__device__ void prolong_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* xc, T* xf, int64_t p) {
     const int gy = (F.Nyg > 1) ? 1 : 0;
+    int kf, ifn, jf;
+    int64_t cfl;
+    decomp(F, p, kf, cfl, ifn, jf);
     if (kf == 1 || kf == F.Nzg || ifn == 1 || ifn == F.Nxg || (gy && (jf == 1 || jf == F.Nyg))) return;
     if (F.per && ifn == F.Nxg - 1) return;   // periodic x: the repeated column stays zero
     const int2 zi = __ldg(reinterpret_cast<const int2*>(F.piz) + (kf - 1));
@@ -1026,14 +1018,7 @@ __device__ __forceinline__ void prolong_value(const LevelDev<T>& F, const LevelD
     };
     T v = wz0 * Py(zi.x);
     if (wz1 != T(0)) v += wz1 * Py(zi.y);
-    *x += v;
-}
-template <typename T>
-__device__ void prolong_item(const LevelDev<T>& F, const LevelDev<T>& Cc, const T* xc, T* xf, int64_t p) {
-    int kf, ifn, jf;
-    int64_t cfl;
-    decomp(F, p, kf, cfl, ifn, jf);
-    prolong_value(F, Cc, xc, xf + p, kf, ifn, jf);
+    xf[p] += v;
 }
 
 // Coarsest level, row r of x = A^{-1} b.

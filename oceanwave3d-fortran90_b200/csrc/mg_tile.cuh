@@ -13,7 +13,7 @@ constexpr int kTileMaxNzg = 34;
 // reads lo x_{k-1} + dg x_k + up x_{k+1} + off = b_k, id = 1 / dg, g = lo / dg.
 template <typename T>
 struct UniTab {
-    T id[kTileMaxNzg], g[kTileMaxNzg], lo[kTileMaxNzg], dg[kTileMaxNzg], up[kTileMaxNzg];
+    T id[kTileMaxNzg], g[kTileMaxNzg], lo[kTileMaxNzg], up[kTileMaxNzg];
     T t0, t1, t6;             // bottom row: x_1 = (b_1 - t0 x_2 - t1 x_3) t6
     T wxl, wxr, wyd, wyu;     // neighbour columns' weights
     T gx[2][3], gy[2][3];     // ghost rows (low, high wall): nearest, second, 1 / ghost weight

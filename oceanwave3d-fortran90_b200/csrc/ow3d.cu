@@ -239,7 +239,7 @@ TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vec
         const double lo = s3 * sz(1, k, 0) + cz * sz(2, k, 0), up = s3 * sz(1, k, 2) + cz * sz(2, k, 2);
         u.id[k - 1] = T(1.0 / dg);
         u.g[k - 1] = T(lo / dg);
-        u.lo[k - 1] = T(lo); u.dg[k - 1] = T(dg); u.up[k - 1] = T(up);
+        u.lo[k - 1] = T(lo); u.up[k - 1] = T(up);
     }
     u.t0 = T(bt[8 * q0]); u.t1 = T(bt[8 * q0 + 1]); u.t6 = T(bt[8 * q0 + 6]);
     u.wxl = T(sx(2, 2, 0)); u.wxr = T(sx(2, 2, 2));
