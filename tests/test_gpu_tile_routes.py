@@ -25,7 +25,7 @@ def _expected(sim, modes, mixed, coop):
     N = [sim.level_size(l) for l in range(nl)]
     ncolor = [sim.level_dims(l)[3] for l in range(nl)]
     ld = max([l for l in range(1, nl - 1) if N[l] <= DENSE], default=0)
-    cross = sim.cross
+    cross = [sim.cross] * nl if not sim.top_cross else [False] * (nl - 1) + [True]
 
     def every(l):
         return all(modes[q] != tf.NONE for q in range(ld + 1, l + 1))
@@ -37,7 +37,7 @@ def _expected(sim, modes, mixed, coop):
             return 1
         if modes[l] != tf.NONE:
             return 2 + cycle(l - 1)
-        return 2 * (ncolor[l] + (2 if cross else 0)) + 3 + cycle(l - 1)
+        return 2 * (ncolor[l] + (2 if cross[l] else 0)) + 3 + cycle(l - 1)
 
     top = nl - 1
     fine = modes[top] != tf.NONE and (N[top] > coop or every(top))
@@ -46,14 +46,14 @@ def _expected(sim, modes, mixed, coop):
     return n, [l for l in range(ld + 1, nl) if modes[l] != tf.NONE], nl - 1 - ld
 
 
-def _compare(ow3d, p, geo, precision, slope=False, tiled="all", coop=COOP):
+def _compare(ow3d, p, geo, precision, slope=False, tiled="all", coop=COOP, top_cross=False):
     L = ow3d.lib()
     modes = [f[0] for f in tf.forms(ow3d, p, geo, precision)]
     assert p.precision == precision
     old_coop = L.ow3d_test_set_coop_max_points(coop)
     try:
         with ow3d.Simulation(p, **geo) as sim:
-            sim.cross = slope
+            sim.cross, sim.top_cross = slope, top_cross
             r = np.random.default_rng(3).standard_normal(sim.N)
             if p.periodic_x:   # image columns are identity rows with a zero right-hand side
                 r3 = r.reshape(sim.Nyg, sim.Nxg, sim.Nzg)
@@ -150,3 +150,23 @@ def test_tall_slope_fp64(ow3d, n, tiled, coop):
 def test_varying_depth_without_slopes(ow3d, precision):
     p, geo = _slope((65, 33, 9))
     _compare(ow3d, p, dict(h=geo["h"]), precision, tiled=0)
+
+
+@pytest.mark.parametrize("coop", [COOP, 0])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("coarse", ["varying", "flat"])
+def test_form_changes_between_levels(ow3d, coarse, precision, coop):
+    """A slope at one column that the coarse grids skip: a tiled level with
+    mixed-derivative terms above levels without them, which are flat and tiled,
+    or of varying depth and per-phase (their iterate is cleared by the tiled
+    level's way down)."""
+    p, geo = _slope((257, 65, 13), **({} if coarse == "varying" else {"amp": 0.0}))
+    h = np.array(geo["h"]).reshape(67, 259)
+    hx = np.zeros_like(h)
+    h[30, 50] *= 0.99
+    hx[30, 50] = 0.05
+    g = dict(h=h.ravel(), hx=hx.ravel())
+    modes = [f[0] for f in tf.forms(ow3d, p, g, precision)]
+    below = tf.NONE if coarse == "varying" else tf.UNIFORM
+    assert modes[-1] == tf.CROSS and set(modes[1:-1]) == {below}
+    _compare(ow3d, p, g, precision, tiled=1 if coarse == "varying" else "all", coop=coop, top_cross=True)
