@@ -74,8 +74,10 @@ def _compare(ow3d, p, geo, precision, slope=False, tiled="all", coop=COOP, top_c
         L.ow3d_test_set_coop_max_points(old_coop)
     if tiled == "all":
         assert len(which) == above and above > 0
-    else:
+    elif tiled is not None:
         assert len(which) == tiled
+    else:
+        assert which
     assert (c1 - c0, c2 - c1) == (n, off)
     eps = 2.0 ** -53 if precision == 0 else 2.0 ** -24
     assert np.all(np.isfinite(u))
@@ -138,7 +140,7 @@ def test_periodic_basin(ow3d, n, precision):
 @pytest.mark.parametrize("coop", [COOP, 0])
 @pytest.mark.parametrize("n,tiled", [((65, 33, 25), 3), ((65, 33, 33), 1)])
 def test_tall_slope_fp64(ow3d, n, tiled, coop):
-    """In FP64 a sloping level of 25 or more sigma levels that is wide enough
+    """In FP64 a sloping level of 23 or more sigma levels that is wide enough
     has no tile form: its smallest core with its halo exceeds the shared
     memory. Such a basin's levels up to coop points run fused, tiled or not;
     with coop 0 per-phase levels stand above tiled ones."""
@@ -170,3 +172,13 @@ def test_form_changes_between_levels(ow3d, coarse, precision, coop):
     below = tf.NONE if coarse == "varying" else tf.UNIFORM
     assert modes[-1] == tf.CROSS and set(modes[1:-1]) == {below}
     _compare(ow3d, p, g, precision, tiled=1 if coarse == "varying" else "all", coop=coop, top_cross=True)
+
+
+@pytest.mark.parametrize("strategy", [1, 2])
+@pytest.mark.parametrize("n", [(65, 33, 17), (17, 65, 33), (33, 33, 33)])
+def test_coarsening_strategies(ow3d, n, strategy):
+    """Levels coarsened in one direction at a time, or in all three at once."""
+    for precision in (0, 1):
+        for make, slope in ((_flat, False), (_slope, True)):
+            p, geo = make(n, MGCoarseningStrategy=strategy)
+            _compare(ow3d, p, geo, precision, slope=slope, tiled=None, coop=0)
