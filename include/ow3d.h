@@ -447,7 +447,8 @@ int ow3d_set_paddle_signal(ow3d_handle* h, int nt, int n2, double dt, const doub
  * together (ow3d_step_batch): the coarse cycles of different simulations then
  * overlap, where a grid-wide cycle takes the whole device for its duration.
  * Levels that run on the fused tile kernels (flat, or sloping with the slopes
- * given, nu1 = nu2 = 1) are plain launches that overlap either way; where the
+ * given, with nu1 = nu2 = maxit = 1; not FP64 basins that slope and have more
+ * than 22 sigma levels) are plain launches that overlap either way; where the
  * coarse levels do run fused, measured on a B200 over a stream of simulations:
  * 1.55x the batched throughput and half the step latency, and a handle stepped
  * alone is 10-30% slower, so the default is off. Results are bitwise the same

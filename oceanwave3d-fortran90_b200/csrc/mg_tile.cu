@@ -1572,12 +1572,20 @@ void size_geo(const LevelDev<T>& L, TileGeo& g, int cx, int cy, bool cross, bool
 template <typename T>
 void tile_geometry(const LevelDev<T>& L, TileLevel<T>& t) {
     const bool three = L.Nyg > 1, cross = t.mode == kTileCross;
-    // Of the cores that leave room for two blocks per SM, the one of least
-    // waves x (columns of a tile with its halo + 200): a tile's time is its
-    // columns' share of the staging and the phases plus the phases' latency,
-    // worth some 200 columns. Levels of few tiles so take smaller cores, and
-    // large ones the largest that fits (way up at 1025x257x17 FP64: 16x8 80 us,
-    // 24x8 70 us; one level below, 561 tiles of 16x8 21 us, 374 of 24x8 23 us).
+    // Of the cores that leave shared memory for two blocks per SM (the smallest
+    // core: for one), the one of least waves x (columns of a tile with its halo
+    // + 200): a tile's time is its columns' share of the staging and the phases
+    // plus the phases' latency, worth some 200 columns. Levels of few tiles so
+    // take smaller cores, and large ones the largest that fits (way up at
+    // 1025x257x17 FP64: 16x8 80 us, 24x8 70 us; one level below, 561 tiles of
+    // 16x8 21 us, 374 of 24x8 23 us). Uniform levels run two blocks per SM, as
+    // the waves are counted (FP64 96 to 128 registers at 256 or 320 threads).
+    // The 3-D sloping forms do not: at 98 to 128 registers a block of 384
+    // threads or more is alone on its SM, so 165 tiles (257x33x9 FP64, finest
+    // level) are a second wave of 17 tiles, 27 and 23 us a launch against 17
+    // and 15 us for the 51 tiles of the level below. In FP64 the smallest core,
+    // 8x8 with its halo of 7, fits up to 22 sigma levels on a wide level;
+    // taller ones take the per-phase kernels.
     static const int uni3[][2] = {{32, 8}, {24, 8}, {16, 8}, {8, 4}}, cross3[][2] = {{16, 16}, {16, 8}, {8, 8}};
     static const int line[][2] = {{64, 1}, {32, 1}, {16, 1}};
     const int (*cand)[2] = three ? (cross ? cross3 : uni3) : line;
@@ -1679,7 +1687,12 @@ void up_ordered(const LevelF& F, const LevelF& Cc, const TileLevel<float>& t, Rh
              F, Cc, b.p, xs, xc, out, t.r, g);
 }
 
-// Uniform levels: the level counts of the decks' usual Nz unrolled. Cross
+// Uniform levels: the columns of 9 and, in 3-D, 17 sigma levels, the usual
+// counts, unrolled, any other by the general form, which takes those two as
+// well but slower: a V cycle at 1025x257x17 258 us unrolled against 347 (FP32
+// 209, 294), at 1025x257x9 162 against 220, of a 513x9 flume 24 against 35; at
+// 1025x257x13, by the general form, 280. (The unrolled FP64 way up of 17 levels
+// spills 76 bytes a thread at the 128 registers of two blocks per SM.) Cross
 // levels: the lanes per column (FP64, and FP32 with two rows per lane: two
 // rows each; else one).
 #define OW3D_TILE(way, ...)                                                     \

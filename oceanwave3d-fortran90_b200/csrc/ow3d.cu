@@ -182,7 +182,8 @@ int upload(ow3d_handle* H, T** p, const std::vector<double>& v) {
 // 1e-12, so the FP32 cross kernels keep the per-phase kernels' order; flat
 // levels move by 1e-11 at most in FP32. Periodic levels with an odd period
 // (the two colours would meet at its ends) have none, nor has a period of two
-// columns (a core holds three or more).
+// columns (a core holds three or more). A level none of whose cores fits the
+// shared memory or a launch (tile_geometry) has none either.
 template <typename T>
 TileLevel<T> tile_level(const LevelHost& h, const LevelDev<T>& d, const std::vector<double>& cf,
                         const std::vector<double>& bt, bool same) {
