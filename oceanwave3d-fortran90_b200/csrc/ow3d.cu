@@ -180,7 +180,10 @@ int upload(ow3d_handle* H, T** p, const std::vector<double>& v) {
 // steep basins' results by up to 1e-8 (65x33x9 shoal, which stops at the matvec
 // limit: 2e-9; two-dimensional 65x17 and 257x17 flumes: 1e-9), in FP64 by
 // 1e-12, so the FP32 cross kernels keep the per-phase kernels' order; flat
-// levels move by 1e-11 at most in FP32. Periodic levels with an odd period
+// levels in FP32 move by 1e-11 under the flexible solver, and with left GMRES,
+// whose mixed form is 1e-7 to 1e-5 off FP64 either way, by as much as that
+// error, which is no larger than with the per-phase kernels (medians over 16
+// seas and periodic waves: eta 1.7e-6 against 2.1e-6). Periodic levels with an odd period
 // (the two colours would meet at its ends) have none, nor has a period of two
 // columns (a core holds three or more). A level none of whose cores fits the
 // shared memory or a launch (tile_geometry) has none either.
